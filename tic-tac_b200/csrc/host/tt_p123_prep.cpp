@@ -1,9 +1,12 @@
 // Host tables for the device P123 builder.  See tt_p123.h.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
+#include <map>
 #include <unordered_map>
+#include <utility>
 
 #include "tt_math.h"
 #include "tt_p123.h"
@@ -115,7 +118,11 @@ bool p123_prepare(const RunParams& rp, const FWPStates& fwp, const PWChannel& ch
   t.lenl = spharm_len(max_l3);
   const int Lmax = max_L12 + max_l3;
   t.plm1.resize((size_t)t.Nx * t.lenl);
-  for (int ix = 0; ix < t.Nx; ix++) legendre_spharm_array(max_l3, t.x[ix], &t.plm1[(size_t)ix * t.lenl]);
+  std::vector<double> row(t.lenl);
+  for (int ix = 0; ix < t.Nx; ix++) {
+    legendre_spharm_array(max_l3, t.x[ix], row.data());
+    for (int i = 0; i < t.lenl; i++) t.plm1[(size_t)i * t.Nx + ix] = row[i];
+  }
   t.L12.assign(ch.L_2N, ch.L_2N + ch.Nalpha);
   t.l3.assign(ch.L_1N, ch.L_1N + ch.Nalpha);
 
@@ -137,10 +144,49 @@ bool p123_prepare(const RunParams& rp, const FWPStates& fwp, const PWChannel& ch
               ch, a, ap, &n9[((size_t)a * (Lmax + 1) + Lt) * 2], &n9[((size_t)ap * (Lmax + 1) + Lt) * 2], s6);
       }
 
-  // Term lists.  The reference evaluates Gtilde for (row alpha' = alphap_idx,
-  // column alpha = alpha_idx) with Atilde_store[alphap][alpha] and
+  // Pairs and their F.  The reference evaluates Gtilde for (row alpha' =
+  // alphap_idx, column alpha = alpha_idx) with Atilde_store[alphap][alpha] and
   // L12 = L(alpha'), l3 = l(alpha'), L12' = L(alpha), l3' = l(alpha)
   // (make_permutation_matrix.cpp:755-787, auxiliary.cpp:950-1067).
+  // F are keyed (o, Lt, o'), so that the F of one B set are neighbours.
+  std::map<std::pair<int, int>, int> orb_idx;
+  std::vector<std::pair<int, int>> orbs;
+  std::vector<int> orb(Na);
+  for (int a = 0; a < Na; a++) {
+    const auto key = std::make_pair(ch.L_2N[a], ch.L_1N[a]);
+    const auto it = orb_idx.emplace(key, (int)orbs.size()).first;
+    if (it->second == (int)orbs.size()) orbs.push_back(key);
+    orb[a] = it->second;
+  }
+  std::map<std::array<int, 3>, int> f_idx;  // (o, Lt, o') -> f
+  struct PairTerm {
+    std::array<int, 3> key;
+    double c;
+  };
+  std::vector<PairTerm> pair_terms;
+  t.pair_off.push_back(0);
+  for (int ap = 0; ap < Na; ap++) {
+    for (int a = 0; a < Na; a++) {
+      const int L12 = ch.L_2N[ap], l3 = ch.L_1N[ap];
+      const int L12p = ch.L_2N[a], l3p = ch.L_1N[a];
+      const double* A = &At[((size_t)ap * Na + a) * (Lmax + 1)];
+      const int Lt_lo = std::max(std::abs(L12 - l3), std::abs(L12p - l3p));
+      const int Lt_hi = std::min((t.two_J_3N + 5) / 2, std::min(L12 + l3, L12p + l3p));
+      const size_t n_before = pair_terms.size();
+      for (int Lt = Lt_lo; Lt <= Lt_hi; Lt++) {
+        const double fac1 = 8.0 * M_PI * M_PI * A[Lt];
+        if (fac1 == 0) continue;
+        const std::array<int, 3> key{orb[a], Lt, orb[ap]};
+        f_idx.emplace(key, 0);
+        pair_terms.push_back({key, fac1 * std::sqrt((2.0 * L12 + 1) / (4 * M_PI))});
+      }
+      if (pair_terms.size() > n_before) {
+        t.pair_ap.push_back(ap);
+        t.pair_a.push_back(a);
+        t.pair_off.push_back((int32_t)pair_terms.size());
+      }
+    }
+  }
   // Clebsch-Gordan values recur across pairs: each argument set is evaluated once
   std::unordered_map<uint64_t, double> cg_memo;
   auto cg = [&](int j1, int j2, int j3, int m1, int m2, int m3) {
@@ -152,48 +198,60 @@ bool p123_prepare(const RunParams& rp, const FWPStates& fwp, const PWChannel& ch
     cg_memo.emplace(key, c);
     return c;
   };
-  t.pair_term_off.push_back(0);
-  for (int ap = 0; ap < Na; ap++) {
-    for (int a = 0; a < Na; a++) {
-      const int L12 = ch.L_2N[ap], l3 = ch.L_1N[ap];
-      const int L12p = ch.L_2N[a], l3p = ch.L_1N[a];
-      const double* A = &At[((size_t)ap * Na + a) * (Lmax + 1)];
-      const int Lt_lo = std::max(std::abs(L12 - l3), std::abs(L12p - l3p));
-      const int Lt_hi = std::min((t.two_J_3N + 5) / 2, std::min(L12 + l3, L12p + l3p));
-      size_t n_before = t.terms.size();
-      for (int Lt = Lt_lo; Lt <= Lt_hi; Lt++) {
-        const double fac1 = 8.0 * M_PI * M_PI * A[Lt];
-        if (fac1 == 0) continue;
-        const int Mlim = std::min(l3, Lt);
-        for (int M = -Mlim; M <= Mlim; M++) {
-          const double cgm = cg(2 * L12, 2 * l3, 2 * Lt, 0, 2 * M, 2 * M) * sign_pow(M);
-          bool first = true;
-          for (int Mp = -L12p; Mp <= L12p; Mp++) {
-            if (std::abs(M - Mp) > l3p) continue;
-            GTerm g;
-            g.fac1 = fac1;
-            g.cgm = cgm;
-            g.cg2 = cg(2 * L12p, 2 * l3p, 2 * Lt, 2 * Mp, 2 * M - 2 * Mp, 2 * M);
-            g.i1 = spharm_index(l3, std::abs(M));
-            g.i2 = spharm_index(L12p, std::abs(Mp));
-            g.i3 = spharm_index(l3p, std::abs(M - Mp));
-            g.signs = 0;
-            if (M < 0 && (M % 2) == -1) g.signs |= 1;
-            if (Mp < 0 && (Mp % 2) == -1) g.signs |= 2;
-            if ((M - Mp) < 0 && ((M - Mp) % 2) == -1) g.signs |= 4;
-            if (first) g.signs |= 8;
-            first = false;
-            t.terms.push_back(g);
-          }
-        }
-      }
-      if (t.terms.size() > n_before) {
-        t.pair_ap.push_back(ap);
-        t.pair_a.push_back(a);
-        t.pair_term_off.push_back((int32_t)t.terms.size());
-        t.pair_norm.push_back(std::sqrt((2.0 * L12 + 1) / (4 * M_PI)));
-      }
+  const auto sign_of = [](int m) { return m < 0 && m % 2 != 0 ? -1.0 : 1.0; };  // (-1)^m for m < 0
+  constexpr int kPhaseB = 64;  // B of a phase, more where one (o, Lt) alone needs them
+  t.b_off.push_back(0);
+  t.f_off.push_back(0);
+  t.phase_b.push_back(0);
+  t.phase_f.push_back(0);
+  for (auto it = f_idx.begin(); it != f_idx.end();) {
+    // the F of one (o, Lt) and the B they read
+    const int o = it->first[0], Lt = it->first[1];
+    const int L12p = orbs[o].first, l3p = orbs[o].second;
+    auto end = it;
+    int Mmax = 0;
+    bool one_parity = true;
+    for (; end != f_idx.end() && end->first[0] == o && end->first[1] == Lt; ++end) {
+      const auto& op = orbs[end->first[2]];
+      Mmax = std::max(Mmax, std::min(op.second, Lt));
+      one_parity = one_parity && (op.first + op.second + L12p + l3p) % 2 == 0;
     }
+    const int Mlo = one_parity ? 0 : -Mmax, nB = Mmax - Mlo + 1;
+    int base = (int)t.b_off.size() - 1 - t.phase_b.back();  // the group's first B in its phase
+    if (base > 0 && base + nB > kPhaseB) {
+      t.phase_b.push_back((int32_t)t.b_off.size() - 1);
+      t.phase_f.push_back((int32_t)t.f_off.size() - 1);
+      base = 0;
+    }
+    t.max_phase_b = std::max(t.max_phase_b, base + nB);
+    for (int M = Mlo; M <= Mmax; M++) {
+      for (int Mp = -L12p; Mp <= L12p; Mp++) {
+        if (std::abs(M - Mp) > l3p) continue;
+        const double c = cg(2 * L12p, 2 * l3p, 2 * Lt, 2 * Mp, 2 * M - 2 * Mp, 2 * M);
+        if (c != 0)
+          t.b_terms.push_back({c * sign_of(Mp) * sign_of(M - Mp), spharm_index(L12p, std::abs(Mp)),
+                               spharm_index(l3p, std::abs(M - Mp))});
+      }
+      t.b_off.push_back((int32_t)t.b_terms.size());
+    }
+    for (; it != end; ++it) {
+      const int L12 = orbs[it->first[2]].first, l3 = orbs[it->first[2]].second;
+      const int Mlim = std::min(l3, Lt);
+      for (int M = one_parity ? 0 : -Mlim; M <= Mlim; M++) {
+        const double c = cg(2 * L12, 2 * l3, 2 * Lt, 0, 2 * M, 2 * M) * sign_pow(M) * sign_of(M);
+        if (c != 0)
+          t.f_terms.push_back({one_parity && M > 0 ? 2 * c : c, spharm_index(l3, std::abs(M)), base + M - Mlo});
+      }
+      it->second = (int)t.f_off.size() - 1;
+      t.f_off.push_back((int32_t)t.f_terms.size());
+    }
+  }
+  t.n_f = (int)t.f_off.size() - 1;
+  t.phase_b.push_back((int32_t)t.b_off.size() - 1);
+  t.phase_f.push_back(t.n_f);
+  for (const PairTerm& p : pair_terms) {
+    t.pair_f.push_back(f_idx.at(p.key));
+    t.pair_c.push_back(p.c);
   }
   return true;
 }
