@@ -46,3 +46,53 @@ def test_p123_of_waves_of_both_parities():
     A[r, c], B[r_o, c_o] = v, v_o
     assert rel(A, B) <= P123_TOL
     run.close()
+
+
+def run_and_oracle_U(c, run, Np, Nq):
+    """Oracle U of a run's channel, from the oracle's own A and G on the run's P123."""
+    T, E_com, q_idx = run.energies()
+    pw = run.host_array(0, c).reshape(-1, 9)
+    rowptr, col, val = run.P123_csr(c, run.build_P123(c))
+    rows = np.repeat(np.arange(len(rowptr) - 1, dtype=np.int32), np.diff(rowptr))
+    lay = oracle.layout(pw, Np, *[run.host_array(k) for k in range(3, 9)])
+    G = np.stack([oracle.resolvent(lay, pw.shape[0], Nq, Np, run.host_array(2), e + run.E_bound) for e in E_com])
+    A = oracle.build_A(lay, pw.shape[0], Nq, Np, rows, col, val)
+    return oracle.dense_solve(A, G, q_idx, oracle.deuterons(pw), Nq, Np)
+
+
+# the sub-panel kernel's layouts: one row per thread up to 480 rows of a CTA, two up
+# to 825; complex128 CTAs of up to 395 rows; the last sub-panel narrower than a
+# register block.  U to the refinement's and the suite's 1e-10 per element.
+@pytest.mark.parametrize("Np,Nq", [(6, 6),     # n = 396: two complex128 CTAs, last sub-panel 12 wide
+                                   (9, 5),     # n = 495: two rows per thread, last 15 wide
+                                   (15, 5),    # n = 825: the largest single complex64 CTA, last 25 wide
+                                   (19, 4),    # n = 836: two complex64 CTAs
+                                   (17, 10)])  # n = 1,870
+@pytest.mark.parametrize("batch", [1, 4])
+def test_subpanel_layouts(Np, Nq, batch):
+    from conftest import rel_elem
+
+    run = tt.Run(potential_model="LO_internal", J_2N_max=1, two_J_3N_max=1, Np_WP=Np, Nq_WP=Nq, Nphi=12, Nx=12,
+                 lab_energies="5,30", energy_batch=batch, chebyshev_s=150)
+    U_o = run_and_oracle_U(0, run, Np, Nq)
+    for prec in (tt.PRECISION_FP64, tt.PRECISION_MIXED, tt.PRECISION_MIXED_SIMT):
+        U, rep = run.solve(0, prec)
+        assert rel_elem(U, U_o) <= 1e-10, (prec, rep)
+    run.close()
+
+
+@pytest.mark.parametrize("precision", [tt.PRECISION_FP64, tt.PRECISION_MIXED])
+@pytest.mark.parametrize("i0", [0, 37, 511])
+def test_zero_column_is_reported_singular(precision, i0):
+    # A = diag(2 v), G = 1 / A in one element: column i0 of 1 - A G is exactly zero
+    Np = Nq = 16
+    n = 2 * Np * Nq
+    pw = np.array([[0, 0, 0, 1, 0, 1, 1, 1, 1], [0, 1, 1, 0, 0, 1, 1, 1, 1]], dtype=np.int32)
+    eye, e = np.tile(np.eye(Np).ravel(), 6), np.tile(np.linspace(-2, 100, Np + 1), 6)
+    swp = tt.SWP(Np, Nq, 6, 0, -2.0, e, None, eye, None, np.linspace(0, 1000, Nq + 1))
+    G = np.full(n, 0.125 + 0.25j)
+    G[i0] = 0.5
+    with pytest.raises(tt.TicTacError) as err:
+        tt.solve_faddeev(G, np.ones(n), np.arange(n, dtype=np.int32), np.arange(n + 1, dtype=np.uint64), eye, None, swp,
+                         [3], [1], tt.PW(pw), precision=precision, tensor_force=0, isospin_breaking_1S0=0)
+    assert err.value.code == tt.TT_ERR_SINGULAR and f"column {i0 + 1} " in str(err.value)

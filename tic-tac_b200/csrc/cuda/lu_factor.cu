@@ -4,14 +4,11 @@
 //
 // Outer panels of NB columns (512 for the complex64 / tensor-core path, 128
 // for complex128).  Each panel is factored in IB = 32 column sub-panels:
-//   k_subpanel_smem  cooperative kernel with each block's rows in shared
-//                memory, ONE grid barrier per column: every block posts its
-//                best pivot candidate as a packed 64-bit key (atomicMax) and a
-//                copy of that row (the owner of the diagonal row posts it too),
-//                so after the barrier every block reads the key and the pivot
-//                row and the two owners swap their rows without a second
-//                barrier (k_subpanel: the same from global memory, for
-//                sub-panels too tall for shared memory)
+//   k_subpanel_ll  cooperative kernel with each block's rows on chip and no
+//                grid barrier: every block posts its best pivot row in tagged
+//                records that the others poll (k_subpanel: from global
+//                memory with a grid barrier per column, for sub-panels too
+//                tall for shared memory)
 //   k_laswp2     the sub-panel's interchanges on the rest of the panel
 //   k_trsm_blk   U = L^{-1} U for the 32-wide unit-lower diagonal block
 //   tc_gemm_sub / k_gemm_sub  rank-32 update of the remaining panel columns
@@ -22,6 +19,7 @@
 
 #include <algorithm>
 #include <functional>
+#include <vector>
 
 #include "tc2_pack.cuh"
 #include "tt_kernels.h"
@@ -61,8 +59,8 @@ __device__ __forceinline__ T cdiv_smith(T a, T b) {
 
 constexpr int IB = 32;
 constexpr int SP = IB + 1;                     // shared-memory row stride of a staged sub-panel
-constexpr size_t kSubpanelSmem = 220 * 1024;  // bound on one block's staged sub-panel rows
-constexpr int SP_THREADS = 512;               // threads of the shared-memory sub-panel kernel
+constexpr size_t kSubpanelSmem = 226 * 1024;  // shared memory of a CTA of the on-chip sub-panel kernel
+constexpr int SP_WARPS = 16;                  // most warps of a CTA of the on-chip sub-panel kernel
 
 template <typename T>
 struct PivotScratch {
@@ -70,19 +68,18 @@ struct PivotScratch {
   int* idx;                 // [2][G]
   T* row;                   // [2][G][IB]
   T* top;                   // [2][IB]
-  unsigned long long* key;  // [n], zero before the factorization: column j's packed pivot
 };
 
 // Matrices of equal n factored together: the sub-panel grid is split into B
-// equal groups of blocks, group b working on matrix b, all sharing each grid
-// barrier (the barrier, not the work, bounds a sub-panel column).
+// equal groups of blocks, group b working on matrix b (the exchange of the
+// pivot, not the work, bounds a sub-panel column).
 constexpr int kMaxBatch = 4;
 template <typename T>
 struct SubpanelBatch {
   T* A[kMaxBatch];
   int32_t* ipiv[kMaxBatch];
-  unsigned long long* key[kMaxBatch];  // [n] each, zero before the factorization
   int* info;                           // [B]
+  int* err;                            // set when a wait ran out
   int B;
 };
 // a[i] by predicated selects: a runtime index into a kernel parameter array
@@ -231,208 +228,517 @@ __global__ void __launch_bounds__(256) k_subpanel(T* __restrict__ A, int n, int 
   }
 }
 
-// (value, row) pivot candidates: larger |re| + |im| wins, ties go to the lower
-// row, as in LAPACK's izamax; row < 0 marks "no candidate"
-template <typename V>
-__device__ __forceinline__ bool cand_better(V v, int i, V bv, int bi) {
-  return i >= 0 && (bi < 0 || v > bv || (v == bv && i < bi));
+// ---- sub-panel resident on chip
+//
+// The CTAs of a matrix hold its sub-panel rows, one thread per row (two where
+// the rows outnumber the threads), columns in register blocks of CB: within a
+// block a column's elimination touches registers only; the columns right of the
+// block wait in shared memory and take all CB pivots in one rank-CB update.
+// Every element still sees the pivots one after another in ascending order.
+//
+// What bounds a column is the exchange of its pivot.  Each CTA posts its best
+// row as 16-byte records {element, tag, row index}, one atomic store each: the
+// tag (column + 1) tells a reader that the record is this column's, so there is
+// no barrier, no fence and no flag beside the data.  Up to LL_ONE_HOP CTAs a
+// matrix, every CTA reads all posted rows and picks the winner itself: one
+// store-to-load trip through L2.  With more, the rows would cost more L2
+// traffic than a second trip, so it reads the candidates' own elements, then the
+// winner's row.  The diagonal row always lives in the matrix's first CTA, which
+// posts it for the interchange; a matrix of one CTA exchanges in shared memory.
+// Records are double-buffered by column parity: a CTA posts column j + 2 only
+// after it has seen every CTA's column j + 1, posted after their reads of j.
+//
+// Per sub-panel of 32 columns, against the kernel before it (a row per warp in
+// shared memory, one cooperative grid barrier, an atomicMax and two dependent
+// reads per column), two complex64 matrices: n = 512 118 -> 43 us, n = 10,944
+// 134 -> 82 us, n = 16,128 139 -> 86 us, n = 42,300 201 -> 113 us; four at
+// n = 20,160 178 -> 97 us; one complex128 at n = 8,496 135 -> 101 us.  Of a
+// column's 2.5 to 6 thousand cycles the trips through L2 take about 1,200 each;
+// the rest is the latency of its own instructions.
+// Waits end after LL_SPINS polls: the error word is set and the rest of the
+// launch runs without waiting.
+constexpr int LL_ONE_HOP = 32;
+constexpr int LL_SPINS = 1 << 20;
+constexpr int SP_ROWS = 480;  // rows of a CTA, where the CTAs suffice: one per thread of 15 warps
+constexpr int LL_PER_WARP = 4;  // posted rows that a warp gathers, the diagonal row among them
+
+__device__ __forceinline__ void ll_store(void* p, unsigned long long lo, unsigned long long hi) {
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
+               "l"(lo), "l"(hi)
+               : "memory");
 }
-// best of lanes [0, W) into lane 0 (W a power of two <= 32)
-template <int W, typename V>
-__device__ __forceinline__ void warp_argmax(V& v, int& i) {
-#pragma unroll
-  for (int o = W / 2; o > 0; o >>= 1) {
-    const V ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (cand_better(ov, oi, v, i)) {
-      v = ov;
-      i = oi;
-    }
+__device__ __forceinline__ void ll_load(const void* p, unsigned long long& lo, unsigned long long& hi) {
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+}
+// one element of a posted row: complex64 in one record, complex128 in two
+template <typename T>
+struct LL;
+template <>
+struct LL<float2> {
+  static constexpr int BYTES = 16;
+  static __device__ __forceinline__ void post(unsigned char* p, float2 v, unsigned long long hi) {
+    ll_store(p, (unsigned long long)__float_as_uint(v.x) | ((unsigned long long)__float_as_uint(v.y) << 32), hi);
   }
+  static __device__ __forceinline__ bool poll(const unsigned char* p, float2& v, unsigned long long& hi,
+                                              unsigned tag) {
+    unsigned long long lo;
+    ll_load(p, lo, hi);
+    v = make_float2(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)));
+    return (unsigned)hi == tag;
+  }
+};
+template <>
+struct LL<double2> {
+  static constexpr int BYTES = 32;
+  static __device__ __forceinline__ void post(unsigned char* p, double2 v, unsigned long long hi) {
+    ll_store(p, (unsigned long long)__double_as_longlong(v.x), hi);
+    ll_store(p + 16, (unsigned long long)__double_as_longlong(v.y), hi);
+  }
+  static __device__ __forceinline__ bool poll(const unsigned char* p, double2& v, unsigned long long& hi,
+                                              unsigned tag) {
+    unsigned long long lx, ly, h2;
+    ll_load(p, lx, hi);
+    ll_load(p + 16, ly, h2);
+    v = make_double2(__longlong_as_double((long long)lx), __longlong_as_double((long long)ly));
+    return (unsigned)hi == tag && (unsigned)h2 == tag;
+  }
+};
+
+// Pivot candidates as keys: 0 for none (NaN magnitudes included), else the bits
+// of |re| + |im| plus one, which order as the magnitudes do; ties go to the
+// lower row, as in LAPACK's izamax.
+__device__ __forceinline__ unsigned pivot_key(float2 v) {
+  const float m = fabsf(v.x) + fabsf(v.y);
+  return m >= 0 ? __float_as_uint(m) + 1u : 0u;
 }
-// A candidate packed so that a larger key is the better candidate: the top 44
-// bits of the non-negative double magnitude (exact for FP32 magnitudes;
-// complex128 magnitudes that agree to 2^-32 relative count as equal), then
-// the complement of the row offset (lower row wins ties).  0 = no candidate.
-__device__ __forceinline__ unsigned long long pivot_key(double v, int off) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v) >> 20;
-  return (b << 20) | (unsigned long long)(0xFFFFF - off);
+__device__ __forceinline__ unsigned long long pivot_key(double2 v) {
+  const double m = fabs(v.x) + fabs(v.y);
+  return m >= 0 ? (unsigned long long)__double_as_longlong(m) + 1ull : 0ull;
+}
+__device__ __forceinline__ unsigned warp_max(unsigned k) { return __reduce_max_sync(0xffffffffu, k); }
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+  return ((unsigned long long)hi << 32) | lo;
+}
+// the warp's best (key, row) to every lane, the lower row on ties; returns the lane that held it
+template <typename K>
+__device__ __forceinline__ int warp_best(K& key, int& row) {
+  const K best = warp_max(key);
+  unsigned who = __ballot_sync(0xffffffffu, key == best);
+  if (who & (who - 1)) {
+    const int r = (int)__reduce_min_sync(0xffffffffu, key == best ? (unsigned)row : 0x7fffffffu);
+    who = __ballot_sync(0xffffffffu, key == best && row == r);
+  }
+  const int lane = __ffs(who) - 1;
+  key = best;
+  row = __shfl_sync(0xffffffffu, row, lane);
+  return lane;
 }
 
-// Same algorithm with each block's rows of the sub-panel resident in shared
-// memory for all w columns: one coalesced load and one store per element.
-// Warps own rows and lanes own columns.  One pass per column applies the
-// multipliers (times the pivot's reciprocal, as LAPACK's zgetf2 scales),
-// updates the remaining columns and tracks the next column's candidate.  The
-// pivot is chosen through one 64-bit atomicMax per block on the column's key,
-// so after the grid barrier each block reads one word, then the winner's
-// published row: one grid barrier, two dependent L2 reads and two block
-// barriers per column.  Row offsets below 2^20 - 1 (checked by the caller).
-// With a batch, blocks [b Gb, (b+1) Gb) factor matrix b (gridDim.x = B Gb).
-// With pk0 < pk1, the sub-panel's interchanges are also applied to the other
-// columns [pk0, c0) and [c0 + w, pk1) of its panel after one more grid barrier.
+// 1 / b by one reciprocal, b scaled by a power of two where |b|^2 would leave the
+// range it is formed in without loss
+__device__ __forceinline__ float2 pivot_recip(float2 b) {
+  const float big = fmaxf(fabsf(b.x), fabsf(b.y));
+  float sc = 1.0f;
+  if (!(big > 0x1p-50f && big < 0x1p50f)) {
+    const int e = min(max((int)(__float_as_uint(big) >> 23) - 127, -126), 126);
+    sc = __uint_as_float((unsigned)(127 - e) << 23);
+  }
+  const float x = b.x * sc, y = b.y * sc;
+  const float r = sc * __frcp_rn(fmaf(x, x, y * y));
+  return make_float2(x * r, -y * r);
+}
+__device__ __forceinline__ double2 pivot_recip(double2 b) {
+  const double big = fmax(fabs(b.x), fabs(b.y));
+  double sc = 1.0;
+  if (!(big > 0x1p-400 && big < 0x1p400)) {
+    const int e = min(max((int)(((unsigned long long)__double_as_longlong(big)) >> 52) - 1023, -1022), 1022);
+    sc = __longlong_as_double((long long)((unsigned long long)(1023 - e) << 52));
+  }
+  const double x = b.x * sc, y = b.y * sc;
+  const double r = sc * __drcp_rn(fma(x, x, y * y));
+  return make_double2(x * r, -y * r);
+}
+
+// a column's U elements of a block, by 16-byte loads
+__device__ __forceinline__ void load_u(const float2* p, float2 (&u)[8]) {
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const float4 f = reinterpret_cast<const float4*>(p)[c];
+    u[2 * c] = make_float2(f.x, f.y);
+    u[2 * c + 1] = make_float2(f.z, f.w);
+  }
+}
+__device__ __forceinline__ void load_u(const double2* p, double2 (&u)[4]) {
+#pragma unroll
+  for (int c = 0; c < 4; c++) u[c] = p[c];
+}
+
 template <typename T>
-__global__ void __launch_bounds__(SP_THREADS) k_subpanel_smem(SubpanelBatch<T> bt, int n, int c0, int w, int pk0,
-                                                              int pk1, PivotScratch<T> scr) {
-  cg::grid_group grid = cg::this_grid();
-  extern __shared__ unsigned char sp_raw[];
-  T* sA = reinterpret_cast<T*>(sp_raw);  // [chunk][SP]
-  using R = typename Real<T>::R;
-  constexpr int NW = SP_THREADS / 32;
-  const int G = gridDim.x;  // scratch row slots are indexed by the global block
-  const int Gb = G / bt.B, grp = blockIdx.x / Gb, cta = blockIdx.x - grp * Gb;
+struct SubpanelCfg {
+  using Key = decltype(pivot_key(T{}));
+  static constexpr int CB = sizeof(T) == 8 ? 8 : 4;  // columns of a register block
+  static constexpr int RW = IB + CB;                 // padded row: a block read past column 31 stays inside
+  // shared memory beside the rows: the gathered rows and diagonal rows (two
+  // columns' worth), the block's U rows, candidates and pivots
+  static constexpr size_t EXTRA = sizeof(T) * (2 * SP_WARPS * RW + 2 * RW + CB * IB) +
+                                  2 * SP_WARPS * 2 * (sizeof(Key) + sizeof(int)) + IB * sizeof(int) + 16;
+  static constexpr int MAX_ROWS = (int)((kSubpanelSmem - EXTRA) / (SP * sizeof(T)));
+};
+// rows per thread of a CTA of `rows` rows, and its threads: the row warps and one more
+inline int sp_rpt(int rows) { return rows > 32 * (SP_WARPS - 1) ? 2 : 1; }
+inline int sp_threads(int rows) { return 32 * ((rows + 32 * sp_rpt(rows) - 1) / (32 * sp_rpt(rows)) + 1); }
+
+// Sub-panel rows [c0, n), columns [c0, c0 + w) of bt.B matrices, Gb = gridDim.x / B
+// CTAs each (group b works on matrix b); at least IB rows in the first CTA.
+// Warps but the last own rows, the last solves the block's U rows meanwhile.
+// With pk0 < pk1, the sub-panel's interchanges are also applied to the other
+// columns [pk0, c0) and [c0 + w, pk1) of its panel.  rec: [2][B][Gb + 1][IB]
+// records, zero before the factorisation.
+template <typename T, int RPT>
+__global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<T> bt, int n, int c0, int w, int pk0,
+                                                                  int pk1, unsigned char* __restrict__ rec) {
+  using CF = SubpanelCfg<T>;
+  using Key = typename CF::Key;
+  constexpr int CB = CF::CB, RW = CF::RW, NONE = 0x7fffffff;
+  extern __shared__ __align__(16) unsigned char sp_raw[];
+  const int Gb = gridDim.x / bt.B, grp = blockIdx.x / Gb, cta = blockIdx.x - grp * Gb;
   T* __restrict__ A = batch_pick(bt.A, grp);
-  int32_t* __restrict__ ipiv = batch_pick(bt.ipiv, grp);
-  unsigned long long* __restrict__ keys = batch_pick(bt.key, grp);
-  T* __restrict__ top = scr.top + (size_t)grp * 2 * IB;  // [2][IB] per matrix
   const int m = n - c0;
   const int chunk = (m + Gb - 1) / Gb;
-  const int lo = c0 + cta * chunk;
-  const int hi = min(n, lo + chunk);
-  const int nr = max(0, hi - lo);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __shared__ R s_wv[NW];
-  __shared__ int s_wi[NW];
-  __shared__ T s_prow[IB];
-  __shared__ int s_zero;
+  const int lo = cta * chunk;  // first row of this CTA, from c0
+  const int nr = max(0, min(m, lo + chunk) - lo);
+  T* sRow = reinterpret_cast<T*>(sp_raw);                  // [2][SP_WARPS][RW] gathered rows
+  T* sTop = sRow + 2 * SP_WARPS * RW;                      // [2][RW] diagonal row
+  T* sU = sTop + 2 * RW;                                   // [IB][CB] solved pivot rows of the block, by column
+  Key* sKey = reinterpret_cast<Key*>(sU + CB * IB);        // [2][2][SP_WARPS] candidates: own, gathered
+  int* sIdx = reinterpret_cast<int*>(sKey + 4 * SP_WARPS);  // [2][2][SP_WARPS]
+  int* sPiv = sIdx + 4 * SP_WARPS;                         // [IB]
+  int* sFlag = sPiv + IB;                                  // a wait ran out
+  T* sA = reinterpret_cast<T*>(sp_raw + CF::EXTRA);        // [chunk][SP]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int NW = blockDim.x >> 5, NWR = NW - 1;
+  const bool helper = warp == NWR;
+  const int col = min(lane, w - 1);
+  auto slot = [&](int buf, int g) { return rec + (((size_t)buf * bt.B + grp) * (Gb + 1) + g) * IB * LL<T>::BYTES; };
+#pragma unroll 16
   for (int r = warp; r < nr; r += NW)
-    if (lane < w) sA[r * SP + lane] = A[(size_t)(lo + r) * n + c0 + lane];
+    if (lane < w) sA[r * SP + lane] = A[(size_t)(c0 + lo + r) * n + c0 + lane];
+  if (tid == 0) *sFlag = *(volatile int*)bt.err;
   __syncthreads();
-  // this block's candidate for column jc: warp 0 reduces the warps' and posts
-  // it, with a copy of the candidate row (and of the diagonal row, if held here)
-  auto publish = [&](int jc, R best, int bidx) {
-    if (lane == jc) {
-      s_wv[warp] = best;
-      s_wi[warp] = bidx;
+  // a[i][k]: column jj + k of this thread's row i, jj the column at work.  The
+  // registers move down by one each column, so that one copy of the code serves
+  // all of them; finished columns are in shared memory.
+  T a[RPT][CB];
+  auto row_of = [&](int i) { return (warp * RPT + i) * 32 + lane; };  // local row i of this thread
+  auto owner_warp = [&](int r) { return r / (32 * RPT); };
+  // local row r whole, lane = column, in its owner's warp: the block's columns
+  // [jj, end) from the owner's registers, the others from shared memory
+  auto row_values = [&](int r, int jj, int end) -> T {
+    T v = sA[r * SP + col];
+    const int src = r & 31;
+    const bool second = RPT == 2 && (r >> 5 & 1);
+#pragma unroll
+    for (int k = 0; k < CB; k++) {
+      const T x = second ? a[RPT - 1][k] : a[0][k];
+      const T y = T{__shfl_sync(0xffffffffu, x.x, src), __shfl_sync(0xffffffffu, x.y, src)};
+      if (lane == jj + k && lane < end) v = y;
     }
-    __syncthreads();
-    if (warp == 0) {
-      R v = lane < NW ? s_wv[lane] : R(-1);
-      int i = lane < NW ? s_wi[lane] : -1;
-      warp_argmax<NW>(v, i);
-      i = __shfl_sync(0xffffffffu, i, 0);  // lanes >= NW reduced only among themselves
-      const int buf = jc & 1, j = c0 + jc;
-      if (lane == 0 && i >= 0) atomicMax(&keys[j], pivot_key((double)v, i - c0));
-      if (i >= 0 && lane < w) scr.row[((size_t)buf * G + blockIdx.x) * IB + lane] = sA[(i - lo) * SP + lane];
-      if (j >= lo && j < hi && lane < w) top[buf * IB + lane] = sA[(j - lo) * SP + lane];
+    return v;
+  };
+  // local row r replaced, in its owner's warp
+  auto set_row = [&](int r, const T* row, int jj) {
+    if (lane < w) sA[r * SP + lane] = row[lane];
+#pragma unroll
+    for (int i = 0; i < RPT; i++)
+      if (row_of(i) == r)
+#pragma unroll
+        for (int k = 0; k < CB; k++) a[i][k] = row[jj + k];
+  };
+  auto load_block = [&](int b0) {
+#pragma unroll
+    for (int i = 0; i < RPT; i++)
+#pragma unroll
+      for (int k = 0; k < CB; k++) {
+        a[i][k] = T{0, 0};
+        if (!helper && row_of(i) < nr && b0 + k < w) a[i][k] = sA[row_of(i) * SP + b0 + k];
+      }
+  };
+  // poll until every lane's record is this column's, at most LL_SPINS times
+  auto wait_row = [&](const unsigned char* p, unsigned tag, T& v, unsigned long long& hi) {
+    for (int spin = 0;; spin++) {
+      const bool ok = LL<T>::poll(p, v, hi, tag);
+      if (__all_sync(0xffffffffu, ok)) return;
+      if (spin >= LL_SPINS || *(volatile int*)sFlag) {
+        if (lane == 0) {
+          *(volatile int*)sFlag = 1;
+          atomicExch(bt.err, 1);
+        }
+        return;
+      }
     }
   };
-  // candidate of column jc over its rows without an update (first column, or
-  // after a zero pivot)
-  auto scan = [&](int jc) {
-    R best = -1;
-    int bidx = -1;
-    for (int r = max(0, c0 + jc - lo) + warp; r < nr; r += NW) {
-      if (lane == jc) {
-        const T v = sA[r * SP + jc];
-        const R a = fabs(v.x) + fabs(v.y);
-        if (a > best) {
-          best = a;
-          bidx = lo + r;
-        }
-      }
-    }
-    publish(jc, best, bidx);
-  };
-  scan(0);
-  for (int jj = 0; jj < w; jj++) {
-    const int j = c0 + jj;
-    const int buf = jj & 1;
-    grid.sync();
-    // warp 0: the column's pivot, then the winner's row and the diagonal row
-    if (warp == 0) {
-      unsigned long long k = 0;
-      if (lane == 0) k = __ldcg(&keys[j]);
-      k = __shfl_sync(0xffffffffu, k, 0);
-      const bool zero = (k >> 20) == 0;
-      const int piv = zero ? j : c0 + (0xFFFFF - (int)(k & 0xFFFFF));
-      if (lane == 0) {
-        s_zero = zero;
-        if (cta == 0) {
-          ipiv[j] = piv;
-          if (zero && bt.info[grp] == 0) bt.info[grp] = j + 1;
-        }
-      }
-      if (!zero && lane < w) {
-        const int owner = grp * Gb + (piv - c0) / chunk;
-        const T pr = scr.row[((size_t)buf * G + owner) * IB + lane];
-        const T tp = top[buf * IB + lane];
-        s_prow[lane] = pr;
-        if (piv != j && piv >= lo && piv < hi) sA[(piv - lo) * SP + lane] = tp;
-        if (j >= lo && j < hi) sA[(j - lo) * SP + lane] = pr;
-      }
-    }
-    __syncthreads();
-    if (s_zero) {
-      // singular column: nothing to eliminate; the next column's candidate
-      if (jj + 1 < w) scan(jj + 1);
-      continue;
-    }
-    const T d = s_prow[jj];
-    T rd;
-    rd.x = 1;
-    rd.y = 0;
-    rd = cdiv_smith(rd, d);
-    const T u = lane < w ? s_prow[lane] : T{0, 0};
-    const int jn = jj + 1;
-    R best = -1;
-    int bidx = -1;
-    // four rows per warp per iteration, independent, for latency hiding
-    constexpr int RU = 4;
-    for (int rb = max(0, j + 1 - lo) + warp; rb < nr; rb += NW * RU) {
-      T a[RU];
+  const bool one_hop = Gb <= LL_ONE_HOP && Gb < LL_PER_WARP * NW;
+  load_block(0);
+  for (int b0 = 0; b0 < w; b0 += CB) {
+    const int end = min(b0 + CB, w);
+#pragma unroll 1
+    for (int jj = b0; jj < end; jj++) {
+      const int buf = jj & 1;
+      const unsigned tag = (unsigned)(c0 + jj) + 1u;
+      Key* kOwn = sKey + buf * 2 * SP_WARPS;
+      Key* kAll = kOwn + SP_WARPS;
+      int* iOwn = sIdx + buf * 2 * SP_WARPS;
+      int* iAll = iOwn + SP_WARPS;
+      T* rows = sRow + buf * SP_WARPS * RW;
+      T* top = sTop + buf * RW;
+      // ---- this CTA's candidate among its rows from the diagonal on
+      Key key = 0;
+      int idx = NONE;
+      if (!helper) {
 #pragma unroll
-      for (int k = 0; k < RU; k++) {
-        const int r = rb + k * NW;
-        a[k] = (r < nr && lane >= jj && lane < w) ? sA[r * SP + lane] : T{0, 0};  // columns < jj are final
-      }
-#pragma unroll
-      for (int k = 0; k < RU; k++) {
-        T p, l;
-        p.x = __shfl_sync(0xffffffffu, a[k].x, jj);
-        p.y = __shfl_sync(0xffffffffu, a[k].y, jj);
-        l.x = p.x * rd.x - p.y * rd.y;
-        l.y = p.x * rd.y + p.y * rd.x;
-        if (lane == jj) {
-          a[k] = l;
-        } else {
-          a[k].x -= l.x * u.x - l.y * u.y;
-          a[k].y -= l.x * u.y + l.y * u.x;
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < RU; k++) {
-        const int r = rb + k * NW;
-        if (r < nr) {
-          if (lane >= jj && lane < w) sA[r * SP + lane] = a[k];
-          if (lane == jn) {
-            const R av = fabs(a[k].x) + fabs(a[k].y);
-            if (av > best) {
-              best = av;
-              bidx = lo + r;
+        for (int i = 0; i < RPT; i++) {
+          const int r = row_of(i);
+          if (r < nr && lo + r >= jj) {
+            const Key k = pivot_key(a[i][0]);
+            if (k > key) {
+              key = k;
+              idx = lo + r;
             }
+          }
+        }
+        warp_best(key, idx);
+        if (lane == 0) {
+          kOwn[warp] = key;
+          iOwn[warp] = idx;
+        }
+      }
+      __syncthreads();
+      key = lane < NWR ? kOwn[lane] : Key(0);
+      idx = lane < NWR ? iOwn[lane] : NONE;
+      warp_best(key, idx);
+      const bool have = key != 0;
+      const bool diag_best = cta == 0 && have && idx == jj;  // one row to post, as candidate and diagonal row
+      if (warp == (have ? owner_warp(idx - lo) : 0)) {
+        T v = T{0, 0};
+        if (have) v = row_values(idx - lo, jj, end);
+        if (Gb > 1) {
+          LL<T>::post(slot(buf, cta) + lane * LL<T>::BYTES, v,
+                      (unsigned long long)tag | ((unsigned long long)(unsigned)(have ? idx : NONE) << 32));
+        } else {
+          rows[lane] = v;
+        }
+        if (diag_best) {
+          if (Gb > 1) LL<T>::post(slot(buf, Gb) + lane * LL<T>::BYTES, v, tag);
+          else top[lane] = v;
+        }
+      }
+      if (cta == 0 && !diag_best && warp == owner_warp(jj)) {
+        const T v = row_values(jj, jj, end);
+        if (Gb > 1) LL<T>::post(slot(buf, Gb) + lane * LL<T>::BYTES, v, tag);
+        else top[lane] = v;
+      }
+      // ---- the column's pivot row and the diagonal row, from all CTAs
+      if (Gb > 1) {
+        Key bk = 0;
+        int bi = NONE;
+        if (one_hop) {
+          // all of this warp's slots are asked for before the first is waited for
+          T v[LL_PER_WARP], bv = T{0, 0};
+          unsigned long long hi[LL_PER_WARP];
+          bool ok[LL_PER_WARP];
+#pragma unroll
+          for (int k = 0; k < LL_PER_WARP; k++) {
+            const int g = warp + k * NW;
+            ok[k] = true;
+            if (g <= Gb) ok[k] = LL<T>::poll(slot(buf, g) + lane * LL<T>::BYTES, v[k], hi[k], tag);
+          }
+#pragma unroll
+          for (int k = 0; k < LL_PER_WARP; k++) {
+            const int g = warp + k * NW;
+            if (g <= Gb) {
+              if (!__all_sync(0xffffffffu, ok[k])) {
+                T tv;
+                unsigned long long th;
+                wait_row(slot(buf, g) + lane * LL<T>::BYTES, tag, tv, th);
+                v[k] = tv;
+                hi[k] = th;
+              }
+              if (g == Gb) {
+                top[lane] = v[k];
+              } else {
+                const int gi = (int)(hi[k] >> 32);
+                T d;
+                d.x = __shfl_sync(0xffffffffu, v[k].x, jj);
+                d.y = __shfl_sync(0xffffffffu, v[k].y, jj);
+                const Key gk = gi != NONE ? pivot_key(d) : Key(0);
+                if (gk > bk || (gk == bk && gi < bi)) {
+                  bk = gk;
+                  bi = gi;
+                  bv = v[k];
+                }
+              }
+            }
+          }
+          rows[warp * RW + lane] = bv;
+        } else if (helper) {
+          T v;
+          unsigned long long hi;
+          wait_row(slot(buf, Gb) + lane * LL<T>::BYTES, tag, v, hi);
+          top[lane] = v;
+        } else {
+          for (int g0 = warp * 32; g0 < Gb; g0 += NWR * 32) {
+            const int g = min(g0 + lane, Gb - 1);
+            T v;
+            unsigned long long hi;
+            wait_row(slot(buf, g) + jj * LL<T>::BYTES, tag, v, hi);
+            const int gi = (int)(hi >> 32);
+            const Key gk = gi != NONE ? pivot_key(v) : Key(0);
+            if (gk > bk || (gk == bk && gi < bi)) {
+              bk = gk;
+              bi = gi;
+            }
+          }
+          warp_best(bk, bi);
+        }
+        if (lane == 0) {
+          kAll[warp] = bk;
+          iAll[warp] = bi;
+        }
+      }
+      __syncthreads();
+      int ww = 0;
+      if (Gb > 1) {
+        key = lane < NW ? kAll[lane] : Key(0);
+        idx = lane < NW ? iAll[lane] : NONE;
+        ww = warp_best(key, idx);
+        if (!one_hop) {
+          // the second trip: one warp fetches the winner's row (more readers of
+          // these few lines of L2 make it slower)
+          if (helper && key != 0) {
+            T v;
+            unsigned long long hi;
+            wait_row(slot(buf, min(idx / chunk, Gb - 1)) + lane * LL<T>::BYTES, tag, v, hi);
+            rows[ww * RW + lane] = v;
+          }
+          __syncthreads();
+        }
+      }
+      const bool zero = key <= 1;  // no candidate, or a column of zeros
+      const int piv = zero ? jj : min(idx, m - 1);  // within the matrix whatever a run-out wait left
+      const T* prow = zero ? top : rows + ww * RW;
+      if (helper) {
+        // the pivot row solved with the block's earlier pivots, for the columns right of the block
+        T v = prow[lane], us[CB];
+        load_u(sU + lane * CB, us);
+#pragma unroll
+        for (int d = 0; d < CB; d++) {
+          const T l = prow[b0 + d];
+          if (d < jj - b0) {
+            v.x -= l.x * us[d].x - l.y * us[d].y;
+            v.y -= l.x * us[d].y + l.y * us[d].x;
+          }
+        }
+        sU[lane * CB + jj - b0] = v;
+        if (lane == 0) {
+          sPiv[jj] = c0 + piv;
+          if (cta == 0 && zero && bt.info[grp] == 0) bt.info[grp] = c0 + jj + 1;
+        }
+        continue;
+      }
+      // ---- interchange
+      if (piv != jj) {
+        const int rp = piv - lo;
+        if (rp >= 0 && rp < nr && warp == owner_warp(rp)) set_row(rp, top, jj);
+        if (cta == 0 && warp == owner_warp(jj)) set_row(jj, prow, jj);
+      }
+      // ---- eliminate within the block; column jj goes to shared memory
+      const T rd = pivot_recip(prow[jj]);
+      T u[CB];
+#pragma unroll
+      for (int k = 1; k < CB; k++) u[k] = prow[jj + k];
+#pragma unroll
+      for (int i = 0; i < RPT; i++) {
+        const int r = row_of(i);
+        const bool on = r < nr && lo + r > jj && !zero;
+        T l = T{0, 0};
+        if (on) {
+          l.x = a[i][0].x * rd.x - a[i][0].y * rd.y;
+          l.y = a[i][0].x * rd.y + a[i][0].y * rd.x;
+        }
+        if (r < nr) sA[r * SP + jj] = on ? l : a[i][0];
+#pragma unroll
+        for (int k = 1; k < CB; k++) {
+          a[i][k - 1] = a[i][k];
+          if (on) {
+            a[i][k - 1].x -= l.x * u[k].x - l.y * u[k].y;
+            a[i][k - 1].y -= l.x * u[k].y + l.y * u[k].x;
           }
         }
       }
     }
-    if (jn < w) publish(jn, best, bidx);
+    // ---- the columns right of the block take its CB pivots
+    __syncthreads();
+    if (!helper && b0 + CB < w) {
+      // (a block followed by another has all its CB columns)
+      T l[RPT][CB];
+#pragma unroll
+      for (int i = 0; i < RPT; i++)
+#pragma unroll
+        for (int c = 0; c < CB; c++) l[i][c] = row_of(i) < nr ? sA[row_of(i) * SP + b0 + c] : T{0, 0};
+      // QU columns at a time: independent chains, since few warps share a scheduler
+      constexpr int QU = 4;
+      for (int q0 = b0 + CB; q0 < w; q0 += QU) {
+        T v[RPT][QU];
+#pragma unroll
+        for (int i = 0; i < RPT; i++)
+#pragma unroll
+          for (int j = 0; j < QU; j++) v[i][j] = row_of(i) < nr ? sA[row_of(i) * SP + min(q0 + j, IB)] : T{0, 0};
+#pragma unroll
+        for (int j = 0; j < QU; j++) {
+          T us[CB];
+          load_u(sU + min(q0 + j, IB - 1) * CB, us);
+#pragma unroll
+          for (int i = 0; i < RPT; i++)
+#pragma unroll
+            for (int c = 0; c < CB; c++) {
+              v[i][j].x -= l[i][c].x * us[c].x - l[i][c].y * us[c].y;
+              v[i][j].y -= l[i][c].x * us[c].y + l[i][c].y * us[c].x;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < RPT; i++) {
+          const int r = row_of(i), gr = lo + r;
+          if (r >= nr || gr < b0) continue;
+#pragma unroll
+          for (int j = 0; j < QU; j++)
+            if (q0 + j < w)  // a pivot row of this block takes its solved values
+              sA[r * SP + q0 + j] = gr < b0 + CB ? sU[(q0 + j) * CB + gr - b0] : v[i][j];
+        }
+      }
+      load_block(b0 + CB);
+    }
   }
   __syncthreads();
   for (int r = warp; r < nr; r += NW)
-    if (lane < w) A[(size_t)(lo + r) * n + c0 + lane] = sA[r * SP + lane];
+    if (lane < w) A[(size_t)(c0 + lo + r) * n + c0 + lane] = sA[r * SP + lane];
+  if (cta == 0 && tid < w) batch_pick(bt.ipiv, grp)[c0 + tid] = sPiv[tid];
   if (pk1 - pk0 > w) {
-    // every column's pivot is in ipiv once all blocks passed this barrier
-    grid.sync();
+    const unsigned moves = __ballot_sync(0xffffffffu, lane < w && sPiv[col] != c0 + lane);
     const int nl = c0 - pk0, nc = nl + (pk1 - (c0 + w));
-    for (int t = cta * SP_THREADS + threadIdx.x; t < nc; t += Gb * SP_THREADS) {
-      const int c = t < nl ? pk0 + t : c0 + w + (t - nl);
-      for (int jj = 0; jj < w; jj++) {
-        const int j = c0 + jj, p = __ldcg(&ipiv[j]);
-        if (p != j) {
-          const T a = A[(size_t)j * n + c];
-          A[(size_t)j * n + c] = A[(size_t)p * n + c];
-          A[(size_t)p * n + c] = a;
-        }
+    for (int t = cta * blockDim.x + tid; t < nc; t += Gb * blockDim.x) {
+      const int q = t < nl ? pk0 + t : c0 + w + (t - nl);
+      for (unsigned left = moves; left; left &= left - 1) {
+        const int jj = __ffs(left) - 1;
+        T* x = A + (size_t)(c0 + jj) * n + q;
+        T* y = A + (size_t)sPiv[jj] * n + q;
+        const T v = *x;
+        *x = *y;
+        *y = v;
       }
     }
   }
@@ -874,32 +1180,50 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   DevBuf<double> sval;
   DevBuf<int> sidx, d_info;
   DevBuf<T> srow, stop;
-  DevBuf<unsigned long long> skey;
+  DevBuf<unsigned char> srec;
   TT_TRY(sval.alloc(2 * (size_t)G));
   TT_TRY(sidx.alloc(2 * (size_t)G));
   TT_TRY(srow.alloc(2 * (size_t)G * IB));
   TT_TRY(stop.alloc(2 * (size_t)kMaxBatch * IB));
-  TT_TRY(skey.alloc((size_t)B * n));
-  TT_TRY(d_info.alloc(B));
-  TT_CUDA_TRY(cudaMemsetAsync(d_info.ptr, 0, sizeof(int) * B, st));
-  TT_CUDA_TRY(cudaMemsetAsync(skey.ptr, 0, sizeof(unsigned long long) * B * n, st));
-  PivotScratch<T> scr{sval.ptr, sidx.ptr, srow.ptr, stop.ptr, skey.ptr};
-  TT_TRY(smem_limit_once((const void*)k_subpanel_smem<T>, (int)kSubpanelSmem));
-  // the sub-panel of matrices [b0, b0 + nb) in one cooperative launch
-  auto subpanel = [&](int b0, int nb, int j0, int w, int pk0, int pk1, int grid) -> int {
+  // records of B matrices in one launch, or of each matrix in its own: one
+  // region per matrix, since the matrices of separate launches share the tags
+  const size_t rec_region = 2 * ((size_t)G + kMaxBatch) * IB * LL<T>::BYTES, rec_bytes = rec_region * B;
+  TT_TRY(srec.alloc(rec_bytes));
+  TT_TRY(d_info.alloc(B + 1));  // [B] first zero pivots, then the sub-panels' error word
+  TT_CUDA_TRY(cudaMemsetAsync(d_info.ptr, 0, sizeof(int) * (B + 1), st));
+  TT_CUDA_TRY(cudaMemsetAsync(srec.ptr, 0, rec_bytes, st));
+  PivotScratch<T> scr{sval.ptr, sidx.ptr, srow.ptr, stop.ptr};
+  using SC = SubpanelCfg<T>;
+  // rows per thread: complex128 rows fill shared memory before they outnumber the threads
+  const void* sp_kernel[2] = {(const void*)k_subpanel_ll<T, 1>,
+                              sizeof(T) == 8 ? (const void*)k_subpanel_ll<T, sizeof(T) == 8 ? 2 : 1> : nullptr};
+  for (const void* k : sp_kernel)
+    if (k) TT_TRY(smem_limit_once(k, (int)kSubpanelSmem));
+  // CTAs of a matrix of m rows, of at most `most`: one while its shared memory
+  // holds them (no exchange through L2), else about SP_ROWS rows each; 0: too tall
+  auto ctas = [&](size_t m, int most) -> int {
+    const size_t need = (m + SC::MAX_ROWS - 1) / SC::MAX_ROWS;
+    if (need <= 1) return 1;
+    if (need > (size_t)most) return 0;
+    return (int)std::min<size_t>(most, std::max<size_t>(need, (m + SP_ROWS - 1) / SP_ROWS));
+  };
+  // the sub-panel of matrices [b0, b0 + nb) in one cooperative launch of gb CTAs each
+  auto subpanel = [&](int b0, int nb, int j0, int w, int pk0, int pk1, int gb) -> int {
     SubpanelBatch<T> bt{};
     for (int b = 0; b < nb; b++) {
       bt.A[b] = As[b0 + b];
       bt.ipiv[b] = ipivs[b0 + b];
-      bt.key[b] = skey.ptr + (size_t)(b0 + b) * n;
     }
     bt.info = d_info.ptr + b0;
+    bt.err = d_info.ptr + B;
     bt.B = nb;
     int nn = n, cc0 = j0, ww = w, p0 = pk0, p1 = pk1;
-    void* args[] = {&bt, &nn, &cc0, &ww, &p0, &p1, &scr};
-    const size_t chunk = (size_t)(n - j0 + grid / nb - 1) / (grid / nb);
-    TT_CUDA_TRY(cudaLaunchCooperativeKernel((void*)k_subpanel_smem<T>, dim3(grid), dim3(SP_THREADS), args,
-                                            chunk * SP * sizeof(T), st));
+    unsigned char* rec = srec.ptr + rec_region * b0;
+    void* args[] = {&bt, &nn, &cc0, &ww, &p0, &p1, &rec};
+    const int chunk = (n - j0 + gb - 1) / gb;
+    TT_CUDA_TRY(cudaLaunchCooperativeKernel((void*)sp_kernel[sp_rpt(chunk) - 1], dim3(gb * nb),
+                                            dim3(sp_threads(chunk)), args, (size_t)chunk * SP * sizeof(T) + SC::EXTRA,
+                                            st));
     count_launch();
     return TT_OK;
   };
@@ -907,15 +1231,12 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   // with its interchanges applied to the panel's other columns [pk0, j0) and [j0 + w, pk1)
   auto leaf = [&](int j0, int w, int pk0, int pk1) -> int {
     const size_t m = (size_t)(n - j0);
-    const int Gb = G / B;
-    const bool keyed = m < 0xFFFFF;
-    const bool together = B > 1 && keyed && ((m + Gb - 1) / Gb) * SP * sizeof(T) <= kSubpanelSmem;
-    const bool alone = keyed && ((m + G - 1) / G) * SP * sizeof(T) <= kSubpanelSmem;
+    const int together = ctas(m, G / B), alone = ctas(m, G);
     ProfScope prof(TT_PROF_SUBPANEL, st, 4.0 * m * w * w * B, 2.0 * m * w * sizeof(T) * B);
-    if (together) return subpanel(0, B, j0, w, pk0, pk1, Gb * B);
+    if (together) return subpanel(0, B, j0, w, pk0, pk1, together);
     for (int b = 0; b < B; b++) {
       if (alone) {
-        TT_TRY(subpanel(b, 1, j0, w, pk0, pk1, G));
+        TT_TRY(subpanel(b, 1, j0, w, pk0, pk1, alone));
       } else {
         T* Ap = As[b];
         int nn = n, cc0 = j0, ww = w;
@@ -1110,10 +1431,14 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   }
   if (mode == TC_LEGACY_BF16X3) TT_TRY(tc_check_error(st));
   if (mode == TC_TF32 || mode == TC_BF16X3) TT_TRY(tc2_check_error(st));
-  if (info) {
-    TT_CUDA_TRY(cudaMemcpyAsync(info, d_info.ptr, sizeof(int) * B, cudaMemcpyDeviceToHost, st));
-    TT_CUDA_TRY(cudaStreamSynchronize(st));
+  std::vector<int> h_info(B + 1);
+  TT_CUDA_TRY(cudaMemcpyAsync(h_info.data(), d_info.ptr, sizeof(int) * (B + 1), cudaMemcpyDeviceToHost, st));
+  TT_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h_info[B]) {
+    set_error("sub-panel factorisation timed out waiting for a pivot row");
+    return TT_ERR_CUDA;
   }
+  if (info) std::copy(h_info.begin(), h_info.begin() + B, info);
   return TT_OK;
 }
 template int lu_factor_batched_device<double2>(double2* const*, int, int, int32_t* const*, cudaStream_t, int, int*,
