@@ -248,8 +248,10 @@ const char* tt_last_error_string(void);
 int tt_device_count(int* count);
 /* Large device blocks (256 MB and up) that the library releases are kept for
  * its next allocations of about the same size (cudaMalloc / cudaFree of tens
- * of GB cost milliseconds each); this returns the current device's cached
- * blocks to the driver.  tt_run_destroy does the same. */
+ * of GB cost milliseconds each), and smaller ones in a stream-ordered pool that
+ * keeps up to 1 GB of idle memory; this returns the current device's cached
+ * blocks and the pool's idle memory to the driver.  tt_run_destroy returns the
+ * blocks too; an allocation that would fail returns both first. */
 int tt_release_cached_device_memory(void);
 /* Bytes of those blocks currently held for the current device. */
 int tt_cached_device_memory(size_t* bytes);

@@ -96,3 +96,35 @@ def test_zero_column_is_reported_singular(precision, i0):
         tt.solve_faddeev(G, np.ones(n), np.arange(n, dtype=np.int32), np.arange(n + 1, dtype=np.uint64), eye, None, swp,
                          [3], [1], tt.PW(pw), precision=precision, tensor_force=0, isospin_breaking_1S0=0)
     assert err.value.code == tt.TT_ERR_SINGULAR and f"column {i0 + 1} " in str(err.value)
+
+
+def test_buffers_of_concurrent_threads():
+    # every thread works on a stream of its own; buffers released on one stream
+    # are reused on others, and each result must equal the single-threaded one
+    import threading
+
+    opts = [dict(potential_model="LO_internal", J_2N_max=1, two_J_3N_max=1, Np_WP=8 + k, Nq_WP=9, Nphi=12, Nx=12,
+                 lab_energies="5,30") for k in range(3)]
+
+    def work(k, out):
+        run = tt.Run(**opts[k])
+        for prec in (tt.PRECISION_MIXED, tt.PRECISION_FP64):
+            out.append(run.solve(1, prec)[0])
+        run.release(1)
+        out.append(run.solve(1, tt.PRECISION_MIXED)[0])
+        run.close()
+
+    alone = [[] for _ in opts]
+    for k in range(len(opts)):
+        work(k, alone[k])
+    together = [[] for _ in range(2 * len(opts))]
+    threads = [threading.Thread(target=work, args=(i % len(opts), together[i])) for i in range(len(together))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i, got in enumerate(together):
+        for a, b in zip(alone[i % len(opts)], got, strict=True):
+            assert np.array_equal(a, b), i
+    tt.release_cached_device_memory()
+    assert tt.cached_device_memory() == 0

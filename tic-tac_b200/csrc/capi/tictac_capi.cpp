@@ -186,6 +186,7 @@ int dropin_solve(tt_complex* U, tt_complex* dU, int n_theta, const double* dVu, 
   const int n = ch.Nalpha * w.Np_WP * w.Nq_WP;
   if (P_colptr[n] != P_nnz) return fail(TT_ERR_BADARG, "P123 column pointers do not end at nnz");
   cudaStream_t st = default_stream();
+  StreamScope scope(st);
   ChannelSolver cs;
   int s = cs.setup(L, w.q_WP, st);
   if (s != TT_OK) return s;
@@ -314,6 +315,7 @@ int tt_fill_P123_arrays(double** val, int** row, int** col, size_t* nnz, int pro
   std::string err;
   if (!p123_prepare(rp, f, view_of(pw), t, &err)) return fail(TT_ERR_BADARG, err);
   cudaStream_t st = default_stream();
+  StreamScope scope(st);
   DeviceCSR P;
   int s = p123_build_device(t, P, st, nullptr);
   if (s != TT_OK) return s;
@@ -351,6 +353,7 @@ int tt_calculate_resolvent_array_in_SWP_basis(tt_complex* G, double E, const tt_
   std::string err;
   if (!build_channel_layout(rp, view_of(pw), w, Vu, Vc, L, &err)) return fail(TT_ERR_BADARG, err);
   cudaStream_t st = default_stream();
+  StreamScope scope(st);
   ChannelSolver cs;
   int s = cs.setup(L, w.q_WP, st);
   if (s != TT_OK) return s;
@@ -446,6 +449,7 @@ int tt_run_create(tt_run** out, int nopt, const char* const* opts) {
 
 int tt_release_cached_device_memory(void) {
   device_cache_trim();
+  device_pool_trim(0);
   return TT_OK;
 }
 
@@ -471,7 +475,10 @@ int tt_run_set_solve_option(tt_run* run, const char* key, const char* value) {
 
 void tt_run_destroy(tt_run* run) {
   if (!run) return;
-  run->chn.clear();
+  {
+    StreamScope scope(run->stream);
+    run->chn.clear();
+  }
   device_cache_trim();
   if (run->ev0) cudaEventDestroy(run->ev0);
   if (run->ev1) cudaEventDestroy(run->ev1);
@@ -593,6 +600,7 @@ static int ensure_solver(tt_run* run, int chn) {
 int tt_run_build_P123(tt_run* run, int chn, int64_t* nnz) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   // calculate_and_store_P123 = false: the reference reads the channel's file
   // instead of computing P123 (CPP/make_permutation_matrix.cpp:1387-1403)
   if (!run->rp.calculate_and_store_P123) return tt_run_load_P123_h5(run, chn, nullptr, nnz);
@@ -611,6 +619,7 @@ int tt_run_build_P123(tt_run* run, int chn, int64_t* nnz) {
 int tt_run_build_A(tt_run* run, int chn, double* ms) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   if (!run->chn[chn].have_P) TT_TRY(tt_run_build_P123(run, chn, nullptr));
   TT_TRY(run->chn[chn].solver->build_A(run_stream(run), ms));
   run->chn[chn].have_A = true;
@@ -620,6 +629,7 @@ int tt_run_build_A(tt_run* run, int chn, double* ms) {
 int tt_run_build_resolvent(tt_run* run, int chn) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   TT_TRY(ensure_solver(run, chn));
   std::vector<double> E;
   for (double e : run->os.E_com) E.push_back(e + run->swp.E_bound);  // CPP/main.cpp:391
@@ -631,6 +641,7 @@ int tt_run_build_resolvent(tt_run* run, int chn) {
 int tt_run_solve(tt_run* run, int chn, int precision, tt_complex* U, tt_solve_report* report) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   if (!U) return fail(TT_ERR_BADARG, "null U");
   if (precision < TT_PRECISION_FP64 || precision > TT_PRECISION_PADE) return fail(TT_ERR_BADARG, "unknown precision");
   double msA = 0;
@@ -651,6 +662,7 @@ int tt_run_solve_energies(tt_run* run, int chn, int precision, int n_sel, const 
                           tt_solve_report* report) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   if (!U || n_sel < 0 || (n_sel > 0 && !energy_idx)) return fail(TT_ERR_BADARG, "null or negative argument");
   if (precision < TT_PRECISION_FP64 || precision > TT_PRECISION_PADE) return fail(TT_ERR_BADARG, "unknown precision");
   const int nE = (int)run->os.E_com.size();
@@ -683,6 +695,7 @@ int tt_run_solve_adjoint(tt_run* run, int chn, int precision, int n_theta, const
                          tt_complex* U, tt_complex* dU, tt_solve_report* report) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   if (!U || n_theta < 0 || (n_theta > 0 && (!dU || !dVu || (run->swp.n_coup && !dVc))))
     return fail(TT_ERR_BADARG, "null or negative argument");
   if (precision < TT_PRECISION_FP64 || precision > TT_PRECISION_PADE) return fail(TT_ERR_BADARG, "unknown precision");
@@ -711,6 +724,7 @@ int tt_run_solve_adjoint(tt_run* run, int chn, int precision, int n_theta, const
 int tt_run_adjoint_forward(tt_run* run, int chn, int precision, tt_complex* U, tt_solve_report* report) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   if (!U) return fail(TT_ERR_BADARG, "null U");
   if (precision != TT_PRECISION_FP64 && precision != TT_PRECISION_MIXED && precision != TT_PRECISION_MIXED_SIMT)
     return fail(TT_ERR_UNSUPPORTED, "the adjoint needs an LU precision");
@@ -734,6 +748,7 @@ int tt_run_adjoint_backward(tt_run* run, int chn, int n_theta, const double* dVu
                             const tt_complex* U_bar, double* theta_bar, tt_solve_report* report) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   if (n_theta < 0 || (n_theta > 0 && (!U_bar || !theta_bar || !dVu || (run->swp.n_coup && !dVc))))
     return fail(TT_ERR_BADARG, "null or negative argument");
   const int precision = run->chn[chn].fwd_precision;
@@ -820,6 +835,7 @@ int tt_run_lec_derivative(const tt_run* run, int k, double* dVu, double* dVc) {
 int tt_run_release_channel(tt_run* run, int chn) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run->stream);
   run->chn[chn] = ChannelState();
   return TT_OK;
 }
@@ -827,6 +843,7 @@ int tt_run_release_channel(tt_run* run, int chn) {
 int tt_run_release_A(tt_run* run, int chn) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run->stream);
   if (run->chn[chn].solver) run->chn[chn].solver->release_A();
   run->chn[chn].have_A = false;
   run->chn[chn].have_G = false;
@@ -1020,6 +1037,7 @@ int tt_run_breakup_cells(const tt_run* run, int chn, int* num_cells, int* start,
 int tt_run_solve_breakup(tt_run* run, int chn, tt_complex* U, tt_complex* U_BU, tt_solve_report* report) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   if (!U || !U_BU) return fail(TT_ERR_BADARG, "null U or U_BU");
   BreakupCells local;
   const BreakupCells* bu = nullptr;
@@ -1181,6 +1199,7 @@ int tt_run_store_P123_h5(const tt_run* run, int chn, const char* filename) {
 int tt_run_load_P123_h5(tt_run* run, int chn, const char* filename, int64_t* nnz) {
   int s = check_chn(run, chn);
   if (s) return s;
+  StreamScope scope(run_stream(run));
   const PWChannel c = channel_view(run->pw, chn);
   P123H5 want, got;
   s = p123_file_header(c, run->fwp.Np_WP, run->fwp.p_WP.data(), run->fwp.Nq_WP, run->fwp.q_WP.data(), want);

@@ -63,6 +63,33 @@ size_t device_cache_bytes();  // cached on the current device
 size_t device_cache_evict_one();  // frees the longest-held block; its bytes (0: none)
 void device_cache_trim();     // frees the current device's cached blocks
 
+// Smaller buffers come from a stream-ordered pool of the library's own per
+// device: a solve allocates and releases some forty of them, and cudaMalloc +
+// cudaFree took 45-100 us each (half of a solve of order 512, and waits for the
+// whole device).  The entry points open a StreamScope on the stream they work
+// on; a buffer released under a scope is freed in that stream's order, so it may
+// still be in use there, and the driver orders its reuse on other streams and
+// threads.  Every entry point waits for its stream before it returns, so a
+// buffer that outlives the call may next be used under another stream's scope.
+// Without a scope buffers are allocated with cudaMalloc and released with
+// cudaFree, which waits.  The pool keeps at most kPoolKeepBytes of idle memory;
+// device_pool_trim() (an allocation that would fail,
+// tt_release_cached_device_memory) gives idle memory back.
+constexpr size_t kPoolKeepBytes = size_t(1) << 30;
+struct StreamScope {
+  explicit StreamScope(cudaStream_t st);
+  ~StreamScope();
+  StreamScope(const StreamScope&) = delete;
+  StreamScope& operator=(const StreamScope&) = delete;
+
+ private:
+  cudaStream_t prev_;
+};
+cudaError_t device_pool_alloc(void** p, size_t bytes, bool* pooled);
+void device_pool_free(void* p);
+void device_pool_trim(size_t keep);
+size_t device_pool_idle_bytes();  // of the current device's pool
+
 // Owning device buffer.  alloc() reports NOMEM through the status path instead
 // of faulting.
 template <typename T>
@@ -70,10 +97,11 @@ struct DevBuf {
   T* ptr = nullptr;
   size_t count = 0;
   size_t cap = 0;  // bytes of the underlying block
+  bool pooled = false;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : ptr(o.ptr), count(o.count), cap(o.cap) {
+  DevBuf(DevBuf&& o) noexcept : ptr(o.ptr), count(o.count), cap(o.cap), pooled(o.pooled) {
     o.ptr = nullptr;
     o.count = 0;
     o.cap = 0;
@@ -84,6 +112,7 @@ struct DevBuf {
       ptr = o.ptr;
       count = o.count;
       cap = o.cap;
+      pooled = o.pooled;
       o.ptr = nullptr;
       o.count = 0;
       o.cap = 0;
@@ -93,12 +122,14 @@ struct DevBuf {
   ~DevBuf() { release(); }
   void release() {
     if (ptr) {
-      if (cap >= kCacheMinBytes) device_cache_give(ptr, cap);
+      if (pooled) device_pool_free(ptr);
+      else if (cap >= kCacheMinBytes) device_cache_give(ptr, cap);
       else cudaFree(ptr);
     }
     ptr = nullptr;
     count = 0;
     cap = 0;
+    pooled = false;
   }
   int alloc(size_t n) {
     release();
@@ -113,13 +144,25 @@ struct DevBuf {
         return TT_OK;
       }
     }
-    cudaError_t e = cudaMalloc((void**)&ptr, bytes);
-    while (e == cudaErrorMemoryAllocation && device_cache_evict_one() > 0) {
+    auto get = [&]() -> cudaError_t {
+      if (bytes < kCacheMinBytes) return device_pool_alloc((void**)&ptr, bytes, &pooled);
+      return cudaMalloc((void**)&ptr, bytes);
+    };
+    cudaError_t e = get();
+    bool trimmed = false;
+    while (e == cudaErrorMemoryAllocation) {
+      if (!trimmed) {
+        device_pool_trim(0);
+        trimmed = true;
+      } else if (device_cache_evict_one() == 0) {
+        break;
+      }
       cudaGetLastError();
-      e = cudaMalloc((void**)&ptr, bytes);
+      e = get();
     }
     if (e != cudaSuccess) {
       ptr = nullptr;
+      pooled = false;
       cudaGetLastError();
       set_error("device allocation of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
       return e == cudaErrorMemoryAllocation ? TT_ERR_NOMEM : TT_ERR_CUDA;

@@ -1,4 +1,4 @@
-// Cache of large device blocks behind DevBuf (see tt_device.h).
+// Cache of large device blocks and pool of small ones behind DevBuf (see tt_device.h).
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -27,7 +27,67 @@ int current_device() {
   return d;
 }
 
+// one pool per device, never destroyed (as the cache); null: not available
+cudaMemPool_t pool_of(int dev) {
+  static std::mutex* mu = new std::mutex;
+  static auto* pools = new std::map<int, cudaMemPool_t>;
+  std::lock_guard<std::mutex> lk(*mu);
+  const auto it = pools->find(dev);
+  if (it != pools->end()) return it->second;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    pool = nullptr;
+  } else {
+    unsigned long long keep = kPoolKeepBytes;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  pools->emplace(dev, pool);
+  return pool;
+}
+
+thread_local cudaStream_t g_scope = nullptr;
+
 }  // namespace
+
+StreamScope::StreamScope(cudaStream_t st) : prev_(g_scope) { g_scope = st; }
+StreamScope::~StreamScope() { g_scope = prev_; }
+
+cudaError_t device_pool_alloc(void** p, size_t bytes, bool* pooled) {
+  *pooled = false;
+  const cudaMemPool_t pool = g_scope ? pool_of(current_device()) : nullptr;
+  if (!pool) return cudaMalloc(p, bytes);
+  const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, g_scope);
+  *pooled = e == cudaSuccess;
+  return e;
+}
+
+void device_pool_free(void* p) {
+  if (g_scope && cudaFreeAsync(p, g_scope) == cudaSuccess) return;
+  cudaGetLastError();
+  cudaFree(p);
+}
+
+void device_pool_trim(size_t keep) {
+  const cudaMemPool_t pool = pool_of(current_device());
+  if (!pool) return;
+  // frees queued on a stream count once the stream has reached them
+  if (g_scope) cudaStreamSynchronize(g_scope);
+  cudaMemPoolTrimTo(pool, keep);
+}
+
+size_t device_pool_idle_bytes() {
+  const cudaMemPool_t pool = pool_of(current_device());
+  unsigned long long reserved = 0, used = 0;
+  if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return 0;
+  return reserved > used ? reserved - used : 0;
+}
 
 void* device_cache_take(size_t bytes, size_t* capacity) {
   std::lock_guard<std::mutex> lk(cache_mu());

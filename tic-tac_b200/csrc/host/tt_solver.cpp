@@ -555,7 +555,7 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
   if (opt.mixed && nE > 1 && opt.energy_batch > 1) {
     size_t free_b = 0, total_b = 0;
     TT_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    free_b += device_cache_bytes();  // cached blocks are freed when an allocation needs them
+    free_b += device_cache_bytes() + device_pool_idle_bytes();  // given back when an allocation needs them
     const size_t per = (size_t)n * n * sizeof(float2), reserve = (size_t)2 << 30;
     const size_t fit = free_b > reserve + per ? (free_b - reserve) / per : 1;
     B = (int)std::max<size_t>(1, std::min<size_t>(std::min<size_t>((size_t)nE, std::min(opt.energy_batch, 4)), fit));
