@@ -128,3 +128,28 @@ def test_buffers_of_concurrent_threads():
             assert np.array_equal(a, b), i
     tt.release_cached_device_memory()
     assert tt.cached_device_memory() == 0
+
+
+@pytest.mark.parametrize("Np,Nq,labs", [
+    (7, 5, "8"),          # n = 385: odd order, few slabs of rows
+    (6, 7, "5,30,100"),   # n = 462: five energies, on-shell rows in groups of 8 and less
+    (13, 11, "5,30"),     # n = 1,573: odd, more than one block of columns
+])
+def test_pade_series_and_transposed_products(Np, Nq, labs):
+    # TT_PRECISION_PADE against the oracle's restatement on the oracle's A and G, at
+    # the method's accuracy (its approximants differ by up to 1e-6 where they stop)
+    run = tt.Run(potential_model="LO_internal", J_2N_max=1, two_J_3N_max=1, Np_WP=Np, Nq_WP=Nq, Nphi=12, Nx=12,
+                 lab_energies=labs, chebyshev_s=150)
+    pw = run.host_array(0, 1).reshape(-1, 9)
+    T, E_com, q_idx = run.energies()
+    rowptr, col, val = run.P123_csr(1, run.build_P123(1))
+    rows = np.repeat(np.arange(len(rowptr) - 1, dtype=np.int32), np.diff(rowptr))
+    lay = oracle.layout(pw, Np, *[run.host_array(k) for k in range(3, 9)])
+    G = np.stack([oracle.resolvent(lay, pw.shape[0], Nq, Np, run.host_array(2), e + run.E_bound) for e in E_com])
+    A = oracle.build_A(lay, pw.shape[0], Nq, Np, rows, col, val)
+    U_o = oracle.pade_solve(A, G, q_idx, oracle.deuterons(pw), Nq, Np)
+    U, rep = run.solve(1, tt.PRECISION_PADE)
+    assert rel(U, U_o) <= 1e-5 and 1 <= rep["refine_iters"] <= 14
+    U2, _ = run.solve(1, tt.PRECISION_PADE)
+    assert np.array_equal(U, U2)  # no sum depends on the order of threads
+    run.close()

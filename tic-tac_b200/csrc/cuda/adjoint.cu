@@ -10,6 +10,8 @@
 // transposed solve with the stored LU factors (lu.cu), refined in FP64 through
 // y = A^T lambda for the mixed-precision factor.
 
+#include <algorithm>
+
 #include "tt_kernels.h"
 
 namespace tt {
@@ -39,42 +41,101 @@ __global__ void k_transpose_inplace(T* __restrict__ a, int n) {
   }
 }
 
-// y_k += A^T v_k for k < nrhs <= GT_MAXV: CTA = 256 columns x 256 rows of A,
-// one column per thread (coalesced rows), partial sums added atomically
-constexpr int GT_ROWS = 256;
-constexpr int GT_MAXV = 8;
-__global__ void __launch_bounds__(256) k_gemv_t(const double* __restrict__ A, int n, const double2* __restrict__ v,
-                                                int nrhs, double2* __restrict__ y) {
-  __shared__ double2 sv[GT_MAXV][GT_ROWS];
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  const int r0 = blockIdx.y * GT_ROWS, rn = min(GT_ROWS, n - r0);
-  for (int t = threadIdx.x; t < GT_MAXV * GT_ROWS; t += blockDim.x) {
-    const int k = t / GT_ROWS, i = t % GT_ROWS;
-    sv[k][i] = (k < nrhs && i < rn) ? v[(size_t)k * n + r0 + i] : make_double2(0, 0);
-  }
-  __syncthreads();
-  if (c >= n) return;
-  double ar[GT_MAXV], ai[GT_MAXV];
+// part[s][k] = A^T v_k over the rows of slab s = blockIdx.y, k < NV.  A thread owns
+// VEC columns (2 where rows are 16-byte aligned: even n); rows come GT_U at a time,
+// the next ones asked for before the present ones are used, against slices of v
+// in shared memory.  Bound: A read once.  Slabs, not atomics, collect the rows:
+// the sums come out the same every time.  n = 24,300, 4 vectors: 1.17 -> 0.70 ms
+// (6.7 TB/s; a column a thread with atomics before).
+constexpr int GT_MAXV = 8, GT_CHUNK = 128, GT_THREADS = 256;
+template <int NV, int VEC>
+__global__ void __launch_bounds__(GT_THREADS, 2) k_gemv_t(const double* __restrict__ A, int n, int slab,
+                                                          const double2* __restrict__ v, int nrhs,
+                                                          double2* __restrict__ part) {
+  constexpr int U = NV > 4 ? 4 : 8;
+  __shared__ double2 sv[GT_CHUNK][NV];
+  const int c = (blockIdx.x * GT_THREADS + threadIdx.x) * VEC;
+  const int r0 = blockIdx.y * slab, r1 = min(n, r0 + slab);
+  const bool in = c < n;
+  const double* Ac = A + (in ? c : 0);
+  double ar[VEC][NV], ai[VEC][NV];
 #pragma unroll
-  for (int k = 0; k < GT_MAXV; k++) ar[k] = ai[k] = 0;
-  const double* Ac = A + (size_t)r0 * n + c;
-  for (int i = 0; i < rn; i++) {
-    const double a = Ac[(size_t)i * n];
+  for (int x = 0; x < VEC; x++)
 #pragma unroll
-    for (int k = 0; k < GT_MAXV; k++) {
-      if (k < nrhs) {
-        ar[k] += a * sv[k][i].x;
-        ai[k] += a * sv[k][i].y;
+    for (int k = 0; k < NV; k++) ar[x][k] = ai[x][k] = 0.0;
+  double cur[U][VEC], nxt[U][VEC];
+  auto load = [&](int r, double(&d)[U][VEC]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const double* p = Ac + (size_t)min(r + u, n - 1) * n;
+      if constexpr (VEC == 2) {
+        const double2 t = __ldcs(reinterpret_cast<const double2*>(p));
+        d[u][0] = t.x;
+        d[u][1] = t.y;
+      } else {
+        d[u][0] = __ldcs(p);
+      }
+    }
+  };
+  load(r0, nxt);
+  for (int rb = r0; rb < r1; rb += GT_CHUNK) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < GT_CHUNK * NV; t += GT_THREADS) {
+      const int k = t / GT_CHUNK, i = t % GT_CHUNK;
+      sv[i][k] = (k < nrhs && rb + i < r1) ? v[(size_t)k * n + rb + i] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    const int rn = min(GT_CHUNK, r1 - rb);
+    for (int i = 0; i < rn; i += U) {
+#pragma unroll
+      for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int x = 0; x < VEC; x++) cur[u][x] = nxt[u][x];
+      load(rb + i + U, nxt);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+          const double2 s = sv[i + u][k];  // zero past the slab
+#pragma unroll
+          for (int x = 0; x < VEC; x++) {
+            ar[x][k] += cur[u][x] * s.x;
+            ai[x][k] += cur[u][x] * s.y;
+          }
+        }
       }
     }
   }
+  if (!in) return;
 #pragma unroll
-  for (int k = 0; k < GT_MAXV; k++) {
+  for (int k = 0; k < NV; k++)
     if (k < nrhs) {
-      atomicAdd(&y[(size_t)k * n + c].x, ar[k]);
-      atomicAdd(&y[(size_t)k * n + c].y, ai[k]);
+      double2* o = part + ((size_t)blockIdx.y * nrhs + k) * n + c;
+#pragma unroll
+      for (int x = 0; x < VEC; x++) o[x] = make_double2(ar[x][k], ai[x][k]);
     }
+}
+
+// y = sum over the slabs, in order
+__global__ void k_sum_slabs(const double2* __restrict__ part, int slabs, size_t total, double2* __restrict__ y) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  double2 s = part[t];
+  for (int i = 1; i < slabs; i++) {
+    const double2 p = part[(size_t)i * total + t];
+    s.x += p.x;
+    s.y += p.y;
   }
+  y[t] = s;
+}
+
+template <int NV>
+void launch_gemv_t(const double* A, int n, int slab, int slabs, const double2* v, int nrhs, double2* part,
+                   cudaStream_t st) {
+  if (n % 2 == 0)
+    k_gemv_t<NV, 2><<<dim3(ceil_div(n, 2 * GT_THREADS), slabs), GT_THREADS, 0, st>>>(A, n, slab, v, nrhs, part);
+  else
+    k_gemv_t<NV, 1><<<dim3(ceil_div(n, GT_THREADS), slabs), GT_THREADS, 0, st>>>(A, n, slab, v, nrhs, part);
 }
 
 // r_k = e_{rows[k]} - lam_k + G o y_k
@@ -239,13 +300,6 @@ __global__ void k_scale_rows(const double2* __restrict__ R, const double2* __res
   V[t] = make_double2(r.x * g.x - r.y * g.y, r.x * g.y + r.y * g.x);
 }
 
-// out[i] = R[src_row[i]][src_col[i]]
-__global__ void k_pick(const double2* __restrict__ R, int n, const int32_t* __restrict__ src_row,
-                       const int32_t* __restrict__ src_col, int m, double2* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m) out[i] = R[(size_t)src_row[i] * n + src_col[i]];
-}
-
 }  // namespace
 
 int gather_rows_device(const double* d_A, int n, const int32_t* d_rows, int nrows, double* d_R, cudaStream_t st) {
@@ -260,16 +314,6 @@ int scale_rows_device(const double* d_R, const double* d_G, const int32_t* d_e, 
   k_scale_rows<<<ceil_div((size_t)n * nrows, 256), 256, 0, st>>>(reinterpret_cast<const double2*>(d_R),
                                                                  reinterpret_cast<const double2*>(d_G), d_e, n, nrows,
                                                                  reinterpret_cast<double2*>(d_V));
-  count_launch();
-  TT_CUDA_TRY(cudaGetLastError());
-  return TT_OK;
-}
-
-int pick_device(const double* d_R, int n, const int32_t* d_row, const int32_t* d_col, int m, double* d_out,
-                cudaStream_t st) {
-  if (m <= 0) return TT_OK;
-  k_pick<<<ceil_div(m, 128), 128, 0, st>>>(reinterpret_cast<const double2*>(d_R), n, d_row, d_col, m,
-                                           reinterpret_cast<double2*>(d_out));
   count_launch();
   TT_CUDA_TRY(cudaGetLastError());
   return TT_OK;
@@ -291,10 +335,25 @@ int gemv_t_device(const double* d_A, int n, const double* d_v, int nrhs, double*
     set_error("A^T products take at most 8 vectors per call");
     return TT_ERR_BADARG;
   }
+  if (n <= 0 || nrhs <= 0) return TT_OK;
   ProfScope prof(TT_PROF_RESIDUAL, st, 4.0 * n * (double)n * nrhs, 8.0 * n * (double)n);
-  TT_CUDA_TRY(cudaMemsetAsync(d_y, 0, sizeof(double2) * (size_t)n * nrhs, st));
-  dim3 grid(ceil_div(n, 256), ceil_div(n, GT_ROWS));
-  k_gemv_t<<<grid, 256, 0, st>>>(d_A, n, reinterpret_cast<const double2*>(d_v), nrhs, reinterpret_cast<double2*>(d_y));
+  // two CTAs an SM, twice over: that many slabs, of at least 64 rows
+  const int blocks = ceil_div(n, (n % 2 == 0 ? 2 : 1) * GT_THREADS);
+  int slabs = std::max(1, std::min(4 * device_sm_count() / blocks, (n + 63) / 64));
+  const int slab = (ceil_div(n, slabs) + 7) / 8 * 8;
+  slabs = ceil_div(n, slab);
+  DevBuf<double> part;
+  TT_TRY(part.alloc((size_t)2 * n * nrhs * slabs));
+  const double2* v = reinterpret_cast<const double2*>(d_v);
+  double2* pt = reinterpret_cast<double2*>(part.ptr);
+  if (nrhs <= 2) launch_gemv_t<2>(d_A, n, slab, slabs, v, nrhs, pt, st);
+  else if (nrhs <= 4) launch_gemv_t<4>(d_A, n, slab, slabs, v, nrhs, pt, st);
+  else if (nrhs <= 6) launch_gemv_t<6>(d_A, n, slab, slabs, v, nrhs, pt, st);
+  else launch_gemv_t<8>(d_A, n, slab, slabs, v, nrhs, pt, st);
+  count_launch();
+  TT_CUDA_TRY(cudaGetLastError());
+  const size_t total = (size_t)n * nrhs;
+  k_sum_slabs<<<ceil_div(total, 256), 256, 0, st>>>(pt, slabs, total, reinterpret_cast<double2*>(d_y));
   count_launch();
   TT_CUDA_TRY(cudaGetLastError());
   return TT_OK;

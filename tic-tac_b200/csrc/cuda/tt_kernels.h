@@ -140,13 +140,29 @@ template <typename T>
 int transpose_inplace_device(T* a, int n, cudaStream_t st);
 // y_k = A^T v_k, k < nrhs <= 8
 int gemv_t_device(const double* d_A, int n, const double* d_v, int nrhs, double* d_y, cudaStream_t st);
-// Pade path (adjoint.cu): R[k] = A[rows[k], :] as complex; V[k] = R[k] o G[e[k]];
-// out[i] = R[row[i]][col[i]]
+// Pade path (adjoint.cu): R[k] = A[rows[k], :] as complex; V[k] = R[k] o G[e[k]]
 int gather_rows_device(const double* d_A, int n, const int32_t* d_rows, int nrows, double* d_R, cudaStream_t st);
 int scale_rows_device(const double* d_R, const double* d_G, const int32_t* d_e, int n, int nrows, double* d_V,
                       cudaStream_t st);
-int pick_device(const double* d_R, int n, const int32_t* d_row, const int32_t* d_col, int m, double* d_out,
-                cudaStream_t st);
+// The Neumann coefficients of nel elements R[row[e]][col[e]] and their Pade
+// approximants (pade.cu): term() takes coefficient t of the open elements from R,
+// order() forms the [N/N] approximants (coefficients 0 .. 2 N known) and returns
+// how many elements remain open, result() the chosen approximants and their
+// relative differences once none does (at order 14 at the latest).
+struct PadeSeries {
+  static constexpr int kMaxOrder = 14;
+  int nel = 0;
+  int init(const std::vector<int32_t>& row, const std::vector<int32_t>& col, cudaStream_t st);
+  int term(const double* d_R, int n, int t, cudaStream_t st);
+  int order(int N, int* open, cudaStream_t st);
+  int result(std::vector<double>& out, std::vector<double>& diff, cudaStream_t st);
+
+ private:
+  DevBuf<int32_t> row_, col_;
+  DevBuf<double> a_, pa_, out_, diff_;
+  DevBuf<uint8_t> done_;
+  DevBuf<int> open_;
+};
 // r_k = e_{rows[k]} - lam_k + G o y_k
 int residual_t_device(const double* d_lam, const double* d_y, const double* d_G, const int32_t* d_rows, int n,
                       int nrhs, double* d_r, cudaStream_t st);

@@ -2,7 +2,6 @@
 #include "tt_solver.h"
 
 #include <chrono>
-#include <complex>
 #include <cmath>
 #include <cstdlib>
 #include <algorithm>
@@ -210,56 +209,11 @@ int ChannelSolver::resolvent(const std::vector<double>& E, cudaStream_t st) {
 
 namespace {
 
-using cd = std::complex<double>;
-
 // Panel width of the complex64 LU for order n and tensor-core product.
 int tuned_panel_width(int n, int product) {
   for (const PanelWidthRow& r : kPanelWidthTable)
     if (r.product == product && n <= r.n_max) return r.width;
   return 512;
-}
-
-// Determinant by LU with partial pivoting, pivots chosen by |re| + |im| as
-// LAPACK's zgetrf does (determinant, CPP/General_functions/matrix_routines.cpp:82-101).
-cd determinant(std::vector<cd> a, int n) {
-  cd det = 1.0;
-  for (int k = 0; k < n; k++) {
-    int p = k;
-    double best = -1;
-    for (int i = k; i < n; i++) {
-      const double v = std::fabs(a[i * n + k].real()) + std::fabs(a[i * n + k].imag());
-      if (v > best) {
-        best = v;
-        p = i;
-      }
-    }
-    if (a[p * n + k] == cd(0.0)) return 0.0;
-    if (p != k) {
-      for (int c = 0; c < n; c++) std::swap(a[k * n + c], a[p * n + c]);
-      det = -det;
-    }
-    det *= a[k * n + k];
-    for (int i = k + 1; i < n; i++) {
-      const cd l = a[i * n + k] / a[k * n + k];
-      for (int c = k + 1; c < n; c++) a[i * n + c] -= l * a[k * n + c];
-    }
-  }
-  return det;
-}
-
-// [N/M] Pade approximant at z of the series with coefficients a[0 .. N+M]
-// (pade_approximant, CPP/solve_faddeev.cpp:271-296)
-cd pade_approximant(const cd* a, int N, int M, cd z) {
-  std::vector<cd> P((M + 1) * (M + 1)), Q((M + 1) * (M + 1));
-  for (int r = 0; r < M; r++)
-    for (int c = 0; c < M + 1; c++) P[r * (M + 1) + c] = Q[r * (M + 1) + c] = a[N - M + 1 + r + c];
-  for (int c = 0; c < M + 1; c++) {
-    Q[M * (M + 1) + c] = std::pow(z, M - c);
-    cd s = 0.0;
-    for (int j = M - c; j < N + 1; j++) s += a[j - (M - c)] * std::pow(z, j);
-    P[M * (M + 1) + c] = s;
-  }
-  return determinant(P, M + 1) / determinant(Q, M + 1);
 }
 
 }  // namespace
@@ -273,7 +227,6 @@ cd pade_approximant(const cd* a, int N, int M, cd z) {
 // smallest difference of consecutive approximants < 1e-6 |best| or < 1e-7).
 int ChannelSolver::solve_pade(const std::vector<int>& q_idx, const std::vector<int>& deut, std::vector<double>& U,
                               SolveReport& r, cudaStream_t st, const BreakupRequest* bu) {
-  constexpr int NM_MAX = 14, NTERMS = 2 * NM_MAX + 1;
   auto t0 = std::chrono::steady_clock::now();
   const int nE = (int)q_idx.size(), nd = (int)deut.size();
   const int Nq = L_.Nq, Np = L_.Np;
@@ -315,72 +268,37 @@ int ChannelSolver::solve_pade(const std::vector<int>& q_idx, const std::vector<i
       set_error("Pade element outside the on-shell rows");
       return TT_ERR_BADARG;
     }
-  DevBuf<int32_t> d_rows, d_erow, d_prow, d_pcol;
-  DevBuf<double> R, V, picked;
+  DevBuf<int32_t> d_rows, d_erow;
+  DevBuf<double> R, V;
   TT_TRY(d_rows.upload(rows, st));
   TT_TRY(d_erow.upload(erow, st));
-  TT_TRY(d_prow.upload(prow, st));
-  TT_TRY(d_pcol.upload(pcol, st));
   TT_TRY(R.alloc((size_t)2 * n * nrows));
   TT_TRY(V.alloc((size_t)2 * n * nrows));
-  TT_TRY(picked.alloc((size_t)2 * nel));
-  std::vector<cd> a((size_t)nel * NTERMS, 0.0), pa((size_t)nel * (NM_MAX + 1), 0.0), hv(nel);
-  std::vector<char> conv(nel, 0);
-  std::vector<int> best(nel, 0);
-  auto extract = [&](int term) -> int {
-    TT_TRY(pick_device(R.ptr, n, d_prow.ptr, d_pcol.ptr, nel, picked.ptr, st));
-    TT_CUDA_TRY(cudaMemcpyAsync(hv.data(), picked.ptr, sizeof(cd) * nel, cudaMemcpyDeviceToHost, st));
-    TT_CUDA_TRY(cudaStreamSynchronize(st));
-    for (int e = 0; e < nel; e++)
-      if (!conv[e]) a[(size_t)e * NTERMS + term] = hv[e];
-    return TT_OK;
-  };
+  PadeSeries series;
+  TT_TRY(series.init(prow, pcol, st));
   TT_TRY(gather_rows_device(A_.ptr, n, d_rows.ptr, nrows, R.ptr, st));
-  TT_TRY(extract(0));
-  int nconv = 0, top = 0;
-  double worst_diff = 0;
-  for (int NM = 0; NM <= NM_MAX && nconv < nel; NM++) {
-    top = NM;
-    for (int term = 2 * NM - 1; term <= 2 * NM; term++) {
+  TT_TRY(series.term(R.ptr, n, 0, st));
+  int open = nel, top = 0;
+  for (int N = 0; N <= PadeSeries::kMaxOrder && open > 0; N++) {
+    top = N;
+    for (int term = 2 * N - 1; term <= 2 * N; term++) {
       if (term <= 0) continue;
       TT_TRY(scale_rows_device(R.ptr, G_.ptr, d_erow.ptr, n, nrows, V.ptr, st));
       for (int k0 = 0; k0 < nrows; k0 += 8)
         TT_TRY(gemv_t_device(A_.ptr, n, V.ptr + (size_t)2 * n * k0, std::min(8, nrows - k0),
                              R.ptr + (size_t)2 * n * k0, st));
-      TT_TRY(extract(term));
+      TT_TRY(series.term(R.ptr, n, term, st));
     }
-    for (int e = 0; e < nel; e++) {
-      if (conv[e]) continue;
-      cd* p = &pa[(size_t)e * (NM_MAX + 1)];
-      p[NM] = pade_approximant(&a[(size_t)e * NTERMS], NM, NM, 1.0);
-      int idx_best = 0;
-      double min_diff = 1;
-      for (int prev = 0; prev < NM; prev++) {
-        // the reference compares approximant 0 with the slot before it, zero here
-        const double d = std::abs(p[prev] - (prev > 0 ? p[prev - 1] : cd(0.0)));
-        if (d < min_diff && d > 1e-15) {
-          idx_best = prev;
-          min_diff = d;
-        }
-      }
-      const double d = std::abs(p[NM] - (NM > 0 ? p[NM - 1] : cd(0.0)));
-      if (d < min_diff && d > 1e-15) {
-        idx_best = NM;
-        min_diff = d;
-      }
-      if (NM == NM_MAX || NM - idx_best > 4 || min_diff < 1e-6 * std::abs(p[idx_best]) || min_diff < 1e-7) {
-        conv[e] = 1;
-        best[e] = idx_best;
-        nconv++;
-        worst_diff = std::max(worst_diff, min_diff / std::max(1e-300, std::abs(p[idx_best])));
-      }
-    }
+    TT_TRY(series.order(N, &open, st));
   }
+  std::vector<double> val, diff;
+  TT_TRY(series.result(val, diff, st));
+  double worst_diff = 0;
   for (int e = 0; e < nel; e++) {
-    const cd v = pa[(size_t)e * (NM_MAX + 1) + best[e]];
+    worst_diff = std::max(worst_diff, diff[e]);
     double* out = e < nel_el ? &U[2 * (size_t)e] : &(*bu->U_BU)[2 * (size_t)bu_slot[e - nel_el]];
-    out[0] = v.real();
-    out[1] = v.imag();
+    out[0] = val[2 * (size_t)e];
+    out[1] = val[2 * (size_t)e + 1];
   }
   r.ms_solve += ms_since(t0);
   r.refine_iters = top;           // highest [N/N] order formed
