@@ -63,7 +63,8 @@ def run_and_oracle_U(c, run, Np, Nq):
 # the sub-panel kernel's layouts: one row per thread up to 480 rows of a CTA, two up
 # to 825; complex128 CTAs of up to 395 rows; the last sub-panel narrower than a
 # register block.  U to the refinement's and the suite's 1e-10 per element.
-@pytest.mark.parametrize("Np,Nq", [(6, 6),     # n = 396: two complex128 CTAs, last sub-panel 12 wide
+@pytest.mark.parametrize("Np,Nq", [(7, 5),     # n = 385: a substitution block of one row
+                                   (6, 6),     # n = 396: two complex128 CTAs, last sub-panel 12 wide
                                    (9, 5),     # n = 495: two rows per thread, last 15 wide
                                    (15, 5),    # n = 825: the largest single complex64 CTA, last 25 wide
                                    (19, 4),    # n = 836: two complex64 CTAs
@@ -152,4 +153,24 @@ def test_pade_series_and_transposed_products(Np, Nq, labs):
     assert rel(U, U_o) <= 1e-5 and 1 <= rep["refine_iters"] <= 14
     U2, _ = run.solve(1, tt.PRECISION_PADE)
     assert np.array_equal(U, U2)  # no sum depends on the order of threads
+    run.close()
+
+
+@pytest.mark.parametrize("Np,Nq,j", [
+    (33, 2, 1),   # two warps' worth of columns of VC, tiles of 8 rows up to 40
+    (8, 33, 1),   # one chunk of all q', ranges longer than a staged window
+    (7, 13, 2),   # odd rows: 8-byte stores, T rows padded to a k step
+    (30, 6, 1),   # the headline grid's p bins
+])
+def test_A_build_chunks(Np, Nq, j):
+    # FP64 sums of up to a few hundred terms of both signs, against the largest element
+    run = tt.Run(potential_model="LO_internal", J_2N_max=j, two_J_3N_max=1, Np_WP=Np, Nq_WP=Nq, Nphi=10, Nx=10,
+                 lab_energies="8", chebyshev_s=150)
+    pw = run.host_array(0, 0).reshape(-1, 9)
+    rowptr, col, val = run.P123_csr(0, run.build_P123(0))
+    rows = np.repeat(np.arange(len(rowptr) - 1, dtype=np.int32), np.diff(rowptr))
+    lay = oracle.layout(pw, Np, *[run.host_array(k) for k in range(3, 9)])
+    A_o = oracle.build_A(lay, pw.shape[0], Nq, Np, rows, col, val)
+    run.build_A(0)
+    assert rel(run.A(0), A_o) <= 1e-12
     run.close()

@@ -4,21 +4,16 @@
 // factor and back substitution with the upper factor.
 //
 // The factor is read once per substitution, as a stream: after each
-// factorisation the 64 x 64 diagonal blocks of L and U are inverted (one CTA
-// per block, in shared memory) and multiplied into the neighbouring
-// off-diagonal block; each substitution is then one cooperative kernel with
-// one grid barrier per block column (k_trsv).
-
-#include <cooperative_groups.h>
-
+// factorisation the 128 x 128 diagonal blocks of L and U are inverted (one CTA
+// per block, in shared memory); each substitution is then one cooperative kernel
+// whose CTAs pass the solved blocks on in tagged records (k_trsv).
 #include <algorithm>
 #include <cstring>
 #include <vector>
 
+#include "ll_record.cuh"
 #include "tt_kernels.h"
 #include "tt_lu_internal.h"
-
-namespace cg = cooperative_groups;
 
 namespace tt {
 
@@ -33,7 +28,8 @@ struct CT<float2> {
   using R = float;
 };
 
-constexpr int TSB = 64;       // diagonal block of the substitution (both element types)
+constexpr int TW = 128;       // diagonal block of the substitution (both element types)
+constexpr int TSB = TW / 2;   // its halves are inverted, then joined
 constexpr int TLD = TSB + 1;  // padded shared-memory row of a 64 x 64 tile
 
 template <typename T>
@@ -60,192 +56,154 @@ __device__ __forceinline__ T crecip(T b) {
   return r;
 }
 
-__global__ void k_permute(const double2* __restrict__ b, const int32_t* __restrict__ perm, int n, int nrhs,
-                          double2* __restrict__ x) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n * nrhs) return;
-  const int k = (int)(t / n), i = (int)(t % n);
-  x[t] = b[(size_t)k * n + perm[i]];
-}
-
-// x[perm[i]] = w[i]: the row interchanges applied backwards (transposed solves)
-__global__ void k_permute_inv(const double2* __restrict__ w, const int32_t* __restrict__ perm, int n, int nrhs,
-                              double2* __restrict__ x) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n * nrhs) return;
-  const int k = (int)(t / n), i = (int)(t % n);
-  x[(size_t)k * n + perm[i]] = w[t];
+// Blocks in sweep order: block q of the forward sweep starts at row TW q, of the
+// backward one it ends TW q rows before n; only the last can be shorter.
+__host__ __device__ __forceinline__ int blk_rows(int n, int q) { return n - q * TW < TW ? n - q * TW : TW; }
+template <bool UPPER>
+__host__ __device__ __forceinline__ int blk_start(int n, int q) {
+  return UPPER ? n - q * TW - blk_rows(n, q) : q * TW;
 }
 
 // ---------------------------------------------------------------------------
-// Inverses of the diagonal blocks: inv[b] (64 x 64, row-major) of the lower
-// (UPPER = false) or upper (UPPER = true) triangle of block b of the factor,
-// with a unit diagonal (UNIT) or the stored one.  The factor of L U keeps the
-// unit lower and the upper triangle; its transpose (for transposed solves)
-// keeps the non-unit lower and the unit upper triangle.  Rows and columns past
-// n are the identity.  In place in shared memory, right-looking, row j being
-// final when step j starts:
-// lower, j ascending: row j is scaled by 1/D[j][j], then
-// X[r][c] -= L[r][j] X[j][c] for r > j, c <= j;
-// upper, j descending: row j is scaled by 1/D[j][j], then
-// X[r][c] -= U[r][j] X[j][c] for r < j, c >= j.
+// Inverses of the diagonal blocks, inv[q] (128 x 128, row-major), of a factor's
+// lower and upper triangle (blockIdx.y = 0, 1), with a unit diagonal or the
+// stored one.  The factor of L U keeps the unit lower and the upper triangle; its
+// transpose (TRANSPOSED, for transposed solves) keeps the non-unit lower and the
+// unit upper triangle.  Rows and columns past the block are the identity's.
+// A CTA inverts the block's two 64 x 64 diagonal halves at once, 256 threads each,
+// in place in shared memory, right-looking, row j being final when step j starts
+// (lower, j ascending: row j is scaled by 1/D[j][j], then X[r][c] -= L[r][j] X[j][c]
+// for r > j, c <= j; upper, j descending, mirrored), and joins them:
+// X21 = -X22 (L21 X11), or X12 = -X11 (U12 X22).
 template <typename T, bool UPPER, bool UNIT>
-__global__ void __launch_bounds__(512) k_inv_diag(const T* __restrict__ LU, int n, T* __restrict__ inv) {
-  extern __shared__ unsigned char ism[];
-  T* M = reinterpret_cast<T*>(ism);  // [TSB][TLD]
-  __shared__ T col[TSB];
-  const int b = blockIdx.x, r0 = b * TSB, bs = min(TSB, n - r0);
+__device__ void inv_block(const T* __restrict__ LU, int n, int q, T* __restrict__ out, T* sm, T* cols) {
+  const int tid = threadIdx.x, half = tid >> 8, t = tid & 255;
+  const int r0 = blk_start<UPPER>(n, q), rows = blk_rows(n, q);
   const T zero = {0, 0}, one = {1, 0};
-  // stored entries of the triangle (the diagonal only when it is not unit)
-  auto stored = [](int r, int c) { return UPPER ? (UNIT ? c > r : c >= r) : (UNIT ? c < r : c <= r); };
-  for (int t = threadIdx.x; t < TSB * TSB; t += blockDim.x) {
-    const int r = t / TSB, c = t % TSB;
+  T* M = sm + half * TSB * TLD;   // this half's diagonal tile
+  T* O = sm + 2 * TSB * TLD;      // the off-diagonal tile
+  T* col = cols + half * TSB;
+  const int h0 = half * TSB, bs = max(0, min(TSB, rows - h0));
+  for (int e = t; e < TSB * TSB; e += 256) {
+    const int r = e / TSB, c = e % TSB;
+    const bool stored = UPPER ? (UNIT ? c > r : c >= r) : (UNIT ? c < r : c <= r);
     T v = (r == c) ? one : zero;
-    if (r < bs && c < bs && stored(r, c)) v = LU[(size_t)(r0 + r) * n + r0 + c];
+    if (r < bs && c < bs && stored) v = LU[(size_t)(r0 + h0 + r) * n + r0 + h0 + c];
     M[r * TLD + c] = v;
   }
-  __syncthreads();
-  if (!UPPER) {
-    for (int j = 0; j < bs; j++) {
-      T d = one;
-      if (!UNIT) {
-        d = crecip(M[j * TLD + j]);
-        __syncthreads();
-        for (int c = threadIdx.x; c < j; c += blockDim.x) M[j * TLD + c] = cmul(M[j * TLD + c], d);
-        if (threadIdx.x == 0) M[j * TLD + j] = d;
-      }
-      for (int r = j + 1 + threadIdx.x; r < bs; r += blockDim.x) col[r] = M[r * TLD + j];
-      __syncthreads();
-      const int w = j + 1, cnt = (bs - 1 - j) * w;
-      for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-        const int r = j + 1 + t / w, c = t % w;
-        const T l = col[r];
-        if (c == j) {
-          const T p = cmul(l, d);
-          M[r * TLD + j] = T{-p.x, -p.y};
-        } else {
-          const T p = cmul(l, M[j * TLD + c]);
-          T v = M[r * TLD + c];
-          v.x -= p.x;
-          v.y -= p.y;
-          M[r * TLD + c] = v;
-        }
-      }
-      __syncthreads();
-    }
-  } else {
-    for (int j = bs - 1; j >= 0; j--) {
-      T d = one;
-      if (!UNIT) {
-        d = crecip(M[j * TLD + j]);
-        __syncthreads();
-        for (int c = j + 1 + threadIdx.x; c < bs; c += blockDim.x) M[j * TLD + c] = cmul(M[j * TLD + c], d);
-        if (threadIdx.x == 0) M[j * TLD + j] = d;
-      }
-      for (int r = threadIdx.x; r < j; r += blockDim.x) col[r] = M[r * TLD + j];
-      __syncthreads();
-      const int w = bs - j, cnt = j * w;
-      for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-        const int r = t / w, c = j + t % w;
-        const T u = col[r];
-        if (c == j) {
-          const T p = cmul(u, d);
-          M[r * TLD + j] = T{-p.x, -p.y};
-        } else {
-          const T p = cmul(u, M[j * TLD + c]);
-          T v = M[r * TLD + c];
-          v.x -= p.x;
-          v.y -= p.y;
-          M[r * TLD + c] = v;
-        }
-      }
-      __syncthreads();
-    }
+  for (int e = tid; e < TSB * TSB; e += 512) {
+    const int r = e / TSB + (UPPER ? 0 : TSB), c = e % TSB + (UPPER ? TSB : 0);
+    O[(e / TSB) * TLD + e % TSB] = (r < rows && c < rows) ? LU[(size_t)(r0 + r) * n + r0 + c] : zero;
   }
-  T* out = inv + (size_t)b * TSB * TSB;
-  for (int t = threadIdx.x; t < TSB * TSB; t += blockDim.x) {
-    const int r = t / TSB, c = t % TSB;
-    const bool keep = r < bs && c < bs && (UPPER ? c >= r : c <= r);
-    out[t] = keep ? M[r * TLD + c] : ((r == c) ? one : zero);
+  __syncthreads();
+  for (int step = 0; step < TSB; step++) {
+    const int j = UPPER ? TSB - 1 - step : step;
+    const int w = UPPER ? TSB - j : j + 1;       // columns of row j, from c0
+    const int c0 = UPPER ? j : 0, f0 = UPPER ? 0 : j + 1, cnt = TSB - w;  // rows still to be updated: [f0, f0 + cnt)
+    T d = one;
+    if (!UNIT) {
+      d = crecip(M[j * TLD + j]);
+      __syncthreads();
+      for (int c = t; c < w - 1; c += 256) {
+        const int cc = UPPER ? j + 1 + c : c;
+        M[j * TLD + cc] = cmul(M[j * TLD + cc], d);
+      }
+      if (t == 0) M[j * TLD + j] = d;
+    }
+    for (int r = t; r < cnt; r += 256) col[f0 + r] = M[(f0 + r) * TLD + j];
+    __syncthreads();
+    // 4 threads a row
+    for (int r = f0 + (t >> 2); r < f0 + cnt; r += 64) {
+      const T l = col[r];
+      for (int c = c0 + (t & 3); c < c0 + w; c += 4) {
+        const T p = cmul(l, c == j ? d : M[j * TLD + c]);
+        const T v = c == j ? zero : M[r * TLD + c];
+        M[r * TLD + c] = T{v.x - p.x, v.y - p.y};
+      }
+    }
+    __syncthreads();
+  }
+  // join: 8 elements a thread, row tr, columns tc + 8 u
+  const T* X1 = sm;               // inverse of the first half
+  const T* X2 = sm + TSB * TLD;   // of the second
+  const int tr = tid >> 3, tc = tid & 7;
+  auto product = [&](const T* a, const T* b, T(&acc)[8]) {
+#pragma unroll
+    for (int u = 0; u < 8; u++) acc[u] = zero;
+    for (int k = 0; k < TSB; k++) {
+      const T x = a[tr * TLD + k];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const T p = cmul(x, b[k * TLD + tc + 8 * u]);
+        acc[u].x += p.x;
+        acc[u].y += p.y;
+      }
+    }
+  };
+  T acc[8];
+  product(O, UPPER ? X2 : X1, acc);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 8; u++) O[tr * TLD + tc + 8 * u] = acc[u];
+  __syncthreads();
+  product(UPPER ? X1 : X2, O, acc);
+  T* o = out + (size_t)q * TW * TW;
+#pragma unroll
+  for (int u = 0; u < 8; u++) {
+    const int c = tc + 8 * u;
+    o[(size_t)(tr + (UPPER ? 0 : TSB)) * TW + c + (UPPER ? TSB : 0)] = T{-acc[u].x, -acc[u].y};
+    o[(size_t)(tr + (UPPER ? TSB : 0)) * TW + c + (UPPER ? 0 : TSB)] = zero;
+    o[(size_t)tr * TW + c] = X1[tr * TLD + c];
+    o[(size_t)(tr + TSB) * TW + c + TSB] = X2[tr * TLD + c];
   }
 }
-
-// M[b] = inv[b] LU[b, prev(b)] for the blocks after the first in sweep order
-// (prev = b-1 forward, b+1 backward): the product that carries the solved
-// previous block into block b, so that x_b = inv[b] x_b - M[b] x_prev.
-template <typename T, bool UPPER>
-__global__ void __launch_bounds__(512) k_prev_mul(const T* __restrict__ LU, int n, const T* __restrict__ inv,
-                                                  T* __restrict__ Mo) {
-  extern __shared__ unsigned char psm[];
-  T* sI = reinterpret_cast<T*>(psm);  // [TSB][TLD]
-  T* sT = sI + TSB * TLD;             // [TSB][TLD]
-  const int nb = (n + TSB - 1) / TSB, b = blockIdx.x;
-  const int prev = UPPER ? b + 1 : b - 1;
-  if (prev < 0 || prev >= nb) return;
-  const int r0 = b * TSB, rows = min(TSB, n - r0), c0 = prev * TSB, cols = min(TSB, n - c0);
-  for (int t = threadIdx.x; t < TSB * TSB; t += blockDim.x) {
-    const int r = t / TSB, c = t % TSB;
-    sI[r * TLD + c] = inv[(size_t)b * TSB * TSB + t];
-    sT[r * TLD + c] = (r < rows && c < cols) ? LU[(size_t)(r0 + r) * n + c0 + c] : T{0, 0};
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < TSB * TSB; t += blockDim.x) {
-    const int r = t / TSB, c = t % TSB;
-    T acc = {0, 0};
-    for (int u = 0; u < TSB; u++) {
-      const T p = cmul(sI[r * TLD + u], sT[u * TLD + c]);
-      acc.x += p.x;
-      acc.y += p.y;
-    }
-    Mo[(size_t)b * TSB * TSB + t] = acc;
-  }
+template <typename T, bool TRANSPOSED>
+__global__ void __launch_bounds__(512) k_inv_blocks(const T* __restrict__ LU, int n, T* __restrict__ invL,
+                                                    T* __restrict__ invU) {
+  extern __shared__ __align__(16) unsigned char ism[];
+  __shared__ T cols[2 * TSB];
+  T* sm = reinterpret_cast<T*>(ism);  // [3][TSB][TLD]
+  if (blockIdx.y == 0) inv_block<T, false, !TRANSPOSED>(LU, n, blockIdx.x, invL, sm, cols);
+  else inv_block<T, true, TRANSPOSED>(LU, n, blockIdx.x, invU, sm, cols);
 }
 
 // ---------------------------------------------------------------------------
-// One substitution (forward with L when !UPPER, backward with U when UPPER)
-// for kn <= RHS right-hand sides x[k][n], cooperative, one grid barrier per
-// block column.  Blocks are visited in sweep order q = 0, 1, .. (block q for
-// the forward sweep, block nb-1-q for the backward one).  Arithmetic is in the
-// factor's precision (FP32 for the complex64 factor, whose solves only feed the
-// FP64-residual refinement; FP64 for the complex128 factor); x stays complex128.
-//  - CTA 0 owns the serial chain: at step s it solves block q = s+1,
-//    x_{s+1} = inv[s+1] x_{s+1} - M[s+1] x_s, one 64 x 128 product with both
-//    tiles already in shared memory (cp.async issued a step ahead, during the
-//    barrier), and writes the solved block to x.
-//  - Blocks q >= 2 are owned round-robin by CTAs 1..G-1, which keep their rows
-//    of x in shared memory for the whole sweep: at step s every owner applies
-//    block column s to its unsolved blocks (q >= s+2) and publishes block s+2
-//    to x, which CTA 0 reads at the next step.  Eight lanes share a row (four
-//    rows per warp) against x_s staged in shared memory, and the next owned
-//    tile is loaded while the current one is applied.  x is never read-modify-written in global
-//    memory.
+// One substitution (forward with L when !UPPER, backward with U when UPPER) for
+// kn <= RHS right-hand sides, of B factors (Gb CTAs each), cooperative.  Blocks of
+// 128 rows are visited in sweep order q = 0, 1, ..  Arithmetic is in the factor's
+// precision (FP32 for the complex64 factor, whose solves only feed the
+// FP64-residual refinement; FP64 for the complex128 factor); the vectors are
+// complex128.
+//  - LEADS lead CTAs solve the blocks: when block q's right-hand side y is
+//    complete, they form x_q = inv[q] y, 32 rows each, the rows of inv asked for
+//    while y is awaited.
+//  - The other CTAs own the rows, two neighbouring ones at a time in turn, and keep
+//    their values in shared memory.  When x_q is there, a warp applies block column q
+//    to four of its CTA's unsolved rows at a time; those of block q + 1 come first
+//    and are posted at once, so the leads solve block q + 1 while the rest of the
+//    column is applied.
+// y and x pass through tagged records (ll_record.cuh), so a step costs two trips
+// through L2 and no grid barrier.  Slots are reused: y_q's for y_{q+2}, posted by
+// owners that have all of x_{q+1}, so every lead has read y_q; x_q's for
+// x_{q+X_SLOTS}.  Every owner that still waits for x_q has its next pair of rows in
+// a block no later than q + 1 + (GO - 1) / 64, and x_{q+X_SLOTS} needs that block's y,
+// so X_SLOTS = 4 serves up to 192 owners.  Bound: the factor read once from HBM where its rows
+// are long, else the two trips (about 2 us a block of 128).  Per sweep, against
+// blocks of 64 with a grid barrier each: n = 512 (2 factors) 28 -> 11 us, 1,859 (4)
+// 115 -> 46 us, 10,944 (1) 670 -> 303 us, 16,128 (2) 1.42 -> 0.68 ms, 20,160 (4)
+// 2.57 -> 1.44 ms, 42,300 (2) 6.5 -> 3.65 ms; complex128 n = 8,496 755 -> 530 us.
 constexpr int RHS = 4;
 constexpr int TRSV_THREADS = 512;
+constexpr int LEADS = 4;
+constexpr int X_SLOTS = 4;
+constexpr int TRSV_SPINS = 1 << 20;
 
-__device__ __forceinline__ void cp_async_elem(void* smem, const void* gmem, int bytes) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  if (bytes == 16)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// 64 x 64 block b of a [nb][64][64] array into dst[TSB][TLD]; no commit
-template <typename T>
-__device__ __forceinline__ void tile_async(const T* __restrict__ src, int b, T* dst) {
-  for (int t = threadIdx.x; t < TSB * TSB; t += blockDim.x)
-    cp_async_elem(&dst[(t / TSB) * TLD + t % TSB], src + (size_t)b * TSB * TSB + t, sizeof(T));
-}
-
-// reduce 16 values over the 32 lanes of a warp: a butterfly that halves the
-// values each round (8+4+2+1 shuffles) and a final pair sum; value lane >> 1
-// ends complete in lanes 2i and 2i+1
-template <typename C>
-__device__ __forceinline__ C butterfly16(C (&acc)[16], int lane) {
+// reduce 2 M values over the 32 lanes of a warp by halving the values each round;
+// value i ends complete in lane i (M = 16) or in lanes 2i and 2i + 1 (M = 8)
+template <int M, typename C>
+__device__ __forceinline__ C butterfly(C (&acc)[2 * M], int lane) {
 #pragma unroll
-  for (int o = 16, m = 8; m >= 1; o >>= 1, m >>= 1) {
+  for (int o = 16, m = M; m >= 1; o >>= 1, m >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
     for (int j = 0; j < m; j++) {
@@ -254,206 +212,233 @@ __device__ __forceinline__ C butterfly16(C (&acc)[16], int lane) {
       acc[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  return acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
+  if (M == 8) return acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
+  return acc[0];
 }
 
-// Up to kMaxSweeps factors swept in one cooperative launch: the grid splits
-// into B equal groups, each with its own lead CTA and owners, sharing every
-// grid barrier.
+// Up to kMaxSweeps factors swept in one cooperative launch.
 constexpr int kMaxSweeps = 4;
 template <typename T>
 struct TrsvBatch {
   const T* LU[kMaxSweeps];
   const T* inv[kMaxSweeps];
-  const T* Mp[kMaxSweeps];
-  double2* x[kMaxSweeps];
+  const double2* in[kMaxSweeps];      // right-hand sides [k][n], row r read at in_perm[r]
+  double2* out[kMaxSweeps];           // solutions [k][n], row r written at out_perm[r]
+  const int32_t* in_perm[kMaxSweeps];
+  const int32_t* out_perm[kMaxSweeps];
+  unsigned char* rec[kMaxSweeps];     // [2 of y, X_SLOTS of x][RHS][TW] records
+  unsigned epoch[kMaxSweeps];         // tags of this sweep are above it
+  int* err[kMaxSweeps];
   int B;
 };
 
-template <typename T, bool UPPER>
-__global__ void __launch_bounds__(TRSV_THREADS, 1) k_trsv(TrsvBatch<T> bt, int n, int kn, int own_max) {
-  const int Gb = gridDim.x / bt.B, grp = blockIdx.x / Gb, local = blockIdx.x - grp * Gb;
-  const T* __restrict__ LU = bt.LU[grp];
-  const T* __restrict__ inv = bt.inv[grp];
-  const T* __restrict__ Mp = bt.Mp[grp];
-  double2* __restrict__ x = bt.x[grp];
-  using C = typename CT<T>::R;
-  constexpr int TILE = TSB * TLD;
-  cg::grid_group grid = cg::this_grid();
-  extern __shared__ __align__(16) unsigned char tsm[];
-  T* tI = reinterpret_cast<T*>(tsm);                         // CTA 0: inverse tile
-  T* tM = tI + TILE;                                         // CTA 0: M tile
-  T* xo = reinterpret_cast<T*>(tsm + 2 * TILE * sizeof(T));  // owners: [own_max][RHS][TSB]
-  __shared__ T xs[RHS][TSB];   // CTA 0: solved block of this step
-  __shared__ T bsh[RHS][TSB];  // CTA 0: published rows of the block being solved
-  __shared__ T ysh[RHS][TSB];  // CTA 0: its solution
-  const int nb = (n + TSB - 1) / TSB;
-  const int G = Gb;  // this factor's CTAs, >= 2
-  const bool lead = local == 0;
-  auto blk = [&](int q) { return UPPER ? nb - 1 - q : q; };
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  auto ld_x = [&](int k, int r) -> T {
-    const double2 v = x[(size_t)k * n + r];
-    return T{(C)v.x, (C)v.y};
-  };
-  // CTA 0: out = tI . bsh - tM . xs for rows warp*4 .. +3 (two pairs), lanes
-  // over the columns lane and lane+32, to ysh and to x rows [r0, r0+rows)
-  auto lead_solve = [&](int r0, int rows) {
+// the 4 elements of a 128-column row segment that a lane holds: pairs of
+// neighbours where 16-byte loads of complex64 are possible (WIDE), else every 32nd
+template <typename T, bool WIDE>
+__device__ __forceinline__ void load_seg(const T* __restrict__ row, int lane, T (&v)[4]) {
+  if constexpr (WIDE && sizeof(T) == 8) {
 #pragma unroll
-    for (int hp = 0; hp < 2; hp++) {
-      C acc[16];
-#pragma unroll
-      for (int hh = 0; hh < 2; hh++) {
-        const int r = warp * 4 + hp * 2 + hh;
-        const T i0 = tI[r * TLD + lane], i1 = tI[r * TLD + lane + 32];
-        const T m0 = tM[r * TLD + lane], m1 = tM[r * TLD + lane + 32];
-#pragma unroll
-        for (int k = 0; k < RHS; k++) {
-          C sr = 0, si = 0;
-          if (k < kn) {
-            const T b0 = bsh[k][lane], b1 = bsh[k][lane + 32], y0 = xs[k][lane], y1 = xs[k][lane + 32];
-            sr = i0.x * b0.x - i0.y * b0.y + i1.x * b1.x - i1.y * b1.y -
-                 (m0.x * y0.x - m0.y * y0.y + m1.x * y1.x - m1.y * y1.y);
-            si = i0.x * b0.y + i0.y * b0.x + i1.x * b1.y + i1.y * b1.x -
-                 (m0.x * y0.y + m0.y * y0.x + m1.x * y1.y + m1.y * y1.x);
-          }
-          acc[(hh * RHS + k) * 2 + 0] = sr;
-          acc[(hh * RHS + k) * 2 + 1] = si;
-        }
-      }
-      const C v = butterfly16<C>(acc, lane);
-      const int idx = lane >> 1, hh = idx >> 3, k = (idx >> 1) & 3, part = idx & 1;
-      const int r = warp * 4 + hp * 2 + hh;
-      if ((lane & 1) == 0 && k < kn) {
-        reinterpret_cast<C*>(&ysh[k][r])[part] = v;
-        if (r < rows) reinterpret_cast<double*>(x + (size_t)k * n + r0 + r)[part] = (double)v;
-      }
-
-    }
-  };
-
-  // owners: slots j of block q = 2 + me + j (G-1)
-  const int me = local - 1;
-  auto first_slot = [&](int s) { return s > me ? (s - me + (G - 1) - 1) / (G - 1) : 0; };
-  auto live = [&](int j) { return j < own_max && 2 + me + j * (G - 1) < nb; };
-
-  if (lead) {
-    // first block: x_0 = inv[0] x_0
-    tile_async<T>(inv, blk(0), tI);
-    cp_async_commit();
-    const int r0 = blk(0) * TSB, bsz = min(TSB, n - r0);
-    for (int e = t; e < TSB * RHS; e += blockDim.x) {
-      const int k = e / TSB, r = e % TSB;
-      bsh[k][r] = (k < kn && r < bsz) ? ld_x(k, r0 + r) : T{0, 0};
-      xs[k][r] = T{0, 0};
-    }
-    for (int e = t; e < TILE; e += blockDim.x) tM[e] = T{0, 0};
-    cp_async_wait_all();
-    __syncthreads();
-    lead_solve(r0, bsz);
-    __syncthreads();
-    for (int e = t; e < TSB * RHS; e += blockDim.x) xs[e / TSB][e % TSB] = ysh[e / TSB][e % TSB];
-    if (nb > 1) {
-      tile_async<T>(inv, blk(1), tI);
-      tile_async<T>(Mp, blk(1), tM);
-      cp_async_commit();
+    for (int u = 0; u < 2; u++) {
+      const float4 f = __ldcs(reinterpret_cast<const float4*>(row) + lane + 32 * u);
+      v[2 * u] = T{f.x, f.y};
+      v[2 * u + 1] = T{f.z, f.w};
     }
   } else {
-    for (int j = 0; j < own_max; j++) {
-      const int q = 2 + me + j * (G - 1);
-      const int r0 = q < nb ? blk(q) * TSB : 0, bsz = q < nb ? min(TSB, n - r0) : 0;
-      for (int e = t; e < TSB * RHS; e += blockDim.x) {
-        const int k = e / TSB, r = e % TSB;
-        xo[((size_t)j * RHS + k) * TSB + r] = (k < kn && r < bsz) ? ld_x(k, r0 + r) : T{0, 0};
-      }
-    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = __ldcs(row + lane + 32 * u);
   }
-  grid.sync();
-  for (int s = 0; s + 1 < nb; s++) {
-    const int c0 = blk(s) * TSB, csz = min(TSB, n - c0);
-    if (lead) {
-      const int nr0 = blk(s + 1) * TSB, nsz = min(TSB, n - nr0);
-      for (int e = t; e < TSB * RHS; e += blockDim.x) {
-        const int k = e / TSB, r = e % TSB;
-        bsh[k][r] = (k < kn && r < nsz) ? ld_x(k, nr0 + r) : T{0, 0};
-      }
-      cp_async_wait_all();
-      __syncthreads();
-      lead_solve(nr0, nsz);
-      __syncthreads();
-      for (int e = t; e < TSB * RHS; e += blockDim.x) xs[e / TSB][e % TSB] = ysh[e / TSB][e % TSB];
-      if (s + 2 < nb) {
-        tile_async<T>(inv, blk(s + 2), tI);
-        tile_async<T>(Mp, blk(s + 2), tM);
-        cp_async_commit();
-      }
-    } else {
-      for (int e = t; e < TSB * RHS; e += blockDim.x) {
-        const int k = e / TSB, r = e % TSB;
-        xs[k][r] = (k < kn && r < csz) ? ld_x(k, c0 + r) : T{0, 0};
-      }
-      __syncthreads();
-      // 8 lanes per row, 4 rows per warp: x_s from shared memory, the next
-      // owned tile loaded while this one is applied
-      const int sub = lane >> 3, sl = lane & 7, row = warp * 4 + sub;
-      T a[8], an[8];
-      auto load8 = [&](int j, T(&dst)[8]) {
-        const int r = blk(2 + me + j * (G - 1)) * TSB + row;
+}
+template <typename T, bool WIDE>
+__device__ __forceinline__ void smem_seg(const T* row, int lane, T (&v)[4]) {
+  if constexpr (WIDE && sizeof(T) == 8) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int c = sl + 8 * u;
-          dst[u] = (r < n && c < csz) ? LU[(size_t)r * n + c0 + c] : T{0, 0};
-        }
-      };
-      // complex128 tiles are not double-buffered: two would not fit in registers
-      constexpr bool PF = sizeof(T) == sizeof(float2);
-      const int j0 = first_slot(s);
-      if (PF && live(j0)) load8(j0, a);
-      for (int j = j0; live(j); j++) {
-        const bool more = PF && live(j + 1);
-        if (more) load8(j + 1, an);
-        if (!PF) load8(j, a);
+    for (int u = 0; u < 2; u++) {
+      const float4 f = reinterpret_cast<const float4*>(row)[lane + 32 * u];
+      v[2 * u] = T{f.x, f.y};
+      v[2 * u + 1] = T{f.z, f.w};
+    }
+  } else {
 #pragma unroll
-        for (int k = 0; k < RHS; k++) {
-          if (k >= kn) break;
-          C sr = 0, si = 0;
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const T v = xs[k][sl + 8 * u];
-            sr += a[u].x * v.x - a[u].y * v.y;
-            si += a[u].x * v.y + a[u].y * v.x;
-          }
-#pragma unroll
-          for (int o = 4; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xffffffffu, sr, o);
-            si += __shfl_xor_sync(0xffffffffu, si, o);
-          }
-          if (sl == 0) {
-            T& d = xo[((size_t)j * RHS + k) * TSB + row];
-            d.x -= sr;
-            d.y -= si;
-          }
-        }
-        if (more) {
-#pragma unroll
-          for (int u = 0; u < 8; u++) a[u] = an[u];
-        }
-      }
-      // publish block s+2 if owned here
-      const int qp = s + 2;
-      if (qp < nb && (qp - 2) % (G - 1) == me) {
-        __syncthreads();
-        const int j = (qp - 2) / (G - 1), r0 = blk(qp) * TSB, bsz = min(TSB, n - r0);
-        for (int e = t; e < TSB * RHS; e += blockDim.x) {
-          const int k = e / TSB, r = e % TSB;
-          if (k < kn && r < bsz) {
-            const T v = xo[((size_t)j * RHS + k) * TSB + r];
-            x[(size_t)k * n + r0 + r] = make_double2((double)v.x, (double)v.y);
-          }
+    for (int u = 0; u < 4; u++) v[u] = row[lane + 32 * u];
+  }
+}
+
+template <typename T, bool UPPER, bool WIDE>
+__global__ void __launch_bounds__(TRSV_THREADS, 1) k_trsv(TrsvBatch<T> bt, int n, int kn) {
+  using C = typename CT<T>::R;
+  const int Gb = gridDim.x / bt.B, grp = blockIdx.x / Gb, local = blockIdx.x - grp * Gb;
+  const T* __restrict__ LU = bt.LU[grp];
+  unsigned char* rec = bt.rec[grp];
+  const unsigned epoch = bt.epoch[grp];
+  extern __shared__ __align__(16) unsigned char tsm[];
+  T* vs = reinterpret_cast<T*>(tsm);  // [2][RHS][TW]: y (leads) or x (owners) of this step, double-buffered
+  T* xo = vs + 2 * RHS * TW;          // owners: [pairs][2][RHS]
+  __shared__ int s_dead;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int nb = (n + TW - 1) / TW;
+  auto slot = [&](int which, int q) {
+    return rec + (size_t)(which ? 2 + q % X_SLOTS : q & 1) * RHS * TW * LL<T>::BYTES;
+  };
+  int* err = bt.err[grp];
+  if (t == 0) s_dead = *(volatile int*)err;
+  // this thread's element of a posted block into vs; RHS * TW threads
+  const int ek = t / TW, ej = t % TW;
+  auto collect = [&](int which, int q) {
+    T v = {0, 0};
+    if (ek < kn && ej < blk_rows(n, q)) {
+      unsigned long long hi;
+      const unsigned char* p = slot(which, q) + t * LL<T>::BYTES;
+      const unsigned tag = epoch + (unsigned)q + 1u;
+      for (int spin = 0; !LL<T>::poll(p, v, hi, tag); spin++) {
+        if (spin >= TRSV_SPINS || *(volatile int*)&s_dead) {
+          *(volatile int*)&s_dead = 1;
+          atomicExch(err, 1);
+          break;
         }
       }
     }
-    grid.sync();
+    vs[(q & 1) * RHS * TW + t] = v;
+  };
+  __syncthreads();
+
+  if (local < LEADS) {
+    const int row = local * (TW / LEADS) + warp * 2;  // two rows a warp
+    T a[2][4];
+    auto load_inv = [&](int q) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) load_seg<T, WIDE>(bt.inv[grp] + (size_t)q * TW * TW + (size_t)(row + h) * TW, lane, a[h]);
+    };
+    load_inv(0);
+    for (int q = 0; q < nb; q++) {
+      collect(0, q);
+      __syncthreads();
+      C acc[16];
+#pragma unroll
+      for (int k = 0; k < RHS; k++) {
+        C sr[2] = {0, 0}, si[2] = {0, 0};
+        if (k < kn) {
+          T y[4];
+          smem_seg<T, WIDE>(vs + ((q & 1) * RHS + k) * TW, lane, y);
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              sr[h] += a[h][u].x * y[u].x - a[h][u].y * y[u].y;
+              si[h] += a[h][u].x * y[u].y + a[h][u].y * y[u].x;
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          acc[(h * RHS + k) * 2] = sr[h];
+          acc[(h * RHS + k) * 2 + 1] = si[h];
+        }
+      }
+      if (q + 1 < nb) load_inv(q + 1);
+      const C v = butterfly<8>(acc, lane);
+      const C im = __shfl_down_sync(0xffffffffu, v, 2);
+      const int i = lane >> 1, h = i >> 3, k = (i >> 1) & 3, j = row + h;
+      if ((lane & 3) == 0 && k < kn && j < blk_rows(n, q)) {
+        LL<T>::post(slot(1, q) + (k * TW + j) * LL<T>::BYTES, T{v, im}, epoch + (unsigned)q + 1u);
+        const int r = blk_start<UPPER>(n, q) + j;
+        bt.out[grp][(size_t)k * n + (bt.out_perm[grp] ? bt.out_perm[grp][r] : r)] = make_double2((double)v, (double)im);
+      }
+    }
+    return;
+  }
+
+  // owners: pair p of sweep rows 2 p, 2 p + 1 belongs to CTA LEADS + p % GO
+  const int GO = Gb - LEADS, me = local - LEADS;
+  const int npairs = (n + 1) / 2;
+  const int mine = me < npairs ? (npairs - me + GO - 1) / GO : 0;
+  auto row_of = [&](int pl, int h) {  // row of local pair pl, or -1
+    const int i = 2 * (me + pl * GO) + h;
+    return i < n ? (UPPER ? n - 1 - i : i) : -1;
+  };
+  for (int e = t; e < mine * 2 * RHS; e += TRSV_THREADS) {
+    const int k = e % RHS, h = (e / RHS) & 1, pl = e / (2 * RHS), r = row_of(pl, h);
+    T v = {0, 0};
+    if (k < kn && r >= 0) {
+      const double2 d = bt.in[grp][(size_t)k * n + (bt.in_perm[grp] ? bt.in_perm[grp][r] : r)];
+      v = T{(C)d.x, (C)d.y};
+      if (2 * (me + pl * GO) < TW)  // block 0 is complete as it is
+        LL<T>::post(slot(0, 0) + (k * TW + r - blk_start<UPPER>(n, 0)) * LL<T>::BYTES, v, epoch + 1u);
+    }
+    xo[e] = v;
+  }
+  // first local pair of block q or later
+  auto first_pair = [&](int q) {
+    const int p0 = q * (TW / 2);
+    return p0 > me ? (p0 - me + GO - 1) / GO : 0;
+  };
+  constexpr int NW = TRSV_THREADS / 32;
+  for (int q = 0; q + 1 < nb && first_pair(q + 1) < mine; q++) {
+    const int c0 = blk_start<UPPER>(n, q);
+    const int y0 = blk_start<UPPER>(n, q + 1), yn = blk_rows(n, q + 1);
+    // two pairs (four rows) a warp at a time, the next ones asked for ahead
+    const int p0 = first_pair(q + 1) + 2 * warp;
+    T a[4][4], an[4][4];
+    auto load = [&](int p, T(&d)[4][4]) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int pl = p + (i >> 1), r = pl < mine ? row_of(pl, i & 1) : -1;
+        if (r >= 0) {
+          load_seg<T, WIDE>(LU + (size_t)r * n + c0, lane, d[i]);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; u++) d[i][u] = T{0, 0};
+        }
+      }
+    };
+    constexpr bool AHEAD = sizeof(T) == 8;  // two sets of complex128 rows do not fit in registers
+    if (p0 < mine) load(p0, a);
+    collect(1, q);
+    __syncthreads();
+    const T* xs = vs + (q & 1) * RHS * TW;
+    for (int p = p0; p < mine; p += 2 * NW) {
+      const bool more = p + 2 * NW < mine;
+      if (AHEAD && more) load(p + 2 * NW, an);
+      C acc[32];
+#pragma unroll
+      for (int k = 0; k < RHS; k++) {
+        T x[4];
+        if (k < kn) smem_seg<T, WIDE>(xs + k * TW, lane, x);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          C sr = 0, si = 0;
+          if (k < kn) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              sr += a[i][u].x * x[u].x - a[i][u].y * x[u].y;
+              si += a[i][u].x * x[u].y + a[i][u].y * x[u].x;
+            }
+          }
+          acc[(i * RHS + k) * 2] = sr;
+          acc[(i * RHS + k) * 2 + 1] = si;
+        }
+      }
+      const C v = butterfly<16>(acc, lane);  // lane = (row i, k, part)
+      C* d = reinterpret_cast<C*>(xo + (size_t)p * 2 * RHS) + lane;
+      const int i = lane >> 3, k = (lane >> 1) & 3, pl = p + (i >> 1);
+      C val = 0;
+      if (pl < mine) {
+        val = *d - v;
+        *d = val;
+      }
+      const C im = __shfl_down_sync(0xffffffffu, val, 1);
+      const int r = pl < mine ? row_of(pl, i & 1) : -1;
+      if ((lane & 1) == 0 && k < kn && r >= y0 && r < y0 + yn)
+        LL<T>::post(slot(0, q + 1) + (k * TW + r - y0) * LL<T>::BYTES, T{val, im}, epoch + (unsigned)q + 2u);
+      if (more) {
+        if (AHEAD) {
+#pragma unroll
+          for (int x = 0; x < 4; x++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) a[x][u] = an[x][u];
+        } else {
+          load(p + 2 * NW, a);
+        }
+      }
+    }
   }
 }
 
@@ -476,37 +461,31 @@ int lu_permutation(const int32_t* d_ipiv, int n, std::vector<int32_t>& perm, cud
 
 template <typename T>
 int lu_trsv_prepare(const T* d_LU, int n, TrsvBlocks<T>& blk, cudaStream_t st, bool transposed) {
-  const int nb = (n + TSB - 1) / TSB;
-  const size_t need = (size_t)nb * TSB * TSB;
+  const int nb = (n + TW - 1) / TW;
+  const size_t need = (size_t)nb * TW * TW;
   if (blk.invL.count < need) {
     TT_TRY(blk.invL.alloc(need));
     TT_TRY(blk.invU.alloc(need));
-    TT_TRY(blk.mL.alloc(need));
-    TT_TRY(blk.mU.alloc(need));
+  }
+  if (!blk.rec.ptr) {
+    const size_t bytes = (size_t)(2 + X_SLOTS) * RHS * TW * LL<T>::BYTES;
+    TT_TRY(blk.rec.alloc(bytes));
+    TT_TRY(blk.err.alloc(1));
+    TT_CUDA_TRY(cudaMemsetAsync(blk.err.ptr, 0, sizeof(int), st));
+    TT_CUDA_TRY(cudaMemsetAsync(blk.rec.ptr, 0, bytes, st));
+    blk.epoch = 0;
   }
   blk.n = n;
-  ProfScope prof(TT_PROF_SUBST_PREP, st, 0.0, 2.0 * (double)n * TSB * sizeof(T));
-  const size_t smem = (size_t)TSB * TLD * sizeof(T);
-  TT_TRY(smem_limit_once((const void*)k_inv_diag<T, false, true>, (int)(smem)));
-  TT_TRY(smem_limit_once((const void*)k_inv_diag<T, true, false>, (int)(smem)));
-  TT_TRY(smem_limit_once((const void*)k_inv_diag<T, false, false>, (int)(smem)));
-  TT_TRY(smem_limit_once((const void*)k_inv_diag<T, true, true>, (int)(smem)));
-  TT_TRY(smem_limit_once((const void*)k_prev_mul<T, false>, (int)(2 * smem)));
-  TT_TRY(smem_limit_once((const void*)k_prev_mul<T, true>, (int)(2 * smem)));
+  ProfScope prof(TT_PROF_SUBST_PREP, st, 0.0, 2.0 * (double)n * TW * sizeof(T));
+  const size_t smem = (size_t)3 * TSB * TLD * sizeof(T);
+  const dim3 grid(nb, 2);
   if (!transposed) {
-    k_inv_diag<T, false, true><<<nb, 512, smem, st>>>(d_LU, n, blk.invL.ptr);
-    count_launch();
-    k_inv_diag<T, true, false><<<nb, 512, smem, st>>>(d_LU, n, blk.invU.ptr);
-    count_launch();
+    TT_TRY(smem_limit_once((const void*)k_inv_blocks<T, false>, (int)smem));
+    k_inv_blocks<T, false><<<grid, 512, smem, st>>>(d_LU, n, blk.invL.ptr, blk.invU.ptr);
   } else {
-    k_inv_diag<T, false, false><<<nb, 512, smem, st>>>(d_LU, n, blk.invL.ptr);
-    count_launch();
-    k_inv_diag<T, true, true><<<nb, 512, smem, st>>>(d_LU, n, blk.invU.ptr);
-    count_launch();
+    TT_TRY(smem_limit_once((const void*)k_inv_blocks<T, true>, (int)smem));
+    k_inv_blocks<T, true><<<grid, 512, smem, st>>>(d_LU, n, blk.invL.ptr, blk.invU.ptr);
   }
-  k_prev_mul<T, false><<<nb, 512, 2 * smem, st>>>(d_LU, n, blk.invL.ptr, blk.mL.ptr);
-  count_launch();
-  k_prev_mul<T, true><<<nb, 512, 2 * smem, st>>>(d_LU, n, blk.invU.ptr, blk.mU.ptr);
   count_launch();
   TT_CUDA_TRY(cudaGetLastError());
   return TT_OK;
@@ -514,11 +493,13 @@ int lu_trsv_prepare(const T* d_LU, int n, TrsvBlocks<T>& blk, cudaStream_t st, b
 template int lu_trsv_prepare<double2>(const double2*, int, TrsvBlocks<double2>&, cudaStream_t, bool);
 template int lu_trsv_prepare<float2>(const float2*, int, TrsvBlocks<float2>&, cudaStream_t, bool);
 
-// forward then backward substitution sweeps over x_b [k][n] in place for the
-// B factors of a batch (one cooperative launch per sweep for all of them)
+// Forward then backward substitution of the right-hand sides x_b [k][n] in place,
+// for the B factors of a batch (one cooperative launch per sweep for all of them):
+// row r of the forward sweep's right-hand side is row in_perm[r] of x_b, row r of
+// the solution goes to out_perm[r] (null: r).
 template <typename T>
-int trsv_sweeps_batched(int B, const T* const* d_LU, int n, const TrsvBlocks<T>* const* blk, double2* const* x,
-                        int nrhs, cudaStream_t st) {
+int trsv_sweeps(int B, const T* const* d_LU, int n, TrsvBlocks<T>* const* blk, double2* const* x,
+                const int32_t* const* in_perm, const int32_t* const* out_perm, int nrhs, cudaStream_t st) {
   if (B < 1 || B > kMaxSweeps) {
     set_error("substitution batch of " + std::to_string(B) + " factors (1.." + std::to_string(kMaxSweeps) + ")");
     return TT_ERR_BADARG;
@@ -528,109 +509,121 @@ int trsv_sweeps_batched(int B, const T* const* d_LU, int n, const TrsvBlocks<T>*
       set_error("triangular solve called without the inverted diagonal blocks of this factor");
       return TT_ERR_BADARG;
     }
-  const int Gb = std::max(2, device_sm_count() / B);
-  const int nb = (n + TSB - 1) / TSB;
-  int own_max = std::max(1, (nb - 2 + (Gb - 1) - 1) / (Gb - 1));
-  const size_t smem = (size_t)2 * TSB * TLD * sizeof(T) + (size_t)own_max * RHS * TSB * sizeof(T);
-  constexpr size_t kMaxSmem = 212 * 1024;  // + up to 12 KB static, within the 227 KB per CTA
+  // CTAs of a factor: the leads, and owners of at least 64 rows (one turn of their warps)
+  const int most = device_sm_count() / B;
+  const int Gb = LEADS + std::max(1, std::min({most - LEADS, (n + 63) / 64, (X_SLOTS - 1) * TW / 2}));
+  const int pairs = ceil_div((n + 1) / 2, Gb - LEADS);
+  const size_t smem = ((size_t)2 * RHS * TW + (size_t)pairs * 2 * RHS) * sizeof(T);
+  constexpr size_t kMaxSmem = 224 * 1024;
   if (smem > kMaxSmem) {
     if (B > 1) {
       // fewer owners per factor would not hold their rows: one factor at a time
-      for (int b = 0; b < B; b++) TT_TRY(trsv_sweeps_batched<T>(1, d_LU + b, n, blk + b, x + b, nrhs, st));
+      for (int b = 0; b < B; b++)
+        TT_TRY(trsv_sweeps<T>(1, d_LU + b, n, blk + b, x + b, in_perm + b, out_perm + b, nrhs, st));
       return TT_OK;
     }
     set_error("triangular solve: n = " + std::to_string(n) + " needs " + std::to_string(smem) +
               " bytes of shared memory per CTA (limit " + std::to_string(kMaxSmem) + ")");
     return TT_ERR_UNSUPPORTED;
   }
-  TT_TRY(smem_limit_once((const void*)k_trsv<T, false>, (int)kMaxSmem));
-  TT_TRY(smem_limit_once((const void*)k_trsv<T, true>, (int)kMaxSmem));
+  // a lane's pairs of complex64 need rows on 16-byte boundaries
+  bool wide = n % 2 == 0;
+  for (int b = 0; b < B; b++) wide = wide && (uintptr_t)d_LU[b] % 16 == 0;
+  const void* lower = wide ? (const void*)k_trsv<T, false, true> : (const void*)k_trsv<T, false, false>;
+  const void* upper = wide ? (const void*)k_trsv<T, true, true> : (const void*)k_trsv<T, true, false>;
+  TT_TRY(smem_limit_once(lower, (int)kMaxSmem));
+  TT_TRY(smem_limit_once(upper, (int)kMaxSmem));
+  DevBuf<double2> mid;  // between the sweeps
+  TT_TRY(mid.alloc((size_t)B * n * std::min(nrhs, RHS)));
+  const unsigned nb = (unsigned)((n + TW - 1) / TW);
   for (int k0 = 0; k0 < nrhs; k0 += RHS) {
     int kn = std::min(RHS, nrhs - k0);
     TrsvBatch<T> bl{}, bu{};
     bl.B = bu.B = B;
     for (int b = 0; b < B; b++) {
+      if (blk[b]->epoch > 0xF0000000u) {  // tags about to run out: start over
+        TT_CUDA_TRY(cudaMemsetAsync(blk[b]->rec.ptr, 0, blk[b]->rec.count, st));
+        blk[b]->epoch = 0;
+      }
       bl.LU[b] = bu.LU[b] = d_LU[b];
       bl.inv[b] = blk[b]->invL.ptr;
       bu.inv[b] = blk[b]->invU.ptr;
-      bl.Mp[b] = blk[b]->mL.ptr;
-      bu.Mp[b] = blk[b]->mU.ptr;
-      bl.x[b] = bu.x[b] = x[b] + (size_t)k0 * n;
+      bl.in[b] = x[b] + (size_t)k0 * n;
+      bl.in_perm[b] = in_perm[b];
+      bl.out[b] = mid.ptr + (size_t)b * n * std::min(nrhs, RHS);
+      bu.in[b] = bl.out[b];
+      bu.out[b] = x[b] + (size_t)k0 * n;
+      bu.out_perm[b] = out_perm[b];
+      bl.err[b] = bu.err[b] = blk[b]->err.ptr;
+      bl.rec[b] = bu.rec[b] = blk[b]->rec.ptr;
+      bl.epoch[b] = blk[b]->epoch;
+      bu.epoch[b] = blk[b]->epoch + nb;
+      blk[b]->epoch += 2 * nb;
     }
     int nn = n;
-    void* argsL[] = {&bl, &nn, &kn, &own_max};
-    TT_CUDA_TRY(cudaLaunchCooperativeKernel((void*)k_trsv<T, false>, dim3(Gb * B), dim3(TRSV_THREADS), argsL, smem,
-                                            st));
+    void* argsL[] = {&bl, &nn, &kn};
+    TT_CUDA_TRY(cudaLaunchCooperativeKernel(lower, dim3(Gb * B), dim3(TRSV_THREADS), argsL, smem, st));
     count_launch();
-    void* argsU[] = {&bu, &nn, &kn, &own_max};
-    TT_CUDA_TRY(cudaLaunchCooperativeKernel((void*)k_trsv<T, true>, dim3(Gb * B), dim3(TRSV_THREADS), argsU, smem,
-                                            st));
+    void* argsU[] = {&bu, &nn, &kn};
+    TT_CUDA_TRY(cudaLaunchCooperativeKernel(upper, dim3(Gb * B), dim3(TRSV_THREADS), argsU, smem, st));
     count_launch();
   }
   return TT_OK;
 }
 
 template <typename T>
-int trsv_sweeps(const T* d_LU, int n, const TrsvBlocks<T>& blk, double2* x, int nrhs, cudaStream_t st) {
-  const TrsvBlocks<T>* pb = &blk;
-  return trsv_sweeps_batched<T>(1, &d_LU, n, &pb, &x, nrhs, st);
+int lu_trsv_check(const TrsvBlocks<T>& blk, cudaStream_t st) {
+  if (!blk.err.ptr) return TT_OK;
+  int bad = 0;
+  TT_CUDA_TRY(cudaMemcpyAsync(&bad, blk.err.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  TT_CUDA_TRY(cudaStreamSynchronize(st));
+  if (bad) {
+    set_error("triangular solve timed out waiting for a block of the solution");
+    return TT_ERR_CUDA;
+  }
+  return TT_OK;
 }
+template int lu_trsv_check<float2>(const TrsvBlocks<float2>&, cudaStream_t);
+template int lu_trsv_check<double2>(const TrsvBlocks<double2>&, cudaStream_t);
 
 template <typename T>
-int lu_solve_batched_device(int B, const T* const* d_LU, int n, const TrsvBlocks<T>* const* blk,
-                            const int32_t* const* d_perm, double* const* d_x, double* d_tmp, int nrhs,
-                            cudaStream_t st) {
+int lu_solve_batched_device(int B, const T* const* d_LU, int n, TrsvBlocks<T>* const* blk,
+                            const int32_t* const* d_perm, double* const* d_x, int nrhs, cudaStream_t st) {
   if (n <= 0 || nrhs <= 0 || B <= 0) return TT_OK;
   ProfScope prof(TT_PROF_TRSV, st, 8.0 * n * (double)n * nrhs * B, (double)n * n * sizeof(T) * B);
   double2* xs[kMaxSweeps];
-  for (int b = 0; b < B; b++) {
-    TT_CUDA_TRY(cudaMemcpyAsync(d_tmp, d_x[b], sizeof(double2) * (size_t)n * nrhs, cudaMemcpyDeviceToDevice, st));
-    xs[b] = reinterpret_cast<double2*>(d_x[b]);
-    k_permute<<<ceil_div((size_t)n * nrhs, 256), 256, 0, st>>>(reinterpret_cast<const double2*>(d_tmp), d_perm[b],
-                                                              n, nrhs, xs[b]);
-    count_launch();
-    TT_CUDA_TRY(cudaGetLastError());
-  }
-  return trsv_sweeps_batched<T>(B, d_LU, n, blk, xs, nrhs, st);
+  const int32_t* none[kMaxSweeps] = {};
+  for (int b = 0; b < std::min(B, kMaxSweeps); b++) xs[b] = reinterpret_cast<double2*>(d_x[b]);
+  return trsv_sweeps<T>(B, d_LU, n, blk, xs, d_perm, none, nrhs, st);
 }
-template int lu_solve_batched_device<float2>(int, const float2* const*, int, const TrsvBlocks<float2>* const*,
-                                             const int32_t* const*, double* const*, double*, int, cudaStream_t);
+template int lu_solve_batched_device<float2>(int, const float2* const*, int, TrsvBlocks<float2>* const*,
+                                             const int32_t* const*, double* const*, int, cudaStream_t);
 
 template <typename T>
-int lu_solve_device(const T* d_LU, int n, const TrsvBlocks<T>& blk, const int32_t* d_perm, double* d_x,
-                    double* d_tmp, int nrhs, cudaStream_t st) {
-  if (n <= 0 || nrhs <= 0) return TT_OK;
-  ProfScope prof(TT_PROF_TRSV, st, 8.0 * n * (double)n * nrhs, (double)n * n * sizeof(T));
-  TT_CUDA_TRY(cudaMemcpyAsync(d_tmp, d_x, sizeof(double2) * (size_t)n * nrhs, cudaMemcpyDeviceToDevice, st));
-  double2* x = reinterpret_cast<double2*>(d_x);
-  k_permute<<<ceil_div((size_t)n * nrhs, 256), 256, 0, st>>>(reinterpret_cast<const double2*>(d_tmp), d_perm, n,
-                                                            nrhs, x);
-  count_launch();
-  TT_CUDA_TRY(cudaGetLastError());
-  return trsv_sweeps<T>(d_LU, n, blk, x, nrhs, st);
+int lu_solve_device(const T* d_LU, int n, TrsvBlocks<T>& blk, const int32_t* d_perm, double* d_x, int nrhs,
+                    cudaStream_t st) {
+  TrsvBlocks<T>* pb = &blk;
+  return lu_solve_batched_device<T>(1, &d_LU, n, &pb, &d_perm, &d_x, nrhs, st);
 }
 
 template <typename T>
-int lu_solve_transposed_device(const T* d_LUt, int n, const TrsvBlocks<T>& blkT, const int32_t* d_perm, double* d_x,
-                               double* d_tmp, int nrhs, cudaStream_t st) {
+int lu_solve_transposed_device(const T* d_LUt, int n, TrsvBlocks<T>& blkT, const int32_t* d_perm, double* d_x,
+                               int nrhs, cudaStream_t st) {
   if (n <= 0 || nrhs <= 0) return TT_OK;
   ProfScope prof(TT_PROF_TRSV, st, 8.0 * n * (double)n * nrhs, (double)n * n * sizeof(T));
+  // x[perm[r]] = row r: the row interchanges applied backwards
+  TrsvBlocks<T>* pb = &blkT;
   double2* x = reinterpret_cast<double2*>(d_x);
-  TT_TRY(trsv_sweeps<T>(d_LUt, n, blkT, x, nrhs, st));
-  TT_CUDA_TRY(cudaMemcpyAsync(d_tmp, d_x, sizeof(double2) * (size_t)n * nrhs, cudaMemcpyDeviceToDevice, st));
-  k_permute_inv<<<ceil_div((size_t)n * nrhs, 256), 256, 0, st>>>(reinterpret_cast<const double2*>(d_tmp), d_perm, n,
-                                                                nrhs, x);
-  count_launch();
-  TT_CUDA_TRY(cudaGetLastError());
-  return TT_OK;
+  const int32_t* none = nullptr;
+  return trsv_sweeps<T>(1, &d_LUt, n, &pb, &x, &none, &d_perm, nrhs, st);
 }
-template int lu_solve_transposed_device<double2>(const double2*, int, const TrsvBlocks<double2>&, const int32_t*,
-                                                 double*, double*, int, cudaStream_t);
-template int lu_solve_transposed_device<float2>(const float2*, int, const TrsvBlocks<float2>&, const int32_t*,
-                                                double*, double*, int, cudaStream_t);
-template int lu_solve_device<double2>(const double2*, int, const TrsvBlocks<double2>&, const int32_t*, double*,
-                                      double*, int, cudaStream_t);
-template int lu_solve_device<float2>(const float2*, int, const TrsvBlocks<float2>&, const int32_t*, double*,
-                                     double*, int, cudaStream_t);
+template int lu_solve_transposed_device<double2>(const double2*, int, TrsvBlocks<double2>&, const int32_t*, double*,
+                                                 int, cudaStream_t);
+template int lu_solve_transposed_device<float2>(const float2*, int, TrsvBlocks<float2>&, const int32_t*, double*, int,
+                                                cudaStream_t);
+template int lu_solve_device<double2>(const double2*, int, TrsvBlocks<double2>&, const int32_t*, double*, int,
+                                      cudaStream_t);
+template int lu_solve_device<float2>(const float2*, int, TrsvBlocks<float2>&, const int32_t*, double*, int,
+                                     cudaStream_t);
 
 }  // namespace tt

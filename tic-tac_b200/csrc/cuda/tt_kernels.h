@@ -97,37 +97,41 @@ int lu_factor_batched_device(T* const* d_L, int B, int n, int32_t* const* d_ipiv
                              int inv_block = 0, bool cta_pairs = false, int mid = 0);
 // Row permutation of the interchange sequence ipiv (host, once per factorisation).
 int lu_permutation(const int32_t* d_ipiv, int n, std::vector<int32_t>& perm, cudaStream_t st);
-// Inverted diagonal blocks of one LU factor (unit lower and upper) and their
-// products with the neighbouring off-diagonal blocks, made by lu_trsv_prepare
-// after each factorisation and read by every solve with it.
+// Inverted 128 x 128 diagonal blocks of one LU factor, made by lu_trsv_prepare
+// after each factorisation and read by every solve with it, and the records its
+// sweeps pass the solved blocks through.
 template <typename T>
 struct TrsvBlocks {
-  DevBuf<T> invL, invU;  // inverted 64 x 64 diagonal blocks
-  DevBuf<T> mL, mU;      // inv[b] times the block that carries the previous solved block into b
+  DevBuf<T> invL, invU;
+  DevBuf<unsigned char> rec;
+  unsigned epoch = 0;  // tags used so far
+  DevBuf<int> err;     // set when a wait of a sweep ran out
   int n = 0;
 };
 // transposed = true: d_LU holds the transpose of a factor (non-unit lower,
 // unit upper), for lu_solve_transposed_device.
 template <typename T>
 int lu_trsv_prepare(const T* d_LU, int n, TrsvBlocks<T>& blk, cudaStream_t st, bool transposed = false);
+// TT_ERR_CUDA if a wait of any solve with blk ran out.  Synchronises.
+template <typename T>
+int lu_trsv_check(const TrsvBlocks<T>& blk, cudaStream_t st);
 // Solve L U x = P b for nrhs complex128 columns [k][n] in place using the factor
-// of type T; d_perm from lu_permutation (uploaded), d_tmp scratch of 2 n nrhs doubles.
+// of type T; d_perm from lu_permutation (uploaded).
 template <typename T>
-int lu_solve_device(const T* d_LU, int n, const TrsvBlocks<T>& blk, const int32_t* d_perm, double* d_x,
-                    double* d_tmp, int nrhs, cudaStream_t st);
-// The same for B <= 4 factors of order n at once (their substitution sweeps
-// share each cooperative launch and grid barrier): x_b with factor b.
+int lu_solve_device(const T* d_LU, int n, TrsvBlocks<T>& blk, const int32_t* d_perm, double* d_x, int nrhs,
+                    cudaStream_t st);
+// The same for B <= 4 factors of order n at once (one cooperative launch per
+// sweep for all): x_b with factor b.
 template <typename T>
-int lu_solve_batched_device(int B, const T* const* d_LU, int n, const TrsvBlocks<T>* const* blk,
-                            const int32_t* const* d_perm, double* const* d_x, double* d_tmp, int nrhs,
-                            cudaStream_t st);
+int lu_solve_batched_device(int B, const T* const* d_LU, int n, TrsvBlocks<T>* const* blk,
+                            const int32_t* const* d_perm, double* const* d_x, int nrhs, cudaStream_t st);
 
 // Solve (P^T L U)^T x = b, i.e. transposed systems of the same factor, for
 // nrhs complex128 columns [k][n] in place: d_LUt is the transpose of the
 // factor (transpose_inplace_device) with blkT from lu_trsv_prepare(..., true).
 template <typename T>
-int lu_solve_transposed_device(const T* d_LUt, int n, const TrsvBlocks<T>& blkT, const int32_t* d_perm, double* d_x,
-                               double* d_tmp, int nrhs, cudaStream_t st);
+int lu_solve_transposed_device(const T* d_LUt, int n, TrsvBlocks<T>& blkT, const int32_t* d_perm, double* d_x,
+                               int nrhs, cudaStream_t st);
 
 // P123 from the reference's host CSC (values, int rows, size_t column pointers)
 // to device CSR with ascending columns per row (csr_build.cu).

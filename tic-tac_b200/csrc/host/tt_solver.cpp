@@ -307,7 +307,7 @@ int ChannelSolver::solve_pade(const std::vector<int>& q_idx, const std::vector<i
 }
 
 int ChannelSolver::adjoint_energy(int j, int nE, int nd, const double* Gj, const int32_t* d_rows, const int32_t* d_perm,
-                                  double* tmp, const double* x, const SolveOptions& opt, void* F,
+                                  const double* x, const SolveOptions& opt, void* F,
                                   TrsvBlocks<float2>& tbT32, TrsvBlocks<double2>& tbT64, double* lam, double* yT,
                                   double* rT, double* u, double* g, double* w, double* h, double* dots,
                                   const AdjointRequest& adj, SolveReport& r, cudaStream_t st) {
@@ -317,8 +317,8 @@ int ChannelSolver::adjoint_energy(int j, int nE, int nd, const double* Gj, const
   // L, so the adjoint needs no second n x n buffer
   auto solve_t = [&](double* v) -> int {
     if (opt.mixed)
-      return lu_solve_transposed_device<float2>(static_cast<const float2*>(F), n, tbT32, d_perm, v, tmp, nd, st);
-    return lu_solve_transposed_device<double2>(static_cast<const double2*>(F), n, tbT64, d_perm, v, tmp, nd, st);
+      return lu_solve_transposed_device<float2>(static_cast<const float2*>(F), n, tbT32, d_perm, v, nd, st);
+    return lu_solve_transposed_device<double2>(static_cast<const double2*>(F), n, tbT64, d_perm, v, nd, st);
   };
   if (opt.mixed) {
     TT_TRY(transpose_inplace_device<float2>(static_cast<float2*>(F), n, st));
@@ -347,12 +347,14 @@ int ChannelSolver::adjoint_energy(int j, int nE, int nd, const double* Gj, const
         break;
       }
     }
+    TT_TRY(lu_trsv_check(tbT32, st));
     r.adjoint_refine_iters = std::max(r.adjoint_refine_iters, std::min(it, opt.refine_max_iter));
     if (!converged) {
       set_error("refinement of the adjoint solve did not converge (last |dx|/|x| = " + std::to_string(worst) + ")");
       return TT_ERR_NOCONVERGE;
     }
   }
+  if (!opt.mixed) TT_TRY(lu_trsv_check(tbT64, st));
   // g = 2 P123^T OP(C) lambda, w = e + G o x
   TT_TRY(block_apply_device(L_, L_.C.ptr, lam, nd, u, st));
   TT_TRY(spmv_t_device(P_, u, nd, g, st));
@@ -497,8 +499,7 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
   // right-hand sides, solutions and refinement vectors of a group's energies:
   // [q][d][n] complex128, energy q of the group, deuteron column d
   const size_t vec = (size_t)2 * n * nd;
-  DevBuf<double> b, x, y, res, tmp;
-  TT_TRY(tmp.alloc(vec));
+  DevBuf<double> b, x, y, res;
   TT_TRY(b.alloc(vec * B));
   TT_TRY(x.alloc(vec * B));
   if (opt.mixed) {
@@ -574,7 +575,7 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
     // the group's complex64 factors solved together (one sweep launch for all)
     auto solve_group = [&](const std::vector<int>& qs, double* v) -> int {
       const float2* F[4];
-      const TrsvBlocks<float2>* TB[4];
+      TrsvBlocks<float2>* TB[4];
       const int32_t* PD[4];
       double* X[4];
       for (size_t i = 0; i < qs.size(); i++) {
@@ -583,7 +584,7 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
         PD[i] = perm_d[qs[i]].ptr;
         X[i] = v + vec * qs[i];
       }
-      return lu_solve_batched_device<float2>((int)qs.size(), F, n, TB, PD, X, tmp.ptr, nd, st);
+      return lu_solve_batched_device<float2>((int)qs.size(), F, n, TB, PD, X, nd, st);
     };
     std::vector<int> all_q;
     for (int q = 0; q < nb; q++) {
@@ -595,10 +596,11 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
         all_q.push_back(q);
       } else {
         TT_TRY(lu_trsv_prepare<double2>(L64.ptr, n, tb64, st));
-        TT_TRY(lu_solve_device<double2>(L64.ptr, n, tb64, perm_d[q].ptr, x.ptr + vec * q, tmp.ptr, nd, st));
+        TT_TRY(lu_solve_device<double2>(L64.ptr, n, tb64, perm_d[q].ptr, x.ptr + vec * q, nd, st));
       }
     }
     if (opt.mixed) TT_TRY(solve_group(all_q, x.ptr));
+    else TT_TRY(lu_trsv_check(tb64, st));
     TT_CUDA_TRY(cudaStreamSynchronize(st));
     r.ms_solve += ms_since(t0);
     if (opt.mixed) {
@@ -642,6 +644,7 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
           }
         }
       }
+      for (int q = 0; q < nb; q++) TT_TRY(lu_trsv_check(tb32[q], st));
       r.ms_refine += ms_since(t0);
       for (int q = 0; q < nb; q++) {
         r.refine_iters = std::max(r.refine_iters, iters[q]);
@@ -668,7 +671,7 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
       const double* Gj = G_.ptr + (size_t)2 * n * j;
       double* xq = x.ptr + vec * q;
       if (adj && adj->n_theta > 0)
-        TT_TRY(adjoint_energy(j, nE, nd, Gj, cols.ptr + (size_t)q * nd, perm_d[q].ptr, tmp.ptr, xq, opt,
+        TT_TRY(adjoint_energy(j, nE, nd, Gj, cols.ptr + (size_t)q * nd, perm_d[q].ptr, xq, opt,
                               opt.mixed ? (void*)factor_of(q) : (void*)L64.ptr, tbT32, tbT64, lam.ptr, yT.ptr, rT.ptr,
                               u.ptr, g.ptr, w.ptr, h.ptr, dots.ptr, *adj, r, st));
       std::vector<double> hx(vec);
@@ -720,8 +723,8 @@ int ChannelSolver::backward(const AdjointRequest& adj, std::vector<double>& dU, 
   dU.assign((size_t)adj.n_theta * 2 * nd * nd * nE, 0.0);
   SolveReport r;
   const size_t vec = (size_t)2 * n * nd;
-  DevBuf<double> tmp, lam, yT, rT, u, g, w, h, dots;
-  for (DevBuf<double>* v : {&tmp, &lam, &yT, &rT, &u, &g, &w, &h}) TT_TRY(v->alloc(vec));
+  DevBuf<double> lam, yT, rT, u, g, w, h, dots;
+  for (DevBuf<double>* v : {&lam, &yT, &rT, &u, &g, &w, &h}) TT_TRY(v->alloc(vec));
   TT_TRY(dots.alloc((size_t)2 * nd * nd));
   TrsvBlocks<float2> tbT32;
   TrsvBlocks<double2> tbT64;
@@ -730,7 +733,7 @@ int ChannelSolver::backward(const AdjointRequest& adj, std::vector<double>& dU, 
   for (int j = 0; j < nE; j++) {
     void* F = kept_.opt.mixed ? (void*)(kept_.L32.ptr + (size_t)j * n * n) : (void*)kept_.L64.ptr;
     TT_TRY(adjoint_energy(j, nE, nd, G_.ptr + (size_t)2 * n * j, kept_.cols.ptr + (size_t)j * nd, kept_.perm[j].ptr,
-                          tmp.ptr, kept_.x.ptr + vec * j, kept_.opt, F, tbT32, tbT64, lam.ptr, yT.ptr, rT.ptr, u.ptr,
+                          kept_.x.ptr + vec * j, kept_.opt, F, tbT32, tbT64, lam.ptr, yT.ptr, rT.ptr, u.ptr,
                           g.ptr, w.ptr, h.ptr, dots.ptr, a, r, st));
   }
   // the factors were transposed in place by the adjoint solves
