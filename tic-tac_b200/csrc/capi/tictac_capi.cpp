@@ -2,7 +2,9 @@
 #include "tictac_b200.h"
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -13,6 +15,7 @@
 #include <memory>
 #include <sstream>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../cuda/tt_kernels.h"
@@ -41,6 +44,27 @@ namespace {
 int fail(int code, const std::string& msg) {
   set_error(msg);
   return code;
+}
+
+// Host memory that tt_free releases, on 2 MB boundaries where it is large, so that
+// its first touch can take huge pages.
+void* host_block(size_t bytes) {
+  constexpr size_t kHuge = size_t(2) << 20;
+  if (bytes < 2 * kHuge) return std::malloc(std::max<size_t>(bytes, 1));
+  bytes = (bytes + kHuge - 1) / kHuge * kHuge;
+  void* p = std::aligned_alloc(kHuge, bytes);
+  if (p) madvise(p, bytes, MADV_HUGEPAGE);
+  return p;
+}
+
+// f on a thread of its own, or here when none can be started
+template <typename F>
+void start_or_run(std::vector<std::thread>& threads, F f) {
+  try {
+    threads.emplace_back(f);
+  } catch (const std::exception&) {
+    f();
+  }
 }
 
 struct ChannelState {
@@ -324,17 +348,35 @@ int tt_fill_P123_arrays(double** val, int** row, int** col, size_t* nnz, int pro
   if (cudaMemcpy(rowptr.data(), P.rowptr.ptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost) != cudaSuccess)
     return fail(TT_ERR_CUDA, "copy of P123 row pointers failed");
   const size_t m = (size_t)P.nnz;
-  *val = (double*)std::malloc(sizeof(double) * std::max<size_t>(m, 1));
-  *row = (int*)std::malloc(sizeof(int) * std::max<size_t>(m, 1));
-  *col = (int*)std::malloc(sizeof(int) * std::max<size_t>(m, 1));
+  *val = static_cast<double*>(host_block(sizeof(double) * m));
+  *row = static_cast<int*>(host_block(sizeof(int) * m));
+  *col = static_cast<int*>(host_block(sizeof(int) * m));
   if (!*val || !*row || !*col) return fail(TT_ERR_NOMEM, "host allocation for P123 failed");
-  if (m) {
-    if (cudaMemcpy(*val, P.val.ptr, sizeof(double) * m, cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(*col, P.col.ptr, sizeof(int) * m, cudaMemcpyDeviceToHost) != cudaSuccess)
-      return fail(TT_ERR_CUDA, "copy of P123 failed");
-  }
-  for (int r = 0; r < n; r++)
-    for (int64_t e = rowptr[r]; e < rowptr[r + 1]; e++) (*row)[e] = r;
+  // the copies run at the pace of the pages' first touch (2.4 GB/s from one
+  // thread): several threads touch val and col, then fill in the row indices
+  // while this one copies
+  double* v = *val;
+  int *r = *row, *c = *col;
+  const int nt = m < (size_t(1) << 20) ? 1 : 8;
+  std::vector<std::thread> touch, rows;
+  auto touch_part = [=](int t) {
+    const size_t lo = m * t / nt, hi = m * (t + 1) / nt;
+    for (size_t e = lo; e < hi; e += 512) v[e] = 0;  // one per 4 KB page
+    for (size_t e = lo; e < hi; e += 1024) c[e] = 0;
+  };
+  auto row_part = [&rowptr, r, n, nt](int t) {
+    for (int i = (int)((int64_t)n * t / nt); i < (int)((int64_t)n * (t + 1) / nt); i++)
+      std::fill(r + rowptr[i], r + rowptr[i + 1], i);
+  };
+  for (int t = 1; t < nt; t++) start_or_run(touch, [=] { touch_part(t); });
+  if (nt > 1) touch_part(0);
+  for (std::thread& th : touch) th.join();
+  for (int t = 1; t < nt; t++) start_or_run(rows, [=] { row_part(t); });
+  const bool copied = m == 0 || (cudaMemcpy(v, P.val.ptr, sizeof(double) * m, cudaMemcpyDeviceToHost) == cudaSuccess &&
+                                 cudaMemcpy(c, P.col.ptr, sizeof(int) * m, cudaMemcpyDeviceToHost) == cudaSuccess);
+  row_part(0);
+  for (std::thread& th : rows) th.join();
+  if (!copied) return fail(TT_ERR_CUDA, "copy of P123 failed");
   *nnz = m;
   return TT_OK;
 }

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import weakref
 from ctypes import POINTER, byref, c_char_p, c_double, c_int, c_int32, c_int64, c_size_t, c_void_p
 
 import numpy as np
@@ -203,6 +204,13 @@ class PW:
         self.Nalpha = t.shape[0]
 
 
+def _owned_array(ptr, m):
+    """The library's m elements at ptr as an array that frees them with itself (no copy)."""
+    buf = (ptr._type_ * max(m, 1)).from_address(ctypes.addressof(ptr.contents))
+    weakref.finalize(buf, _lib.tt_free, ctypes.cast(ptr, c_void_p))
+    return np.frombuffer(buf, dtype=np.dtype(ptr._type_), count=m)
+
+
 def fill_P123_arrays(pw: PW, p_WP, q_WP, production_run=True, **rp_kw):
     """tt_fill_P123_arrays: row-major COO (row, col, val) of P123 built on the GPU."""
     lib = load()
@@ -217,14 +225,7 @@ def fill_P123_arrays(pw: PW, p_WP, q_WP, production_run=True, **rp_kw):
     _check(lib.tt_fill_P123_arrays(byref(val), byref(row), byref(col), byref(nnz), int(production_run), byref(fwp),
                                    byref(pw.s), byref(rp)))
     m = nnz.value
-    try:
-        v = np.ctypeslib.as_array(val, shape=(max(m, 1),))[:m].copy()
-        r = np.ctypeslib.as_array(row, shape=(max(m, 1),))[:m].copy()
-        c = np.ctypeslib.as_array(col, shape=(max(m, 1),))[:m].copy()
-    finally:
-        lib.tt_free(ctypes.cast(val, c_void_p))
-        lib.tt_free(ctypes.cast(row, c_void_p))
-        lib.tt_free(ctypes.cast(col, c_void_p))
+    v, r, c = (_owned_array(p, m) for p in (val, row, col))
     return r, c, v
 
 
@@ -257,14 +258,7 @@ def read_P123_h5(path, pw: PW, p_WP, q_WP):
     _check(lib.tt_read_P123_h5(os.fsencode(path), byref(val), byref(row), byref(col), byref(nnz), byref(fwp),
                                byref(pw.s)))
     m = nnz.value
-    try:
-        v = np.ctypeslib.as_array(val, shape=(max(m, 1),))[:m].copy()
-        r = np.ctypeslib.as_array(row, shape=(max(m, 1),))[:m].copy()
-        c = np.ctypeslib.as_array(col, shape=(max(m, 1),))[:m].copy()
-    finally:
-        lib.tt_free(ctypes.cast(val, c_void_p))
-        lib.tt_free(ctypes.cast(row, c_void_p))
-        lib.tt_free(ctypes.cast(col, c_void_p))
+    v, r, c = (_owned_array(p, m) for p in (val, row, col))
     return r, c, v
 
 
