@@ -60,9 +60,10 @@ int build_A_device(const DeviceLayout& L, const DeviceCSR& P, const int32_t* d_a
 // relative to rowptr[r] (n (Nalpha + 1) int32).
 int alpha_offsets_device(const DeviceLayout& L, const DeviceCSR& P, int32_t* d_aoff, cudaStream_t st);
 
-// L = 1 - A diag(G), complex, row-major; T = double2 (complex128) or float2 (complex64).
+// L_b = 1 - A diag(G_b), complex, row-major, for the nb <= 4 resolvents d_G [nb][n];
+// T = double2 (complex128) or float2 (complex64).
 template <typename T>
-int form_L_device(const double* d_A, const double* d_G, int n, T* d_L, cudaStream_t st);
+int form_L_device(const double* d_A, const double* d_G, int n, T* const* d_L, int nb, cudaStream_t st);
 
 // RHS columns b_k = A[:, cols[k]] as complex128, stored column-by-column [k][n].
 int gather_rhs_device(const double* d_A, int n, const int32_t* d_cols, int nrhs, double* d_b, cudaStream_t st);

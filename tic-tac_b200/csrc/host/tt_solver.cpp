@@ -530,8 +530,8 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
       for (int q = 0; q < nb; q++) {
         Ls[q] = L32all.ptr + (size_t)q * n * n;
         ps[q] = ipiv_all.ptr + (size_t)q * n;
-        TT_TRY(form_L_device<float2>(A_.ptr, G_.ptr + (size_t)2 * n * (g0 + q), n, Ls[q], st));
       }
+      TT_TRY(form_L_device<float2>(A_.ptr, G_.ptr + (size_t)2 * n * g0, n, Ls, nb, st));
       TT_CUDA_TRY(cudaStreamSynchronize(st));
       r.ms_form += ms_since(t0);
       t0 = std::chrono::steady_clock::now();
@@ -540,11 +540,11 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
                                               opt.inverse_block, opt.cta_pairs, opt.mid_panel));
       r.ms_factor += ms_since(t0);
     } else {
-      TT_TRY(form_L_device<double2>(A_.ptr, G_.ptr + (size_t)2 * n * g0, n, L64.ptr, st));
+      double2* L64p = L64.ptr;
+      TT_TRY(form_L_device<double2>(A_.ptr, G_.ptr + (size_t)2 * n * g0, n, &L64p, 1, st));
       TT_CUDA_TRY(cudaStreamSynchronize(st));
       r.ms_form += ms_since(t0);
       t0 = std::chrono::steady_clock::now();
-      double2* L64p = L64.ptr;
       int32_t* piv0 = ipiv_all.ptr;
       TT_TRY(lu_factor_batched_device<double2>(&L64p, 1, n, &piv0, st, 0, &info[0], opt.panel_blocked));
       r.ms_factor += ms_since(t0);
