@@ -60,15 +60,15 @@ def run_and_oracle_U(c, run, Np, Nq):
     return oracle.dense_solve(A, G, q_idx, oracle.deuterons(pw), Nq, Np)
 
 
-# the sub-panel kernel's layouts: one row per thread up to 480 rows of a CTA, two up
-# to 825; complex128 CTAs of up to 395 rows; the last sub-panel narrower than a
-# register block.  U to the refinement's and the suite's 1e-10 per element.
+# the sub-panel kernel's layouts: one CTA up to 480 rows, a cluster up to 7,680,
+# records in L2 beyond; complex128 CTAs of up to 395 rows; the last sub-panel narrower
+# than a register block.  U to the refinement's and the suite's 1e-10 per element.
 @pytest.mark.parametrize("Np,Nq", [(7, 5),     # n = 385: a substitution block of one row
                                    (6, 6),     # n = 396: two complex128 CTAs, last sub-panel 12 wide
-                                   (9, 5),     # n = 495: two rows per thread, last 15 wide
-                                   (15, 5),    # n = 825: the largest single complex64 CTA, last 25 wide
-                                   (19, 4),    # n = 836: two complex64 CTAs
-                                   (17, 10)])  # n = 1,870
+                                   (9, 5),     # n = 495: a cluster of two, last 15 wide
+                                   (15, 5),    # n = 825: a cluster of four, last 25 wide
+                                   (19, 4),    # n = 836
+                                   (17, 10)])  # n = 1,870: clusters of 8
 @pytest.mark.parametrize("batch", [1, 4])
 def test_subpanel_layouts(Np, Nq, batch):
     from conftest import rel_elem
@@ -174,3 +174,19 @@ def test_A_build_chunks(Np, Nq, j):
     run.build_A(0)
     assert rel(run.A(0), A_o) <= 1e-12
     run.close()
+
+
+def test_tall_subpanels_of_a_batch():
+    # four matrices of order 18,207 share 148 CTAs, 37 each and two rows a thread;
+    # one at a time they take 38 CTAs and a row a thread.  The same operations on
+    # every element either way
+    opts = dict(potential_model="LO_internal", J_2N_max=3, two_J_3N_max=7, Np_WP=17, Nq_WP=17, lab_energies="5,30",
+                Nphi=12, Nx=12)
+    U = []
+    for batch in (1, 4):
+        run = tt.Run(**opts, energy_batch=batch)
+        c = run.num_channels - 1
+        assert run.channel_info(c)["n"] == 18_207 and len(run.energies()[0]) == 4
+        U.append(run.solve(c, tt.PRECISION_MIXED)[0])
+        run.close()
+    assert np.array_equal(U[0], U[1])

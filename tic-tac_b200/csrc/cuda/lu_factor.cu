@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(256) k_subpanel(T* __restrict__ A, int n, int 
 // launch runs without waiting.
 constexpr int LL_ONE_HOP = 32;
 constexpr int LL_SPINS = 1 << 20;
+constexpr size_t SP_CLUSTER_ROWS = 256;  // rows of a CTA in a cluster, where 16 suffice
 constexpr int SP_ROWS = 480;  // rows of a CTA, where the CTAs suffice: one per thread of 15 warps
 constexpr int LL_PER_WARP = 4;  // posted rows that a warp gathers, the diagonal row among them
 
@@ -350,12 +351,36 @@ inline int sp_rpt(int rows) { return rows > 32 * (SP_WARPS - 1) ? 2 : 1; }
 inline int sp_threads(int rows) { return 32 * ((rows + 32 * sp_rpt(rows) - 1) / (32 * sp_rpt(rows)) + 1); }
 
 // Sub-panel rows [c0, n), columns [c0, c0 + w) of bt.B matrices, Gb = gridDim.x / B
-// CTAs each (group b works on matrix b); at least IB rows in the first CTA.
+// consecutive CTAs each (group b works on matrix b); at least IB rows in the first.
 // Warps but the last own rows, the last solves the block's U rows meanwhile.
 // With pk0 < pk1, the sub-panel's interchanges are also applied to the other
 // columns [pk0, c0) and [c0 + w, pk1) of its panel.  rec: [2][B][Gb + 1][IB]
 // records, zero before the factorisation.
-template <typename T, int RPT>
+// CLUSTER: a matrix's CTAs are one cluster of up to 16, which exchanges the rows
+// through distributed shared memory: the owner warp stores its row into every CTA,
+// and one cluster barrier takes the place of the records' trip through L2.  Taken for
+// 481 to 7,680 rows (complex128 396 to 6,320), a row per thread: 84 -> 67 us a
+// sub-panel there, complex128 101 -> 84 us.  Two rows a thread in 16 CTAs (to 13,200
+// rows) take 94 us against the records' 88, so taller sub-panels meet in L2.
+__device__ __forceinline__ void sp_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t sp_remote(const void* p, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void sp_store_remote(uint32_t a, float2 v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void sp_store_remote(uint32_t a, double2 v) {
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ void sp_store_remote(uint32_t a, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+template <typename T, int RPT, bool CLUSTER>
 __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<T> bt, int n, int c0, int w, int pk0,
                                                                   int pk1, unsigned char* __restrict__ rec) {
   using CF = SubpanelCfg<T>;
@@ -385,7 +410,8 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
   for (int r = warp; r < nr; r += NW)
     if (lane < w) sA[r * SP + lane] = A[(size_t)(c0 + lo + r) * n + c0 + lane];
   if (tid == 0) *sFlag = *(volatile int*)bt.err;
-  __syncthreads();
+  if (CLUSTER) sp_cluster_sync();  // every CTA's shared memory exists before the first store into it
+  else __syncthreads();
   // a[i][k]: column jj + k of this thread's row i, jj the column at work.  The
   // registers move down by one each column, so that one copy of the code serves
   // all of them; finished columns are in shared memory.
@@ -438,6 +464,16 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
       }
     }
   };
+  // the diagonal row to every CTA, one warp
+  auto post_top = [&](T v, T* top, int buf, unsigned tag) {
+    if (CLUSTER) {
+      for (int g = 0; g < Gb; g++) sp_store_remote(sp_remote(top + lane, g), v);
+    } else if (Gb > 1) {
+      LL<T>::post(slot(buf, Gb) + lane * LL<T>::BYTES, v, tag);
+    } else {
+      top[lane] = v;
+    }
+  };
   const bool one_hop = Gb <= LL_ONE_HOP && Gb < LL_PER_WARP * NW;
   load_block(0);
   for (int b0 = 0; b0 < w; b0 += CB) {
@@ -482,24 +518,23 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
       if (warp == (have ? owner_warp(idx - lo) : 0)) {
         T v = T{0, 0};
         if (have) v = row_values(idx - lo, jj, end);
-        if (Gb > 1) {
+        if (CLUSTER) {
+#pragma unroll 4
+          for (int g = 0; g < Gb; g++) {
+            sp_store_remote(sp_remote(rows + cta * RW + lane, g), v);
+            if (lane == 0) sp_store_remote(sp_remote(iAll + cta, g), have ? idx : NONE);
+          }
+        } else if (Gb > 1) {
           LL<T>::post(slot(buf, cta) + lane * LL<T>::BYTES, v,
                       (unsigned long long)tag | ((unsigned long long)(unsigned)(have ? idx : NONE) << 32));
         } else {
           rows[lane] = v;
         }
-        if (diag_best) {
-          if (Gb > 1) LL<T>::post(slot(buf, Gb) + lane * LL<T>::BYTES, v, tag);
-          else top[lane] = v;
-        }
+        if (diag_best) post_top(v, top, buf, tag);
       }
-      if (cta == 0 && !diag_best && warp == owner_warp(jj)) {
-        const T v = row_values(jj, jj, end);
-        if (Gb > 1) LL<T>::post(slot(buf, Gb) + lane * LL<T>::BYTES, v, tag);
-        else top[lane] = v;
-      }
+      if (cta == 0 && !diag_best && warp == owner_warp(jj)) post_top(row_values(jj, jj, end), top, buf, tag);
       // ---- the column's pivot row and the diagonal row, from all CTAs
-      if (Gb > 1) {
+      if (!CLUSTER && Gb > 1) {
         Key bk = 0;
         int bi = NONE;
         if (one_hop) {
@@ -566,9 +601,14 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
           iAll[warp] = bi;
         }
       }
-      __syncthreads();
+      if (CLUSTER) sp_cluster_sync();
+      else __syncthreads();
       int ww = 0;
-      if (Gb > 1) {
+      if (CLUSTER) {
+        idx = lane < Gb ? iAll[lane] : NONE;
+        key = idx != NONE ? pivot_key(rows[lane * RW + jj]) : Key(0);
+        ww = warp_best(key, idx);
+      } else if (Gb > 1) {
         key = lane < NW ? kAll[lane] : Key(0);
         idx = lane < NW ? iAll[lane] : NONE;
         ww = warp_best(key, idx);
@@ -1154,6 +1194,43 @@ int panel_gemm_sub(int mode, T* C, int ldc, const T* L, int ldl, const T* U, int
   return gemm_sub(C, ldc, L, ldl, U, ldu, M, N, K, st);
 }
 
+// Largest cluster of full-size sub-panel CTAs the device runs: 16, 8 or 1
+template <typename T>
+int subpanel_cluster() {
+  static int largest[16] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int& c = largest[dev & 15];
+  if (c) return c;
+  const void* k = (const void*)k_subpanel_ll<T, 1, true>;
+  const void* k2 = (const void*)k_subpanel_ll<T, sizeof(T) == 8 ? 2 : 1, true>;
+  for (const void* f : {k, k2})
+    if (smem_limit_once(f, (int)kSubpanelSmem) != TT_OK ||
+        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      return c = 1;
+    }
+  for (int g : {16, 8}) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = g;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(g);
+    cfg.blockDim = dim3(32 * SP_WARPS);
+    cfg.dynamicSmemBytes = kSubpanelSmem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0, n2 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n2, k2, &cfg) == cudaSuccess && n > 0 && n2 > 0)
+      return c = g;
+    cudaGetLastError();
+  }
+  return c = 1;
+}
+
 }  // namespace
 
 template <typename T>
@@ -1211,10 +1288,21 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   PivotScratch<T> scr{sval.ptr, sidx.ptr, srow.ptr, stop.ptr};
   using SC = SubpanelCfg<T>;
   // rows per thread: complex128 rows fill shared memory before they outnumber the threads
-  const void* sp_kernel[2] = {(const void*)k_subpanel_ll<T, 1>,
-                              sizeof(T) == 8 ? (const void*)k_subpanel_ll<T, sizeof(T) == 8 ? 2 : 1> : nullptr};
-  for (const void* k : sp_kernel)
-    if (k) TT_TRY(smem_limit_once(k, (int)kSubpanelSmem));
+  constexpr int RPT2 = sizeof(T) == 8 ? 2 : 1;
+  const void* sp_kernel[2][2] = {{(const void*)k_subpanel_ll<T, 1, false>, (const void*)k_subpanel_ll<T, RPT2, false>},
+                                 {(const void*)k_subpanel_ll<T, 1, true>, (const void*)k_subpanel_ll<T, RPT2, true>}};
+  for (const auto& row : sp_kernel)
+    for (const void* k : row) TT_TRY(smem_limit_once(k, (int)kSubpanelSmem));
+  const int max_cluster = subpanel_cluster<T>();
+  // CTAs of the cluster that holds m rows, a row per thread: the smallest power of
+  // two of about SP_CLUSTER_ROWS rows a CTA; 0: too tall, or one CTA holds them
+  const size_t one_row = std::min(SP_ROWS, SC::MAX_ROWS);  // rows of a CTA with a row per thread
+  auto cluster_ctas = [&](size_t m) -> int {
+    if (m <= one_row || m > one_row * max_cluster) return 0;
+    int g = 2;
+    while (g < max_cluster && (m + g - 1) / g > SP_CLUSTER_ROWS) g *= 2;
+    return g;
+  };
   // CTAs of a matrix of m rows, of at most `most`: one while its shared memory
   // holds them (no exchange through L2), else about SP_ROWS rows each; 0: too tall
   auto ctas = [&](size_t m, int most) -> int {
@@ -1223,7 +1311,8 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
     if (need > (size_t)most) return 0;
     return (int)std::min<size_t>(most, std::max<size_t>(need, (m + SP_ROWS - 1) / SP_ROWS));
   };
-  // the sub-panel of matrices [b0, b0 + nb) in one cooperative launch of gb CTAs each
+  // the sub-panel of matrices [b0, b0 + nb) in one launch of gb CTAs each (gb < 0: a
+  // cluster of -gb), cooperative where they meet in L2
   auto subpanel = [&](int b0, int nb, int j0, int w, int pk0, int pk1, int gb) -> int {
     SubpanelBatch<T> bt{};
     for (int b = 0; b < nb; b++) {
@@ -1236,10 +1325,28 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
     int nn = n, cc0 = j0, ww = w, p0 = pk0, p1 = pk1;
     unsigned char* rec = srec.ptr + rec_region * b0;
     void* args[] = {&bt, &nn, &cc0, &ww, &p0, &p1, &rec};
+    const bool cluster = gb < 0;  // -gb CTAs of one cluster
+    if (cluster) gb = -gb;
     const int chunk = (n - j0 + gb - 1) / gb;
-    TT_CUDA_TRY(cudaLaunchCooperativeKernel((void*)sp_kernel[sp_rpt(chunk) - 1], dim3(gb * nb),
-                                            dim3(sp_threads(chunk)), args, (size_t)chunk * SP * sizeof(T) + SC::EXTRA,
-                                            st));
+    const void* kernel = sp_kernel[cluster][sp_rpt(chunk) - 1];
+    const size_t smem = (size_t)chunk * SP * sizeof(T) + SC::EXTRA;
+    if (cluster) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = gb;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(gb * nb);
+      cfg.blockDim = dim3(sp_threads(chunk));
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      TT_CUDA_TRY(cudaLaunchKernelExC(&cfg, kernel, args));
+    } else {
+      TT_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(gb * nb), dim3(sp_threads(chunk)), args, smem, st));
+    }
     count_launch();
     return TT_OK;
   };
@@ -1249,6 +1356,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
     const size_t m = (size_t)(n - j0);
     const int together = ctas(m, G / B), alone = ctas(m, G);
     ProfScope prof(TT_PROF_SUBPANEL, st, 4.0 * m * w * w * B, 2.0 * m * w * sizeof(T) * B);
+    if (const int c = cluster_ctas(m)) return subpanel(0, B, j0, w, pk0, pk1, -c);
     if (together) return subpanel(0, B, j0, w, pk0, pk1, together);
     for (int b = 0; b < B; b++) {
       if (alone) {
