@@ -760,6 +760,69 @@ __device__ __forceinline__ void cfma_add(T& acc, T a, T b) {
   acc.y += a.x * b.y + a.y * b.x;
 }
 
+constexpr int INV32_LD = 34, INV32_SCRATCH = 256;  // of inv_unit32
+
+// One level of inv_unit32: per 32 x 32 block, the pairs of inverted H x H blocks are
+// joined by S = L21 X11, X21 = -X22 S, an output a thread.
+template <int NB, int H, int LD, typename T>
+__device__ __forceinline__ void inv_unit32_join(const T* L, T* X, T* S) {
+  constexpr int PAIRS = 16 / H, XLD = INV32_LD;
+#pragma unroll
+  for (int step = 0; step < 2; step++) {
+    for (int o = threadIdx.x; o < NB * PAIRS * H * H; o += 256) {
+      const int p = o / (H * H), r = o / H % H, c = o % H, q = p / PAIRS, i0 = p % PAIRS * 2 * H;
+      const T* a = step == 0 ? L + (32 * q + i0 + H + r) * LD + 32 * q + i0 : X + (32 * q + i0 + H + r) * XLD + i0 + H;
+      const T* b = step == 0 ? X + (32 * q + i0) * XLD + i0 + c : S + p * H * H + c;
+      T v[2];
+      v[0].x = v[0].y = v[1].x = v[1].y = 0;
+#pragma unroll
+      for (int k = 0; k < H; k++) {
+        if (step == 0)
+          cfma_add(v[k & 1], a[k], b[k * XLD]);
+        else
+          cfma_sub(v[k & 1], a[k], b[k * H]);
+      }
+      v[0].x += v[1].x;
+      v[0].y += v[1].y;
+      if (step == 0)
+        S[o] = v[0];
+      else
+        X[(32 * q + i0 + H + r) * XLD + i0 + c] = v[0];
+    }
+    __syncthreads();
+  }
+}
+
+// Inverses of the NB unit-lower 32 x 32 diagonal blocks of L (shared, row stride LD,
+// only entries below the diagonal are read) into X[NB 32][INV32_LD], zeros above the
+// diagonal; S: scratch of INV32_SCRATCH NB elements; 256 threads, synchronised at the
+// end.  Bound: latency.  A column a lane through all 32 rows took 21,000 clocks, each
+// row waiting for its sums over shared memory; 8 x 8 blocks in registers and two joins
+// take a tenth of that.
+template <int NB, int LD, typename T>
+__device__ __forceinline__ void inv_unit32(const T* L, T* X, T* S) {
+  if (threadIdx.x < NB * 32) {
+    const int c = threadIdx.x & 31, e = c & ~7, row0 = threadIdx.x & ~31;
+    const T* l = L + (row0 + e) * LD + row0 + e;
+    T v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      v[i].x = e + i == c ? 1 : 0;
+      v[i].y = 0;
+#pragma unroll
+      for (int j = 0; j < i; j++) cfma_sub(v[i], l[i * LD + j], v[j]);
+    }
+    T zero;
+    zero.x = zero.y = 0;
+    for (int i = 0; i < e; i++) X[(row0 + i) * INV32_LD + c] = zero;
+#pragma unroll
+    for (int i = 0; i < 8; i++) X[(row0 + e + i) * INV32_LD + c] = v[i];
+  }
+  __syncthreads();
+  inv_unit32_join<NB, 8, LD>(L, X, S);
+  inv_unit32_join<NB, 16, LD>(L, X, S);
+}
+
 // Matrices whose unit-lower blocks are inverted in the same launches: block
 // (blockIdx.y for the diagonal blocks, blockIdx.z / pairs for the joins)
 // picks matrix b, whose inverse is X + b w w and join scratch T + b w w / 2.
@@ -771,10 +834,12 @@ struct InvBatch {
 template <typename T>
 __global__ void __launch_bounds__(256) k_inv_diag32(InvBatch<T> ib, int n, int r0, int w, T* __restrict__ X) {
   __shared__ T sL[32][33];
-  __shared__ T sX[32][33];
+  __shared__ T sX[32][INV32_LD];
+  __shared__ T sS[INV32_SCRATCH];
   const T* __restrict__ A = ib.A[blockIdx.y];
   X += (size_t)blockIdx.y * w * w;
   const int i0 = blockIdx.x * 32, hi = min(32, w - i0);
+#pragma unroll
   for (int t = threadIdx.x; t < 32 * 32; t += 256) {
     const int i = t >> 5, j = t & 31;
     T l;
@@ -784,26 +849,16 @@ __global__ void __launch_bounds__(256) k_inv_diag32(InvBatch<T> ib, int n, int r
     sL[i][j] = l;
   }
   __syncthreads();
-  // one warp, lane = column c of the inverse: row i = e_i - sum_{j<i} L[i][j] X[j]
-  if (threadIdx.x < 32) {
-    const int c = threadIdx.x;
-    for (int i = 0; i < hi; i++) {
-      T v;
-      v.x = (i == c) ? 1 : 0;
-      v.y = 0;
-      for (int j = c; j < i; j++) cfma_sub(v, sL[i][j], sX[j][c]);
-      sX[i][c] = v;
-    }
-  }
-  __syncthreads();
+  inv_unit32<1, 33>(&sL[0][0], &sX[0][0], sS);
   // the whole 32-row band of X: the diagonal block, zeros elsewhere in the band
-  for (int t = threadIdx.x; t < hi * w; t += 256) {
-    const int i = t / w, c = t % w;
-    T v;
-    v.x = 0;
-    v.y = 0;
-    if (c >= i0 && c - i0 < hi && c - i0 <= i) v = sX[i][c - i0];
-    X[(size_t)(i0 + i) * w + c] = v;
+  for (int i = threadIdx.x >> 5; i < hi; i += 8) {
+    T* row = X + (size_t)(i0 + i) * w;
+    const int lane = threadIdx.x & 31;
+    T zero;
+    zero.x = zero.y = 0;
+    const T v = lane <= i ? sX[i][lane] : zero;
+#pragma unroll 4
+    for (int c = lane; c < w; c += 32) row[c] = c - lane == i0 ? v : zero;
   }
 }
 
@@ -1027,6 +1082,104 @@ __global__ void __launch_bounds__(256) k_trsm_blk(TrsmBatch<T> tb, int n, int r0
   }
 }
 
+// X <- L^{-1} X for the h x h unit-lower block (h = 32 NB <= 128) at (r0, r0) of each
+// matrix of the batch (blockIdx.y), X = rows [r0, r0 + h) of columns [cb, ce),
+// complex64, also packed as the B operand of the update that follows.  A CTA inverts
+// the 32 x 32 diagonal blocks (inv_unit32), then takes chunks of 8 columns: block by
+// block x_j = D_j^{-1} b_j, an element a thread, and L x_j off the rows below, L as
+// 16-byte broadcasts.  Bound: latency of these steps (8 columns a CTA, as narrow as a
+// 64-byte row segment allows).  It stands for the explicit inverse of a mid-panel's
+// block, a pack, a tensor-core product and another pack (66 -> 13 us on average at 128 x up to
+// 384, n = 16,128) and for k_trsm_blk's substitution row by row (10 -> 4 us at 32 x up to 96).
+constexpr int TR_MAX = 128, TR_COLS = 8, TR_XLD = TR_COLS + 1;
+template <int NB>
+constexpr size_t trsm_rows_smem() {
+  return sizeof(float2) * (32 * NB * (32 * NB + 2) + 32 * NB * TR_XLD + 32 * NB * INV32_LD + INV32_SCRATCH * NB);
+}
+__device__ __forceinline__ void tr_cp_async8(float2* dst, const float2* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+template <int NB>
+__global__ void __launch_bounds__(256) k_trsm_rows(TrsmBatch<float2> tb, int n, int r0, int cb, int ce, int pack_mode) {
+  constexpr int H = 32 * NB, LD = H + 2;
+  extern __shared__ __align__(16) unsigned char tr_raw[];
+  float2* sL = reinterpret_cast<float2*>(tr_raw);  // [H][LD]
+  float2* sX = sL + H * LD;                        // [H][TR_XLD]
+  float2* sD = sX + H * TR_XLD;                    // [H][INV32_LD]
+  float2* sS = sD + H * INV32_LD;
+  float2* A = tb.A[blockIdx.y];
+  void* WB = tb.WB + tb.plane * blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = threadIdx.x / TR_COLS, col = threadIdx.x % TR_COLS;
+  for (int i = warp; i < H; i += 8)
+    for (int q = 0; q <= i / 32; q++)
+      tr_cp_async8(sL + i * LD + 32 * q + lane, A + (size_t)(r0 + i) * n + r0 + 32 * q + lane);
+  for (int c0 = cb + blockIdx.x * TR_COLS; c0 < ce; c0 += gridDim.x * TR_COLS) {
+    const int c = c0 + col;
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+      const int i = 32 * q + row;
+      if (c < ce)
+        tr_cp_async8(sX + i * TR_XLD + col, A + (size_t)(r0 + i) * n + c);
+      else
+        sX[i * TR_XLD + col] = make_float2(0, 0);
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    if (c0 == cb + (int)blockIdx.x * TR_COLS) inv_unit32<NB, LD>(sL, sD, sS);
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+      const float2* Y = sD + (32 * j + row) * INV32_LD;
+      const float2* xj = sX + 32 * j * TR_XLD + col;
+      float2 v[2] = {make_float2(0, 0), make_float2(0, 0)};
+#pragma unroll 4
+      for (int k = 0; k < warp * 4; k += 2) {
+        const float4 y = *reinterpret_cast<const float4*>(Y + k);
+        cfma_add(v[0], make_float2(y.x, y.y), xj[k * TR_XLD]);
+        cfma_add(v[1], make_float2(y.z, y.w), xj[(k + 1) * TR_XLD]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (warp * 4 + u <= row) cfma_add(v[u & 1], Y[warp * 4 + u], xj[(warp * 4 + u) * TR_XLD]);
+      __syncthreads();
+      sX[(32 * j + row) * TR_XLD + col] = make_float2(v[0].x + v[1].x, v[0].y + v[1].y);
+      __syncthreads();
+      if (j + 1 < NB) {
+        constexpr int REST = NB > 1 ? NB - 1 : 1;
+        float2 a[REST];
+#pragma unroll
+        for (int u = 0; u < REST; u++)
+          if (j + 1 + u < NB) a[u] = sX[(32 * (j + 1 + u) + row) * TR_XLD + col];
+#pragma unroll 4
+        for (int k = 0; k < 32; k += 2) {
+          const float2 b0 = xj[k * TR_XLD], b1 = xj[(k + 1) * TR_XLD];
+#pragma unroll
+          for (int u = 0; u < REST; u++)
+            if (j + 1 + u < NB) {
+              const float4 l = *reinterpret_cast<const float4*>(sL + (32 * (j + 1 + u) + row) * LD + 32 * j + k);
+              cfma_sub(a[u], make_float2(l.x, l.y), b0);
+              cfma_sub(a[u], make_float2(l.z, l.w), b1);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < REST; u++)
+          if (j + 1 + u < NB) sX[(32 * (j + 1 + u) + row) * TR_XLD + col] = a[u];
+        __syncthreads();
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NB; q++)
+      if (c < ce) A[(size_t)(r0 + 32 * q + row) * n + c] = sX[(32 * q + row) * TR_XLD + col];
+    if (c0 + warp < ce) {
+#pragma unroll
+      for (int q = 0; q < NB; q++)
+        tc2_pack_b(pack_mode, WB, ce - cb, H, c0 + warp - cb, 32 * q + lane, sX[(32 * q + lane) * TR_XLD + warp]);
+    }
+    __syncthreads();
+  }
+}
+
 // C[M x N] -= L[M x K] U[K x N], complex, leading dimensions ld*; 64 x 64 tiles.
 template <typename T>
 __global__ void __launch_bounds__(256) k_gemm_sub(T* __restrict__ C, int ldc, const T* __restrict__ L, int ldl,
@@ -1172,6 +1325,35 @@ int trsm_blk_batched(T* const* As, int B, int n, int r0, int w, int cb, int ce, 
   count_launch();
   TT_CUDA_TRY(cudaGetLastError());
   return TT_OK;
+}
+
+// k_trsm_rows of B <= 4 matrices, h a multiple of 32 up to TR_MAX; one CTA an SM at
+// most, as its block inverses serve all its chunks
+template <int NB>
+int launch_trsm_rows(const TrsmBatch<float2>& tb, int B, int n, int r0, int cb, int ce, int pack_mode,
+                     cudaStream_t st) {
+  const int chunks = ceil_div(ce - cb, TR_COLS), per = std::max(1, device_sm_count() / B);
+  constexpr size_t smem = trsm_rows_smem<NB>();
+  TT_TRY(smem_limit_once((const void*)k_trsm_rows<NB>, (int)smem));
+  k_trsm_rows<NB><<<dim3(ceil_div(chunks, ceil_div(chunks, per)), B), 256, smem, st>>>(tb, n, r0, cb, ce, pack_mode);
+  count_launch();
+  TT_CUDA_TRY(cudaGetLastError());
+  return TT_OK;
+}
+int trsm_rows_batched(float2* const* As, int B, int n, int r0, int h, int cb, int ce, int pack_mode, unsigned char* WB,
+                      size_t plane, cudaStream_t st) {
+  ProfScope prof(TT_PROF_PANEL_TRSM, st, 4.0 * h * h * (double)(ce - cb) * B,
+                 2.0 * h * (double)(ce - cb) * sizeof(float2) * B);
+  TrsmBatch<float2> tb{};
+  for (int b = 0; b < B; b++) tb.A[b] = As[b];
+  tb.WB = WB;
+  tb.plane = plane;
+  switch (h / 32) {
+    case 1: return launch_trsm_rows<1>(tb, B, n, r0, cb, ce, pack_mode, st);
+    case 2: return launch_trsm_rows<2>(tb, B, n, r0, cb, ce, pack_mode, st);
+    case 3: return launch_trsm_rows<3>(tb, B, n, r0, cb, ce, pack_mode, st);
+    default: return launch_trsm_rows<4>(tb, B, n, r0, cb, ce, pack_mode, st);
+  }
 }
 
 template <typename T>
@@ -1504,9 +1686,14 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
           float2* Cs[kMaxBatch];
           const float2* Ls[kMaxBatch];
           const float2* Us[kMaxBatch];
-          TT_TRY(trsm_blk_batched<T>(As, B, n, j0, w, j0 + w, m0 + mw, st, mode, WB, plane));
+          float2* Af[kMaxBatch];
+          for (int b = 0; b < B; b++) Af[b] = reinterpret_cast<float2*>(As[b]);
+          if (w == 32)
+            TT_TRY(trsm_rows_batched(Af, B, n, j0, w, j0 + w, m0 + mw, mode, WB, plane, st));
+          else
+            TT_TRY(trsm_blk_batched<T>(As, B, n, j0, w, j0 + w, m0 + mw, st, mode, WB, plane));
           for (int b = 0; b < B; b++) {
-            float2* A = reinterpret_cast<float2*>(As[b]);
+            float2* A = Af[b];
             Cs[b] = A + (size_t)(j0 + w) * n + (j0 + w);
             Ls[b] = A + (size_t)(j0 + w) * n + j0;
             Us[b] = A + (size_t)j0 * n + (j0 + w);
@@ -1523,8 +1710,27 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
       }
       const int right_out = k + kb - (m0 + mw);
       if (right_out > 0) {
-        TT_TRY(trsm_all(m0, mw, m0 + mw, k + kb));
-        TT_TRY(gemm_all(m0 + mw, m0 + mw, m0 + mw, m0, m0, m0 + mw, n - m0 - mw, right_out, mw));
+        if (inv_solve && mw <= std::min(TR_MAX, IVB) && mw % 32 == 0) {
+          int ws = TT_OK;
+          unsigned char* WB = static_cast<unsigned char*>(tc2_b_workspace(mode, right_out, mw, &ws, B));
+          TT_TRY(ws);
+          float2* Cs[kMaxBatch];
+          const float2* Ls[kMaxBatch];
+          const float2* Us[kMaxBatch];
+          float2* Af[kMaxBatch];
+          for (int b = 0; b < B; b++) {
+            float2* A = Af[b] = reinterpret_cast<float2*>(As[b]);
+            Cs[b] = A + (size_t)(m0 + mw) * n + (m0 + mw);
+            Ls[b] = A + (size_t)(m0 + mw) * n + m0;
+            Us[b] = A + (size_t)m0 * n + (m0 + mw);
+          }
+          TT_TRY(trsm_rows_batched(Af, B, n, m0, mw, m0 + mw, k + kb, mode, WB, tc2_b_plane_bytes(mode, right_out, mw),
+                                  st));
+          TT_TRY(tc2_gemm_sub_batched(mode, B, Cs, n, Ls, n, Us, n, n - m0 - mw, right_out, mw, st, 0, true));
+        } else {
+          TT_TRY(trsm_all(m0, mw, m0 + mw, k + kb));
+          TT_TRY(gemm_all(m0 + mw, m0 + mw, m0 + mw, m0, m0, m0 + mw, n - m0 - mw, right_out, mw));
+        }
       }
     }
     // ---- interchanges outside the panel; U12 = L11^{-1} A12 with the
