@@ -60,11 +60,10 @@ def run_and_oracle_U(c, run, Np, Nq):
     return oracle.dense_solve(A, G, q_idx, oracle.deuterons(pw), Nq, Np)
 
 
-# the sub-panel kernel's layouts: one CTA up to 480 rows, a cluster up to 7,680,
-# records in L2 beyond; complex128 CTAs of up to 395 rows; the last sub-panel narrower
-# than a register block.  U to the refinement's and the suite's 1e-10 per element.
+# the sub-panel kernel's layouts: one CTA up to 224 rows, a cluster up to 4,096,
+# records in L2 beyond; the last sub-panel narrower than a register block.  U to the refinement's and the suite's 1e-10 per element.
 @pytest.mark.parametrize("Np,Nq", [(7, 5),     # n = 385: a substitution block of one row
-                                   (6, 6),     # n = 396: two complex128 CTAs, last sub-panel 12 wide
+                                   (6, 6),     # n = 396: a cluster of two, last sub-panel 12 wide
                                    (9, 5),     # n = 495: a cluster of two, last 15 wide
                                    (15, 5),    # n = 825: a cluster of four, last 25 wide
                                    (19, 4),    # n = 836
@@ -190,3 +189,39 @@ def test_tall_subpanels_of_a_batch():
         U.append(run.solve(c, tt.PRECISION_MIXED)[0])
         run.close()
     assert np.array_equal(U[0], U[1])
+
+
+# where a sub-panel's pivots lie: on the diagonal, off it but in the 32 x 32 diagonal
+# block, in a few columns below the block, or anywhere; each energy's matrix its own way.
+# n = 512: a cluster, then one CTA; n = 4,608: records in L2 first
+@pytest.mark.parametrize("Np,kinds", [(16, ("diagonal", "block", "below", "anywhere")), (16, ("anywhere", "anywhere")),
+                                      (48, ("below", "block"))])
+@pytest.mark.parametrize("precision", [tt.PRECISION_FP64, tt.PRECISION_MIXED, tt.PRECISION_MIXED_SIMT])
+def test_pivots_in_and_below_the_diagonal_block(precision, Np, kinds):
+    import torch
+
+    n, rng = 2 * Np * Np, np.random.default_rng(5)
+    pw = np.array([[0, 0, 0, 1, 0, 1, 1, 1, 1], [0, 1, 1, 0, 0, 1, 1, 1, 1]], dtype=np.int32)
+    eye, e = np.tile(np.eye(Np).ravel(), 6), np.tile(np.linspace(-2, 100, Np + 1), 6)
+    swp = tt.SWP(Np, Np, 6, 0, -2.0, e, None, eye, None, np.linspace(0, 1000, Np + 1))
+    # A = 2 P, strong within the 32 x 32 diagonal blocks and in the columns j of `far` at row j + 300
+    P = rng.standard_normal((n, n)) * (1e-2 / np.sqrt(n))
+    block = np.arange(n) // 32
+    P += np.where(block[:, None] == block[None, :], rng.standard_normal((n, n)), 0) * 2e-2
+    far = np.arange(17, n - 300, 97)
+    far = far[(far % 32 != 0) & (far % 7 != 0)]
+    scale = {"diagonal": 0.1, "block": 100.0, "below": 0.1, "anywhere": 3e4}
+    G = np.stack([scale[k] * np.exp(1j * rng.uniform(0, 2 * np.pi, n)) for k in kinds])
+    P[far + 300, far] = 1.0
+    for j, k in enumerate(kinds):
+        G[j, far] = 40.0 if k == "below" else 0.01
+    q_idx = np.arange(3, 3 + len(kinds))
+    rows = np.tile(np.arange(n, dtype=np.int32), n)
+    U, rep = tt.solve_faddeev(G, P.T.ravel(), rows, np.arange(0, n * n + 1, n, dtype=np.uint64), eye, None, swp, q_idx,
+                              [1], tt.PW(pw), precision=precision, tensor_force=0, isospin_breaking_1S0=0)
+    A = torch.from_numpy(2 * P).cuda()
+    for j in range(len(kinds)):
+        L = torch.eye(n, dtype=torch.complex128, device="cuda") - A * torch.from_numpy(G[j]).cuda()
+        row = Np * Np + int(q_idx[j]) * Np
+        want = torch.linalg.solve(L, A[:, row].to(L.dtype))[row].item()
+        assert abs(U[j] - want) <= 1e-10 * abs(want), (kinds[j], U[j], want, rep)

@@ -4,21 +4,23 @@
 //
 // Outer panels of NB columns (512 for the complex64 / tensor-core path, 128
 // for complex128).  Each panel is factored in IB = 32 column sub-panels:
-//   k_subpanel_ll  cooperative kernel with each block's rows on chip and no
-//                grid barrier: every block posts its best pivot row in tagged
-//                records that the others poll (k_subpanel: from global
-//                memory with a grid barrier per column, for sub-panels too
-//                tall for shared memory)
-//   k_laswp2     the sub-panel's interchanges on the rest of the panel
-//   k_trsm_blk   U = L^{-1} U for the 32-wide unit-lower diagonal block
-//   tc_gemm_sub / k_gemm_sub  rank-32 update of the remaining panel columns
-// then the panel's interchanges outside the panel, the blocked triangular
-// solve for U12 and the trailing update A22 -= L21 U12 (tcgen05 BF16x3 for
-// complex64, CUDA-core complex GEMM for complex128).
+//   k_subpanel_ll  each block's rows on chip and no grid barrier: tries pivots
+//                from the 32 x 32 diagonal block, checked against all rows, else
+//                every block posts its best pivot row of a column in tagged
+//                records that the others poll; also the sub-panel's interchanges
+//                on the rest of the panel (k_subpanel: from global memory with a
+//                grid barrier per column, for sub-panels too tall for shared
+//                memory)
+//   k_trsm_rows / k_trsm_blk  U = L^{-1} U for the unit-lower diagonal block
+//   the update of the remaining panel columns
+// then the panel's interchanges outside the panel (k_laswp2), the triangular
+// solve for U12 and the trailing update A22 -= L21 U12 (tcgen05 for complex64,
+// FP64 tensor cores for complex128).
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <functional>
+#include <type_traits>
 #include <vector>
 
 #include "ll_record.cuh"
@@ -58,6 +60,29 @@ __device__ __forceinline__ T cdiv_smith(T a, T b) {
   return r;
 }
 
+// acc -= a b and acc += a b, complex: two fused multiply-adds a component
+template <typename T>
+__device__ __forceinline__ void cfma_sub(T& acc, T a, T b) {
+  acc.x -= a.x * b.x;
+  acc.x += a.y * b.y;
+  acc.y -= a.x * b.y;
+  acc.y -= a.y * b.x;
+}
+template <typename T>
+__device__ __forceinline__ void cfma_add(T& acc, T a, T b) {
+  acc.x += a.x * b.x;
+  acc.x -= a.y * b.y;
+  acc.y += a.x * b.y;
+  acc.y += a.y * b.x;
+}
+template <typename T>
+__device__ __forceinline__ T cmul(T a, T b) {
+  T r;
+  r.x = a.x * b.x - a.y * b.y;
+  r.y = a.x * b.y + a.y * b.x;
+  return r;
+}
+
 constexpr int IB = 32;
 constexpr int SP = IB + 1;                     // shared-memory row stride of a staged sub-panel
 constexpr size_t kSubpanelSmem = 226 * 1024;  // shared memory of a CTA of the on-chip sub-panel kernel
@@ -81,6 +106,8 @@ struct SubpanelBatch {
   int32_t* ipiv[kMaxBatch];
   int* info;                           // [B]
   int* err;                            // set when a wait ran out
+  int* tries;                          // [B][2] sub-panels to come without a try, and how many after the next failure
+  unsigned char* verdict;              // [B][CTAs of a matrix] records: this CTA's rows agree with the try
   int B;
 };
 // a[i] by predicated selects: a runtime index into a kernel parameter array
@@ -249,19 +276,33 @@ __global__ void __launch_bounds__(256) k_subpanel(T* __restrict__ A, int n, int 
 // Records are double-buffered by column parity: a CTA posts column j + 2 only
 // after it has seen every CTA's column j + 1, posted after their reads of j.
 //
-// Per sub-panel of 32 columns, against the kernel before it (a row per warp in
-// shared memory, one cooperative grid barrier, an atomicMax and two dependent
-// reads per column), two complex64 matrices: n = 512 118 -> 43 us, n = 10,944
-// 134 -> 82 us, n = 16,128 139 -> 86 us, n = 42,300 201 -> 113 us; four at
-// n = 20,160 178 -> 97 us; one complex128 at n = 8,496 135 -> 101 us.  Of a
-// column's 2.5 to 6 thousand cycles the trips through L2 take about 1,200 each;
-// the rest is the latency of its own instructions.
+// Of a column's 2.5 to 6 thousand cycles the trips through L2 take about 1,200
+// each; the rest is the latency of its own instructions.
+//
+// The matrices are 1 - A G: all 32 pivots of a sub-panel lie in its 32 x 32 diagonal
+// block in 96 to 100% of the sub-panels, nearly always on the diagonal.  So the kernel
+// first tries that, without any exchange: every CTA factors the diagonal block for
+// itself (sp_factor_diag, and with interchanges in the block, sp_factor_block, where the
+// diagonal will not do), takes its own rows through the block's U (sp_try_row) and looks
+// at each element before its division: none may exceed the pivot of its column by the
+// same keys that the search compares.  One verdict a CTA, one trip, and if all agree these
+// are the search's pivots and its result.  Else the rows, still unchanged in A, are read
+// again for the search; a matrix whose tries fail in a row goes 1, 3, 7, then 15
+// sub-panels without one, so that a try (a fifth of a search) is lost on few.
+// Bound: the latency of the block's 32 steps (~5 us) and the rows' FP32 multiply-adds.
+//
+// Per sub-panel of 32 columns, search alone -> with tries, two complex64 matrices:
+// n = 10,944 82 -> 22 us, n = 16,128 80 -> 20 us, n = 42,300 113 -> 31 us; four at
+// n = 20,160 93 -> 28 us; one complex128 at n = 8,496 90 -> 29 us.
+// Rows of a CTA: 224 (eight warps, the count the block needs) against 480: channel of
+// n = 16,128 11.7 -> 10.3 ms in all, n = 42,300 43.5 -> 40.5 ms, complex128 17.6 -> 15.5.
 // Waits end after LL_SPINS polls: the error word is set and the rest of the
 // launch runs without waiting.
 constexpr int LL_ONE_HOP = 32;
 constexpr int LL_SPINS = 1 << 20;
-constexpr size_t SP_CLUSTER_ROWS = 256;  // rows of a CTA in a cluster, where 16 suffice
-constexpr int SP_ROWS = 480;  // rows of a CTA, where the CTAs suffice: one per thread of 15 warps
+constexpr size_t SP_CLUSTER_ROWS = 256;  // most rows of a CTA in a cluster
+constexpr int SP_ROWS = 224;  // rows of a CTA, where the CTAs suffice: one per thread of 7 warps
+constexpr int TRY_LD = IB + 2, TRY_THREADS = 256;  // row stride of the tried diagonal block; threads it takes
 constexpr int LL_PER_WARP = 4;  // posted rows that a warp gathers, the diagonal row among them
 
 // Pivot candidates as keys: 0 for none (NaN magnitudes included), else the bits
@@ -300,24 +341,26 @@ __device__ __forceinline__ int warp_best(K& key, int& row) {
 // range it is formed in without loss
 __device__ __forceinline__ float2 pivot_recip(float2 b) {
   const float big = fmaxf(fabsf(b.x), fabsf(b.y));
-  float sc = 1.0f;
+  float x = b.x, y = b.y, r = __frcp_rn(fmaf(x, x, y * y));
   if (!(big > 0x1p-50f && big < 0x1p50f)) {
     const int e = min(max((int)(__float_as_uint(big) >> 23) - 127, -126), 126);
-    sc = __uint_as_float((unsigned)(127 - e) << 23);
+    const float sc = __uint_as_float((unsigned)(127 - e) << 23);
+    x *= sc;
+    y *= sc;
+    r = sc * __frcp_rn(fmaf(x, x, y * y));
   }
-  const float x = b.x * sc, y = b.y * sc;
-  const float r = sc * __frcp_rn(fmaf(x, x, y * y));
   return make_float2(x * r, -y * r);
 }
 __device__ __forceinline__ double2 pivot_recip(double2 b) {
   const double big = fmax(fabs(b.x), fabs(b.y));
-  double sc = 1.0;
+  double x = b.x, y = b.y, r = __drcp_rn(fma(x, x, y * y));
   if (!(big > 0x1p-400 && big < 0x1p400)) {
     const int e = min(max((int)(((unsigned long long)__double_as_longlong(big)) >> 52) - 1023, -1022), 1022);
-    sc = __longlong_as_double((long long)((unsigned long long)(1023 - e) << 52));
+    const double sc = __longlong_as_double((long long)((unsigned long long)(1023 - e) << 52));
+    x *= sc;
+    y *= sc;
+    r = sc * __drcp_rn(fma(x, x, y * y));
   }
-  const double x = b.x * sc, y = b.y * sc;
-  const double r = sc * __drcp_rn(fma(x, x, y * y));
   return make_double2(x * r, -y * r);
 }
 
@@ -348,7 +391,265 @@ struct SubpanelCfg {
 };
 // rows per thread of a CTA of `rows` rows, and its threads: the row warps and one more
 inline int sp_rpt(int rows) { return rows > 32 * (SP_WARPS - 1) ? 2 : 1; }
-inline int sp_threads(int rows) { return 32 * ((rows + 32 * sp_rpt(rows) - 1) / (32 * sp_rpt(rows)) + 1); }
+inline int sp_threads(int rows) {
+  return std::max(TRY_THREADS, 32 * ((rows + 32 * sp_rpt(rows) - 1) / (32 * sp_rpt(rows)) + 1));
+}
+
+// LU of the sub-panel's w x w diagonal block in sD (row stride TRY_LD), every pivot on the
+// diagonal; false (to some thread) if an element of the block would have been the pivot.
+// Thread t of 256 keeps row t / 8, columns 4 (t % 8) to + 3.  A step takes four columns:
+// every thread factors their 4 x 4 diagonal block for itself, solves its own L row and U
+// columns against it and updates its four elements; what the next step reads goes to
+// shared memory, one barrier a step.  sRd, sBest: the pivots' reciprocals and keys.
+// Bound: the chain of 32 reciprocals.
+template <typename T, typename Key>
+__device__ __forceinline__ bool sp_factor_diag(T* sD, T* sRd, Key* sBest, int w, int tid) {
+  constexpr int W = 4;
+  const int i = tid >> 3, g = tid & 7, warp = tid >> 5;
+  bool ok = true;
+  T a[W];
+#pragma unroll
+  for (int c = 0; c < W; c++) a[c] = sD[i * TRY_LD + W * g + c];
+#pragma unroll 1
+  for (int s = 0; W * s < w; s++) {
+    const int j0 = W * s;
+    if (warp >= s && g >= s) {
+      T d[W][W], rd[W], l[W];
+#pragma unroll
+      for (int r = 0; r < W; r++)
+#pragma unroll
+        for (int c = 0; c < W; c++) d[r][c] = sD[(j0 + r) * TRY_LD + j0 + c];
+#pragma unroll
+      for (int c = 0; c < W; c++) l[c] = sD[i * TRY_LD + j0 + c];
+      Key best[W];
+#pragma unroll
+      for (int k = 0; k < W; k++) {
+        rd[k] = pivot_recip(d[k][k]);
+        best[k] = pivot_key(d[k][k]);
+#pragma unroll
+        for (int r = k + 1; r < W; r++) {
+          ok &= pivot_key(d[r][k]) <= best[k];
+          d[r][k] = cmul(d[r][k], rd[k]);
+#pragma unroll
+          for (int c = k + 1; c < W; c++) cfma_sub(d[r][c], d[r][k], d[k][c]);
+        }
+      }
+      // row i takes the pivots above it: all four below the diagonal block
+#pragma unroll
+      for (int k = 0; k < W; k++)
+        if (k < i - j0) {
+          ok &= pivot_key(l[k]) <= best[k];
+          l[k] = cmul(l[k], rd[k]);
+#pragma unroll
+          for (int c = k + 1; c < W; c++) cfma_sub(l[c], l[k], d[k][c]);
+        }
+      if (g > s) {
+#pragma unroll
+        for (int c = 0; c < W; c++) {
+          T u[W];
+#pragma unroll
+          for (int r = 0; r < W; r++) {
+            u[r] = sD[(j0 + r) * TRY_LD + W * g + c];
+#pragma unroll
+            for (int k = 0; k < r; k++) cfma_sub(u[r], d[r][k], u[k]);
+          }
+#pragma unroll
+          for (int k = 0; k < W; k++)
+            if (k < i - j0) cfma_sub(a[c], l[k], u[k]);
+        }
+        if (warp > s)
+#pragma unroll
+          for (int c = 0; c < W; c++) sD[i * TRY_LD + W * g + c] = a[c];
+      } else {
+#pragma unroll
+        for (int c = 0; c < W; c++) a[c] = l[c];
+        if (i == j0)
+#pragma unroll
+          for (int k = 0; k < W; k++) {
+            sRd[j0 + k] = rd[k];
+            sBest[j0 + k] = best[k];
+          }
+      }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+  }
+#pragma unroll
+  for (int c = 0; c < W; c++) sD[i * TRY_LD + W * g + c] = a[c];
+  return ok;
+}
+
+// Pivoted LU of the sub-panel's w x w diagonal block in sD (row stride TRY_LD) by warps
+// 0 to 7, warp q the columns 4q to 4q + 3, lane = row.  The owner of four columns takes
+// them in registers and leaves their multipliers in shared memory; the other warps then
+// interchange and update theirs: a barrier every four columns.  sPiv[j]: pivot row within
+// the block, sRd[j]: its reciprocal, sBest[j]: its key.  Bound by latency.
+template <typename T, typename Key>
+__device__ __forceinline__ void sp_factor_block(T* sD, T* sRd, Key* sBest, int* sPiv, int w, int lane, int warp) {
+  constexpr int CW = 4;  // columns of a warp
+  auto shfl = [&](T v, int src) {
+    T r;
+    r.x = __shfl_sync(0xffffffffu, v.x, src);
+    r.y = __shfl_sync(0xffffffffu, v.y, src);
+    return r;
+  };
+  T a[CW];
+#pragma unroll
+  for (int k = 0; k < CW; k++) a[k] = sD[lane * TRY_LD + CW * warp + k];
+  asm volatile("bar.sync 1, 256;" ::: "memory");  // the block is in registers, sD holds multipliers from here on
+#pragma unroll 1
+  for (int q = 0; CW * q < w; q++) {
+    T* mult = sD + (q & 1) * CW * IB;  // [CW][IB]
+    if (warp == q) {
+#pragma unroll
+      for (int k = 0; k < CW; k++) {
+        const int j = CW * q + k;
+        if (j >= w) break;
+        const Key key = lane >= j && lane < w ? pivot_key(a[k]) : Key(0);
+        const Key best = warp_max(key);
+        const int p = __ffs(__ballot_sync(0xffffffffu, key == best && lane >= j)) - 1;
+        if (p != j) {
+          const int src = lane == j ? p : lane == p ? j : lane;
+#pragma unroll
+          for (int c = 0; c < CW; c++) a[c] = shfl(a[c], src);
+        }
+        const T rd = pivot_recip(shfl(a[k], j));
+        T l = T{0, 0};
+        if (lane > j) {
+          l.x = a[k].x * rd.x - a[k].y * rd.y;
+          l.y = a[k].x * rd.y + a[k].y * rd.x;
+          a[k] = l;
+        }
+        mult[k * IB + lane] = l;
+        if (lane == 0) {
+          sPiv[j] = p;
+          sRd[j] = rd;
+          sBest[j] = best;
+        }
+#pragma unroll
+        for (int c = k + 1; c < CW; c++) {
+          const T u = shfl(a[c], j);
+          if (lane > j) {
+            a[c].x -= l.x * u.x - l.y * u.y;
+            a[c].y -= l.x * u.y + l.y * u.x;
+          }
+        }
+      }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (warp != q) {
+#pragma unroll
+      for (int k = 0; k < CW; k++) {
+        const int j = CW * q + k;
+        if (j >= w) break;
+        const int p = sPiv[j];
+        if (p != j) {
+          const int src = lane == j ? p : lane == p ? j : lane;
+#pragma unroll
+          for (int c = 0; c < CW; c++) a[c] = shfl(a[c], src);
+        }
+        if (warp > q) {
+          const T l = mult[k * IB + lane];
+#pragma unroll
+          for (int c = 0; c < CW; c++) {
+            const T u = shfl(a[c], j);
+            if (lane > j) {
+              a[c].x -= l.x * u.x - l.y * u.y;
+              a[c].y -= l.x * u.y + l.y * u.x;
+            }
+          }
+        }
+      }
+    }
+  }
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+  for (int k = 0; k < CW; k++) sD[lane * TRY_LD + CW * warp + k] = a[k];
+}
+
+// A row below the diagonal block, x <- x U^{-1} in shared memory, CB columns at a time in
+// registers, each element taking the pivots in ascending order; false if one of its
+// elements would have been the column's pivot.
+//
+// a[c] -= l[d] u[d][c] over CB x CB; complex64 in packed pairs, P = a - sum l.x u and
+// Q = sum l.y u, so that a = (P.x + Q.y, P.y - Q.x)
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  return (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(y) << 32);
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+template <int CB>
+struct TryAcc {
+  unsigned long long P[CB], Q[CB];
+  __device__ __forceinline__ void start(const float2* row) {
+#pragma unroll
+    for (int c = 0; c < CB; c++) {
+      P[c] = pack2(row[c].x, row[c].y);
+      Q[c] = 0;
+    }
+  }
+  __device__ __forceinline__ void add(float2 l, const float2* u) {
+    const unsigned long long x = pack2(-l.x, -l.x), y = pack2(l.y, l.y);
+#pragma unroll
+    for (int c = 0; c < CB; c += 2) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(u + c);
+      fma2(P[c], x, v.x);
+      fma2(Q[c], y, v.x);
+      fma2(P[c + 1], x, v.y);
+      fma2(Q[c + 1], y, v.y);
+    }
+  }
+  __device__ __forceinline__ float2 value(int c) const {
+    return make_float2(__uint_as_float((unsigned)P[c]) + __uint_as_float((unsigned)(Q[c] >> 32)),
+                       __uint_as_float((unsigned)(P[c] >> 32)) - __uint_as_float((unsigned)Q[c]));
+  }
+};
+template <int CB>
+struct TryAccD {
+  double2 a[CB];
+  __device__ __forceinline__ void start(const double2* row) {
+#pragma unroll
+    for (int c = 0; c < CB; c++) a[c] = row[c];
+  }
+  __device__ __forceinline__ void add(double2 l, const double2* u) {
+#pragma unroll
+    for (int c = 0; c < CB; c++) cfma_sub(a[c], l, u[c]);
+  }
+  __device__ __forceinline__ double2 value(int c) const { return a[c]; }
+};
+template <typename T, typename Key>
+__device__ __forceinline__ bool sp_try_row(T* row, const T* sD, const T* sRd, const Key* sBest) {
+  constexpr int CB = sizeof(T) == 8 ? 8 : 4;
+  bool ok = true;
+#pragma unroll 1
+  for (int k0 = 0; k0 < IB; k0 += CB) {
+    std::conditional_t<sizeof(T) == 8, TryAcc<CB>, TryAccD<CB>> acc;
+    acc.start(row + k0);
+#pragma unroll 1
+    for (int j0 = 0; j0 < k0; j0 += CB) {
+      T l[CB];
+#pragma unroll
+      for (int d = 0; d < CB; d++) l[d] = row[j0 + d];
+#pragma unroll
+      for (int d = 0; d < CB; d++) acc.add(l[d], sD + (j0 + d) * TRY_LD + k0);
+    }
+    T a[CB];
+#pragma unroll
+    for (int c = 0; c < CB; c++) a[c] = acc.value(c);
+#pragma unroll
+    for (int d = 0; d < CB; d++) {
+      ok &= pivot_key(a[d]) <= sBest[k0 + d];
+      a[d] = cmul(a[d], sRd[k0 + d]);
+      T u[CB];
+      load_u(sD + (k0 + d) * TRY_LD + k0, u);
+#pragma unroll
+      for (int c = d + 1; c < CB; c++) cfma_sub(a[c], a[d], u[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < CB; c++) row[k0 + c] = a[c];
+  }
+  return ok;
+}
 
 // Sub-panel rows [c0, n), columns [c0, c0 + w) of bt.B matrices, Gb = gridDim.x / B
 // consecutive CTAs each (group b works on matrix b); at least IB rows in the first.
@@ -359,9 +660,9 @@ inline int sp_threads(int rows) { return 32 * ((rows + 32 * sp_rpt(rows) - 1) / 
 // CLUSTER: a matrix's CTAs are one cluster of up to 16, which exchanges the rows
 // through distributed shared memory: the owner warp stores its row into every CTA,
 // and one cluster barrier takes the place of the records' trip through L2.  Taken for
-// 481 to 7,680 rows (complex128 396 to 6,320), a row per thread: 84 -> 67 us a
-// sub-panel there, complex128 101 -> 84 us.  Two rows a thread in 16 CTAs (to 13,200
-// rows) take 94 us against the records' 88, so taller sub-panels meet in L2.
+// 225 to 4,096 rows, a row per thread: 84 -> 67 us a search there, complex128 101 ->
+// 84 us, and a verdict costs 900 cycles against 2,500 to 5,000.  Taller sub-panels would
+// need more rows a CTA than SP_ROWS, and meet in L2.
 __device__ __forceinline__ void sp_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -378,6 +679,13 @@ __device__ __forceinline__ void sp_store_remote(uint32_t a, double2 v) {
 }
 __device__ __forceinline__ void sp_store_remote(uint32_t a, int v) {
   asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+template <typename T>
+__device__ __forceinline__ void sp_cp_async(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "n"(sizeof(T))
+               : "memory");
 }
 
 template <typename T, int RPT, bool CLUSTER>
@@ -406,9 +714,33 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
   const bool helper = warp == NWR;
   const int col = min(lane, w - 1);
   auto slot = [&](int buf, int g) { return rec + (((size_t)buf * bt.B + grp) * (Gb + 1) + g) * IB * LL<T>::BYTES; };
-#pragma unroll 16
-  for (int r = warp; r < nr; r += NW)
-    if (lane < w) sA[r * SP + lane] = A[(size_t)(c0 + lo + r) * n + c0 + lane];
+  auto load_rows = [&]() {
+    if (lane < w)
+      for (int r = warp; r < nr; r += NW) sp_cp_async(sA + r * SP + lane, A + (size_t)(c0 + lo + r) * n + c0 + lane);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto load_diag = [&](T* sD) {
+    if (warp < TRY_THREADS / 32)
+#pragma unroll
+      for (int q = 0; q < IB * 32 / TRY_THREADS; q++) {
+        const int r = warp + q * (TRY_THREADS / 32);
+        if (r < w && lane < w)
+          sp_cp_async(sD + r * TRY_LD + lane, A + (size_t)(c0 + r) * n + c0 + lane);
+        else
+          sD[r * TRY_LD + lane] = T{0, 0};
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int* tries = bt.tries + 2 * grp;
+  const bool trying = tries[0] == 0 && (w == IB || w == m);
+  bool tried = false;  // ... and every pivot lies in the diagonal block
+  T* sD = sRow;        // the diagonal block
+  if (trying) load_diag(sD);
+  load_rows();
+  if (trying)
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // the block; the rows come meanwhile
+  else
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (tid == 0) *sFlag = *(volatile int*)bt.err;
   if (CLUSTER) sp_cluster_sync();  // every CTA's shared memory exists before the first store into it
   else __syncthreads();
@@ -475,8 +807,62 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
     }
   };
   const bool one_hop = Gb <= LL_ONE_HOP && Gb < LL_PER_WARP * NW;
-  load_block(0);
-  for (int b0 = 0; b0 < w; b0 += CB) {
+  if (trying) {
+    T* sRd = sTop;
+    Key* sBest = sKey;
+    bool ok = true;
+    if (warp < TRY_THREADS / 32) ok = sp_factor_diag(sD, sRd, sBest, w, tid);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (tid < IB) sPiv[tid] = tid;
+    if (!__syncthreads_and(ok)) {
+      load_diag(sD);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      if (warp < TRY_THREADS / 32) sp_factor_block(sD, sRd, sBest, sPiv, w, lane, warp);
+      __syncthreads();
+    }
+    ok = sBest[col] > 1;  // a column without a pivot is left to the full search
+    if (!helper)
+#pragma unroll 1
+      for (int i = 0; i < RPT; i++)
+        if (row_of(i) < nr && lo + row_of(i) >= w) ok = sp_try_row(sA + row_of(i) * SP, sD, sRd, sBest) && ok;
+    ok = __syncthreads_and(ok);
+    if (CLUSTER) {
+      // sIdx[g] of every CTA: CTA g agrees
+      if (tid < Gb) sp_store_remote(sp_remote(sIdx + cta, tid), (int)ok);
+      sp_cluster_sync();
+      tried = __syncthreads_and(tid >= Gb || sIdx[tid]);
+    } else if (Gb > 1) {
+      unsigned char* v = bt.verdict + (size_t)grp * Gb * LL<float2>::BYTES;
+      const unsigned tag = (unsigned)c0 + 1u;
+      if (tid == 0) LL<float2>::post(v + cta * LL<float2>::BYTES, make_float2(ok ? 1.0f : 0.0f, 0.0f), tag);
+      if (tid < Gb) {
+        float2 r = make_float2(0, 0);
+        unsigned long long hi;
+        for (int spin = 0; !LL<float2>::poll(v + tid * LL<float2>::BYTES, r, hi, tag); spin++)
+          if (spin >= LL_SPINS || *(volatile int*)sFlag) {
+            *(volatile int*)sFlag = 1;
+            atomicExch(bt.err, 1);
+            break;
+          }
+        ok = r.x != 0.0f;
+      }
+      tried = __syncthreads_and(ok);
+    } else {
+      tried = ok;
+    }
+    if (tried) {
+      if (cta == 0 && warp < TRY_THREADS / 32 && lane < w)
+        for (int r = warp; r < w; r += TRY_THREADS / 32) sA[r * SP + lane] = sD[r * TRY_LD + lane];
+      if (tid < w) sPiv[tid] += c0;
+    } else {
+      load_rows();
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+    }
+  }
+  if (!tried) load_block(0);
+  for (int b0 = tried ? w : 0; b0 < w; b0 += CB) {
     const int end = min(b0 + CB, w);
 #pragma unroll 1
     for (int jj = b0; jj < end; jj++) {
@@ -720,9 +1106,27 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
     }
   }
   __syncthreads();
-  for (int r = warp; r < nr; r += NW)
-    if (lane < w) A[(size_t)(c0 + lo + r) * n + c0 + lane] = sA[r * SP + lane];
+  for (int r0 = warp; r0 < nr; r0 += 8 * NW) {
+    T v[8];  // read before the first is written
+#pragma unroll
+    for (int q = 0; q < 8; q++) v[q] = sA[min(r0 + q * NW, nr - 1) * SP + col];
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (r0 + q * NW < nr && lane < w) A[(size_t)(c0 + lo + r0 + q * NW) * n + c0 + lane] = v[q];
+  }
   if (cta == 0 && tid < w) batch_pick(bt.ipiv, grp)[c0 + tid] = sPiv[tid];
+  if (cta == 0 && tid == 0) {
+    // (every CTA has read them by now: its records were waited for)  After a failure in a
+    // row the next 1, 3, 7, then 15 sub-panels go without a try
+    if (!trying) {
+      tries[0] = max(tries[0] - 1, 0);
+    } else if (tried) {
+      tries[1] = 0;
+    } else {
+      tries[0] = tries[1];
+      tries[1] = min(2 * tries[1] + 1, 15);
+    }
+  }
   if (pk1 - pk0 > w) {
     const unsigned moves = __ballot_sync(0xffffffffu, lane < w && sPiv[col] != c0 + lane);
     const int nl = c0 - pk0, nc = nl + (pk1 - (c0 + w));
@@ -749,16 +1153,6 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
 // (k_inv_join_t, k_inv_join_x), all pairs of a level in the same two
 // launches.  Entries above the diagonal are written as zero.
 constexpr int INV_MAX = 512;
-template <typename T>
-__device__ __forceinline__ void cfma_sub(T& acc, T a, T b) {
-  acc.x -= a.x * b.x - a.y * b.y;
-  acc.y -= a.x * b.y + a.y * b.x;
-}
-template <typename T>
-__device__ __forceinline__ void cfma_add(T& acc, T a, T b) {
-  acc.x += a.x * b.x - a.y * b.y;
-  acc.y += a.x * b.y + a.y * b.x;
-}
 
 constexpr int INV32_LD = 34, INV32_SCRATCH = 256;  // of inv_unit32
 
@@ -1463,10 +1857,11 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   // records of B matrices in one launch, or of each matrix in its own: one
   // region per matrix, since the matrices of separate launches share the tags
   const size_t rec_region = 2 * ((size_t)G + kMaxBatch) * IB * LL<T>::BYTES, rec_bytes = rec_region * B;
-  TT_TRY(srec.alloc(rec_bytes));
-  TT_TRY(d_info.alloc(B + 1));  // [B] first zero pivots, then the sub-panels' error word
-  TT_CUDA_TRY(cudaMemsetAsync(d_info.ptr, 0, sizeof(int) * (B + 1), st));
-  TT_CUDA_TRY(cudaMemsetAsync(srec.ptr, 0, rec_bytes, st));
+  const size_t verdicts = (size_t)G * LL<float2>::BYTES;  // of a matrix, behind the records
+  TT_TRY(srec.alloc(rec_bytes + verdicts * B));
+  TT_TRY(d_info.alloc(3 * B + 1));  // [B] first zero pivots, the sub-panels' error word, [B][2] tries
+  TT_CUDA_TRY(cudaMemsetAsync(d_info.ptr, 0, sizeof(int) * (3 * B + 1), st));
+  TT_CUDA_TRY(cudaMemsetAsync(srec.ptr, 0, rec_bytes + verdicts * B, st));
   PivotScratch<T> scr{sval.ptr, sidx.ptr, srow.ptr, stop.ptr};
   using SC = SubpanelCfg<T>;
   // rows per thread: complex128 rows fill shared memory before they outnumber the threads
@@ -1480,7 +1875,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   // two of about SP_CLUSTER_ROWS rows a CTA; 0: too tall, or one CTA holds them
   const size_t one_row = std::min(SP_ROWS, SC::MAX_ROWS);  // rows of a CTA with a row per thread
   auto cluster_ctas = [&](size_t m) -> int {
-    if (m <= one_row || m > one_row * max_cluster) return 0;
+    if (m <= one_row || m > SP_CLUSTER_ROWS * max_cluster) return 0;
     int g = 2;
     while (g < max_cluster && (m + g - 1) / g > SP_CLUSTER_ROWS) g *= 2;
     return g;
@@ -1503,6 +1898,8 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
     }
     bt.info = d_info.ptr + b0;
     bt.err = d_info.ptr + B;
+    bt.tries = d_info.ptr + B + 1 + 2 * b0;
+    bt.verdict = srec.ptr + rec_bytes + verdicts * b0;
     bt.B = nb;
     int nn = n, cc0 = j0, ww = w, p0 = pk0, p1 = pk1;
     unsigned char* rec = srec.ptr + rec_region * b0;
