@@ -1149,9 +1149,8 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
 // k_inv_diag32 inverts the 32 x 32 diagonal blocks (one CTA each), then per
 // level s = 64, 128, .. every pair of inverted s/2 blocks is joined,
 //   [X11 0; X21 X22] with X21 = -X22 (L21 X11),
-// first T = L21 X11, then X21 = -X22 T, one CTA per 32 x 32 tile
-// (k_inv_join_t, k_inv_join_x), all pairs of a level in the same two
-// launches.  Entries above the diagonal are written as zero.
+// first T = L21 X11, then X21 = -X22 T, one CTA per tile (k_inv_join), all pairs
+// of a level in the same two launches.  Entries above the diagonal are written as zero.
 constexpr int INV_MAX = 512;
 
 constexpr int INV32_LD = 34, INV32_SCRATCH = 256;  // of inv_unit32
@@ -1256,96 +1255,66 @@ __global__ void __launch_bounds__(256) k_inv_diag32(InvBatch<T> ib, int n, int r
   }
 }
 
-// Level s: pair p joins the blocks [p s, p s + s/2) and [p s + s/2, p s + s)
-// (the second may be shorter at the end of w) in two launches of one CTA per
-// 32 x 32 tile (ty: tile row of block 2, tx: tile column of block 1):
-//   k_inv_join_t:  Tp = L21 X11          (X11 lower: k from the tile's column)
-//   k_inv_join_x:  X21 = -X22 Tp         (X22 lower: m up to the tile's row)
-// Tp is the pair's h x h scratch at T + p h h.
+// Level s: pair p joins the blocks [p s, p s + h) and [p s + h, p s + s), h = s / 2
+// (the second may be shorter at the end of w) in two launches of one CTA per tile of
+// 32 rows of block 2 (ty) and 16 columns of block 1 (tx):
+//   k_inv_join<.., false>:  Tp = L21 X11     (X11 lower: k from the tile's column)
+//   k_inv_join<.., true>:   X21 = -X22 Tp    (X22 lower: k up to the tile's row)
+// Tp is the pair's h x h scratch at T + p h h.  The whole depth of both operands is
+// asked for at once (cp.async), a thread then sums two elements.  Bound: latency and,
+// from h = 128 on, FP32 issue.  The eight joins of a 512 x 512 block, two matrices,
+// against 32 x 32 tiles staged 32 deep one after another: 127 -> 54 us (n = 16,128).
+constexpr int JT_M = 32, JT_N = 16;
 template <typename T>
-__global__ void __launch_bounds__(256) k_inv_join_t(InvBatch<T> ib, int n, int r0, int w, int s,
-                                                    const T* __restrict__ X, T* __restrict__ Tsc) {
-  __shared__ T sa[32][33];
-  __shared__ T sb[32][33];
-  const int h = s / 2;
+size_t inv_join_smem(int h) {
+  return sizeof(T) * ((size_t)JT_M * (h + 2) + (size_t)h * (JT_N + 1));
+}
+template <typename T, bool SECOND>
+__global__ void __launch_bounds__(256) k_inv_join(InvBatch<T> ib, int n, int r0, int w, int s, T* __restrict__ X,
+                                                  T* __restrict__ Tsc) {
+  extern __shared__ __align__(16) unsigned char join_raw[];
+  const int h = s / 2, lda = h + 2, ldb = JT_N + 1;
+  T* sa = reinterpret_cast<T*>(join_raw);  // [JT_M][lda]
+  T* sb = sa + JT_M * lda;                 // [h][ldb]
   const int pairs = (w + s - 1) / s, mb = blockIdx.z / pairs;
   const int p = blockIdx.z - mb * pairs, base = p * s;
   const T* __restrict__ A = ib.A[mb];
   X += (size_t)mb * w * w;
-  Tsc += (size_t)mb * w * w / 2;
-  const int h2 = min(h, w - base - h);  // rows of the second block
-  const int ty = blockIdx.y, tx = blockIdx.x;
-  if (h2 <= 0 || ty * 32 >= h2) return;
-  const int tid = threadIdx.x, row = tid >> 3, cq = (tid & 7) * 4;
-  const int c0 = base + tx * 32;  // columns of X11
-  T acc[4];
+  T* Tp = Tsc + (size_t)mb * w * w / 2 + (size_t)p * h * h;
+  const int h2 = min(h, w - base - h);  // rows of the second block, a multiple of 32
+  const int i0 = blockIdx.y * JT_M, c0 = blockIdx.x * JT_N;
+  if (i0 >= h2) return;
+  const int k0 = SECOND ? 0 : c0 & ~31, k1 = SECOND ? i0 + JT_M : h;  // multiples of 32
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const T* a = SECOND ? X + (size_t)(base + h + i0) * w + base + h : A + (size_t)(r0 + base + h + i0) * n + r0 + base;
+  const T* b = SECOND ? Tp + c0 : X + (size_t)base * w + base + c0;
+  const int la = SECOND ? w : n, lb = SECOND ? h : w;
+  for (int i = warp; i < JT_M; i += 8)
+    for (int k = k0 + lane; k < k1; k += 32) sp_cp_async(sa + i * lda + k, a + (size_t)i * la + k);
+  const int col = tid % JT_N, row = tid / JT_N;
+  for (int k = k0 + row; k < k1; k += 256 / JT_N) sp_cp_async(sb + k * ldb + col, b + (size_t)k * lb + col);
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  T v[2][2];  // two rows, two partial sums each
 #pragma unroll
-  for (int q = 0; q < 4; q++) acc[q].x = acc[q].y = 0;
-  for (int k0 = tx * 32; k0 < h; k0 += 32) {
-    __syncthreads();
-    for (int t = tid; t < 1024; t += 256) {
-      const int i = t >> 5, j = t & 31;
-      T a;
-      a.x = a.y = 0;
-      if (ty * 32 + i < h2) a = A[(size_t)(r0 + base + h + ty * 32 + i) * n + r0 + base + k0 + j];
-      sa[i][j] = a;
-      sb[i][j] = X[(size_t)(base + k0 + i) * w + c0 + j];
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < 32; kk++) {
-      const T a = sa[row][kk];
-#pragma unroll
-      for (int q = 0; q < 4; q++) cfma_add(acc[q], a, sb[kk][cq + q]);
-    }
+  for (int u = 0; u < 2; u++) v[u][0] = v[u][1] = T{0, 0};
+  const T *x = sa + row * lda, *y = x + JT_M / 2 * lda;
+#pragma unroll 4
+  for (int k = k0; k < k1; k += 2) {
+    const T b0 = sb[k * ldb + col], b1 = sb[(k + 1) * ldb + col];
+    cfma_add(v[0][0], x[k], b0);
+    cfma_add(v[1][0], y[k], b0);
+    cfma_add(v[0][1], x[k + 1], b1);
+    cfma_add(v[1][1], y[k + 1], b1);
   }
-  if (ty * 32 + row < h2) {
-    T* Tp = Tsc + (size_t)p * h * h;
 #pragma unroll
-    for (int q = 0; q < 4; q++) Tp[(size_t)(ty * 32 + row) * h + tx * 32 + cq + q] = acc[q];
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_inv_join_x(int w, int s, T* __restrict__ X, const T* __restrict__ Tsc) {
-  __shared__ T sa[32][33];
-  __shared__ T sb[32][33];
-  const int h = s / 2;
-  const int pairs = (w + s - 1) / s, mb = blockIdx.z / pairs;
-  const int p = blockIdx.z - mb * pairs, base = p * s;
-  X += (size_t)mb * w * w;
-  Tsc += (size_t)mb * w * w / 2;
-  const int h2 = min(h, w - base - h);
-  const int ty = blockIdx.y, tx = blockIdx.x;
-  if (h2 <= 0 || ty * 32 >= h2) return;
-  const int tid = threadIdx.x, row = tid >> 3, cq = (tid & 7) * 4;
-  const T* Tp = Tsc + (size_t)p * h * h;
-  T acc[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) acc[q].x = acc[q].y = 0;
-  for (int m0 = 0; m0 <= ty * 32; m0 += 32) {
-    __syncthreads();
-    for (int t = tid; t < 1024; t += 256) {
-      const int i = t >> 5, j = t & 31;
-      T a, b;
-      a.x = a.y = b.x = b.y = 0;
-      if (ty * 32 + i < h2 && m0 + j < h2) a = X[(size_t)(base + h + ty * 32 + i) * w + base + h + m0 + j];
-      if (m0 + i < h2) b = Tp[(size_t)(m0 + i) * h + tx * 32 + j];
-      sa[i][j] = a;
-      sb[i][j] = b;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < 32; kk++) {
-      const T a = sa[row][kk];
-#pragma unroll
-      for (int q = 0; q < 4; q++) cfma_sub(acc[q], a, sb[kk][cq + q]);
-    }
-  }
-  if (ty * 32 + row < h2) {
-    const int gr = base + h + ty * 32 + row, c0 = base + tx * 32;
-#pragma unroll
-    for (int q = 0; q < 4; q++) X[(size_t)gr * w + c0 + cq + q] = acc[q];
+  for (int u = 0; u < 2; u++) {
+    const int i = i0 + row + u * (JT_M / 2);
+    const T r = T{v[u][0].x + v[u][1].x, v[u][0].y + v[u][1].y};
+    if (SECOND)
+      X[(size_t)(base + h + i) * w + base + c0 + col] = T{-r.x, -r.y};
+    else
+      Tp[(size_t)i * h + c0 + col] = r;
   }
 }
 
@@ -1690,13 +1659,17 @@ int inv_unit_lower(const T* const* As, int B, int n, int r0, int w, T* X, T* Tsc
   k_inv_diag32<T><<<dim3(w / 32, B), 256, 0, st>>>(ib, n, r0, w, X);
   count_launch();
   TT_CUDA_TRY(cudaGetLastError());
+  const int join_smem = (int)inv_join_smem<T>(INV_MAX / 2);
+  TT_TRY(smem_limit_once((const void*)k_inv_join<T, false>, join_smem));
+  TT_TRY(smem_limit_once((const void*)k_inv_join<T, true>, join_smem));
   for (int s = 64; s / 2 < w; s *= 2) {
     const int h = s / 2;
-    dim3 grid(h / 32, h / 32, ((w + s - 1) / s) * B);
-    k_inv_join_t<T><<<grid, 256, 0, st>>>(ib, n, r0, w, s, X, Tsc);
+    const dim3 grid(h / JT_N, h / JT_M, ((w + s - 1) / s) * B);
+    const size_t smem = inv_join_smem<T>(h);
+    k_inv_join<T, false><<<grid, 256, smem, st>>>(ib, n, r0, w, s, X, Tsc);
     count_launch();
     TT_CUDA_TRY(cudaGetLastError());
-    k_inv_join_x<T><<<grid, 256, 0, st>>>(w, s, X, Tsc);
+    k_inv_join<T, true><<<grid, 256, smem, st>>>(ib, n, r0, w, s, X, Tsc);
     count_launch();
     TT_CUDA_TRY(cudaGetLastError());
   }
