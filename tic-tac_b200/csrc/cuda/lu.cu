@@ -70,101 +70,137 @@ __host__ __device__ __forceinline__ int blk_start(int n, int q) {
 // stored one.  The factor of L U keeps the unit lower and the upper triangle; its
 // transpose (TRANSPOSED, for transposed solves) keeps the non-unit lower and the
 // unit upper triangle.  Rows and columns past the block are the identity's.
-// A CTA inverts the block's two 64 x 64 diagonal halves at once, 256 threads each,
-// in place in shared memory, right-looking, row j being final when step j starts
-// (lower, j ascending: row j is scaled by 1/D[j][j], then X[r][c] -= L[r][j] X[j][c]
-// for r > j, c <= j; upper, j descending, mirrored), and joins them:
-// X21 = -X22 (L21 X11), or X12 = -X11 (U12 X22).
+// An upper triangle is taken with its rows and columns in reverse order, as a lower
+// one.  A CTA inverts the block's two 64 x 64 diagonal halves at once, 256 threads
+// each, in place in shared memory: 8 x 8 blocks in registers, a column a thread, then
+// pairs of inverted blocks joined three times, and the halves once,
+//   [X11 0; X21 X22] with X21 = -X22 (L21 X11).
+// Bound: latency; the 64 steps of a right-looking inversion, three barriers each, took
+// 84 us for a factor of order 512 against 34 now, 100 against 38 at 1,859, 142 against
+// 66 for a complex128 one of order 8,496.
+template <typename T>
+__device__ __forceinline__ void cfma(T& acc, T a, T b) {
+  acc.x += a.x * b.x;
+  acc.x -= a.y * b.y;
+  acc.y += a.x * b.y;
+  acc.y += a.y * b.x;
+}
+
+// One join of H x H blocks of a half (256 threads, t the thread), H / 8 elements each;
+// L21 X11 waits in the zeros above the diagonal
+template <int H, typename T>
+__device__ __forceinline__ void inv_join(T* M, int t) {
+  constexpr int U = H / 8;
+  const int i0 = t / (8 * H) * 2 * H, r = t / 8 % H, c = t % 8;
+  T* X11 = M + i0 * TLD + i0;
+  T *S = X11 + H, *X21 = X11 + H * TLD, *X22 = X21 + H;
+  auto product = [&](const T* a, const T* b, T* out, bool minus) {
+    T acc[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) acc[u] = T{0, 0};
+#pragma unroll 8
+    for (int k = 0; k < H; k++) {
+      const T x = a[r * TLD + k];
+#pragma unroll
+      for (int u = 0; u < U; u++) cfma(acc[u], x, b[k * TLD + c + 8 * u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) out[r * TLD + c + 8 * u] = minus ? T{-acc[u].x, -acc[u].y} : acc[u];
+  };
+  product(X21, X11, S, false);
+  __syncthreads();
+  product(X22, S, X21, true);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < U; u++) S[r * TLD + c + 8 * u] = T{0, 0};
+  __syncthreads();
+}
+
 template <typename T, bool UPPER, bool UNIT>
-__device__ void inv_block(const T* __restrict__ LU, int n, int q, T* __restrict__ out, T* sm, T* cols) {
+__device__ void inv_block(const T* __restrict__ LU, int n, int q, T* __restrict__ out, T* sm) {
   const int tid = threadIdx.x, half = tid >> 8, t = tid & 255;
   const int r0 = blk_start<UPPER>(n, q), rows = blk_rows(n, q);
   const T zero = {0, 0}, one = {1, 0};
   T* M = sm + half * TSB * TLD;   // this half's diagonal tile
-  T* O = sm + 2 * TSB * TLD;      // the off-diagonal tile
-  T* col = cols + half * TSB;
-  const int h0 = half * TSB, bs = max(0, min(TSB, rows - h0));
+  T* O = sm + 2 * TSB * TLD;      // the tile below the first half's
+  const int h0 = half * TSB;
+  // row (column) i of the lower triangle worked on is row at(i) of the block
+  auto at = [&](int i) { return UPPER && i < rows ? rows - 1 - i : i; };
+#pragma unroll 4
   for (int e = t; e < TSB * TSB; e += 256) {
     const int r = e / TSB, c = e % TSB;
-    const bool stored = UPPER ? (UNIT ? c > r : c >= r) : (UNIT ? c < r : c <= r);
     T v = (r == c) ? one : zero;
-    if (r < bs && c < bs && stored) v = LU[(size_t)(r0 + h0 + r) * n + r0 + h0 + c];
+    if (h0 + r < rows && h0 + c < rows && (UNIT ? c < r : c <= r))
+      v = LU[(size_t)(r0 + at(h0 + r)) * n + r0 + at(h0 + c)];
     M[r * TLD + c] = v;
   }
+#pragma unroll 4
   for (int e = tid; e < TSB * TSB; e += 512) {
-    const int r = e / TSB + (UPPER ? 0 : TSB), c = e % TSB + (UPPER ? TSB : 0);
-    O[(e / TSB) * TLD + e % TSB] = (r < rows && c < rows) ? LU[(size_t)(r0 + r) * n + r0 + c] : zero;
+    const int r = e / TSB + TSB, c = e % TSB;
+    O[(e / TSB) * TLD + c] = (r < rows && c < rows) ? LU[(size_t)(r0 + at(r)) * n + r0 + at(c)] : zero;
   }
   __syncthreads();
-  for (int step = 0; step < TSB; step++) {
-    const int j = UPPER ? TSB - 1 - step : step;
-    const int w = UPPER ? TSB - j : j + 1;       // columns of row j, from c0
-    const int c0 = UPPER ? j : 0, f0 = UPPER ? 0 : j + 1, cnt = TSB - w;  // rows still to be updated: [f0, f0 + cnt)
-    T d = one;
-    if (!UNIT) {
-      d = crecip(M[j * TLD + j]);
-      __syncthreads();
-      for (int c = t; c < w - 1; c += 256) {
-        const int cc = UPPER ? j + 1 + c : c;
-        M[j * TLD + cc] = cmul(M[j * TLD + cc], d);
+  if (t < TSB) {
+    const int c = t & 7;
+    T* B = M + (t & ~7) * (TLD + 1);
+    T v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      v[i] = i == c ? one : zero;
+#pragma unroll
+      for (int j = 0; j < i; j++) {
+        const T m = B[i * TLD + j];
+        cfma(v[i], T{-m.x, -m.y}, v[j]);
       }
-      if (t == 0) M[j * TLD + j] = d;
+      if (!UNIT) v[i] = cmul(v[i], crecip(B[i * TLD + i]));
     }
-    for (int r = t; r < cnt; r += 256) col[f0 + r] = M[(f0 + r) * TLD + j];
-    __syncthreads();
-    // 4 threads a row
-    for (int r = f0 + (t >> 2); r < f0 + cnt; r += 64) {
-      const T l = col[r];
-      for (int c = c0 + (t & 3); c < c0 + w; c += 4) {
-        const T p = cmul(l, c == j ? d : M[j * TLD + c]);
-        const T v = c == j ? zero : M[r * TLD + c];
-        M[r * TLD + c] = T{v.x - p.x, v.y - p.y};
-      }
-    }
-    __syncthreads();
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; i++) B[i * TLD + c] = v[i];
   }
-  // join: 8 elements a thread, row tr, columns tc + 8 u
+  __syncthreads();
+  inv_join<8>(M, t);
+  inv_join<16>(M, t);
+  inv_join<32>(M, t);
+  // join of the halves: 8 elements a thread, row tr, columns tc + 8 u
   const T* X1 = sm;               // inverse of the first half
   const T* X2 = sm + TSB * TLD;   // of the second
   const int tr = tid >> 3, tc = tid & 7;
   auto product = [&](const T* a, const T* b, T(&acc)[8]) {
 #pragma unroll
     for (int u = 0; u < 8; u++) acc[u] = zero;
+#pragma unroll 4
     for (int k = 0; k < TSB; k++) {
       const T x = a[tr * TLD + k];
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const T p = cmul(x, b[k * TLD + tc + 8 * u]);
-        acc[u].x += p.x;
-        acc[u].y += p.y;
-      }
+      for (int u = 0; u < 8; u++) cfma(acc[u], x, b[k * TLD + tc + 8 * u]);
     }
   };
   T acc[8];
-  product(O, UPPER ? X2 : X1, acc);
+  product(O, X1, acc);
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < 8; u++) O[tr * TLD + tc + 8 * u] = acc[u];
   __syncthreads();
-  product(UPPER ? X1 : X2, O, acc);
+  product(X2, O, acc);
   T* o = out + (size_t)q * TW * TW;
+  const int i1 = at(tr) * TW, i2 = at(tr + TSB) * TW;
 #pragma unroll
   for (int u = 0; u < 8; u++) {
-    const int c = tc + 8 * u;
-    o[(size_t)(tr + (UPPER ? 0 : TSB)) * TW + c + (UPPER ? TSB : 0)] = T{-acc[u].x, -acc[u].y};
-    o[(size_t)(tr + (UPPER ? TSB : 0)) * TW + c + (UPPER ? 0 : TSB)] = zero;
-    o[(size_t)tr * TW + c] = X1[tr * TLD + c];
-    o[(size_t)(tr + TSB) * TW + c + TSB] = X2[tr * TLD + c];
+    const int c = tc + 8 * u, j1 = at(c), j2 = at(c + TSB);
+    o[(size_t)i2 + j1] = T{-acc[u].x, -acc[u].y};
+    o[(size_t)i1 + j2] = zero;
+    o[(size_t)i1 + j1] = X1[tr * TLD + c];
+    o[(size_t)i2 + j2] = X2[tr * TLD + c];
   }
 }
 template <typename T, bool TRANSPOSED>
 __global__ void __launch_bounds__(512) k_inv_blocks(const T* __restrict__ LU, int n, T* __restrict__ invL,
                                                     T* __restrict__ invU) {
   extern __shared__ __align__(16) unsigned char ism[];
-  __shared__ T cols[2 * TSB];
   T* sm = reinterpret_cast<T*>(ism);  // [3][TSB][TLD]
-  if (blockIdx.y == 0) inv_block<T, false, !TRANSPOSED>(LU, n, blockIdx.x, invL, sm, cols);
-  else inv_block<T, true, TRANSPOSED>(LU, n, blockIdx.x, invU, sm, cols);
+  if (blockIdx.y == 0) inv_block<T, false, !TRANSPOSED>(LU, n, blockIdx.x, invL, sm);
+  else inv_block<T, true, TRANSPOSED>(LU, n, blockIdx.x, invU, sm);
 }
 
 // ---------------------------------------------------------------------------
