@@ -211,114 +211,134 @@ __global__ void k_gather_rhs(const double* __restrict__ A, int n, const int32_t*
   b[tid] = make_double2(A[(size_t)i * n + cols[k]], 0.0);
 }
 
-// r_v = b_v - x_v + A y_v for NV <= 4 vectors in one pass over A.  A CTA owns 32
-// rows, 4 per warp; a lane takes VEC columns of each row at a step (2 where rows
-// are 16-byte aligned: even n), and asks for A two steps ahead.  y comes through
-// shared memory, 512 columns at a time, read from L2 once per 32 rows.  Bound: A
-// read once; the loads in flight (two steps x 4 rows x 16 warps an SM, 64 KB)
-// carry on across the refills of y.  n = 42,300: 2 vectors 3.00 -> 2.41 ms
-// (5.9 TB/s), 4 vectors 3.48 -> 3.16 ms (their accumulators leave one step ahead).
-constexpr int R2_ROWS = 32, R2_COLS = 512;
-template <int NV, int VEC>
+// part[slab][v] = A y_v over the slab's columns, for nv <= 4 NT vectors in one pass over
+// A: a real n x n by n x 8 NT product on the FP64 tensor cores (m8n8k4), the real and
+// imaginary parts of a vector being two columns.  A warp takes 16 rows; a lane's four
+// neighbouring columns of a row serve as the k = lane % 4 elements of four products, so
+// A goes from HBM to registers in 16-byte loads (VEC = 2, even n; else 8-byte), asked
+// for two steps of 16 columns ahead, and y comes through shared memory, transposed, 128
+// columns at a time.  Slabs of columns even out the last wave of CTAs: two an SM, their
+// number chosen in residual_slabs.  Bound: A read once.  FMA kernels of up to 4 vectors
+// a launch before: six vectors, n = 16,128 0.87 -> 0.36 ms,
+// n = 42,300 5.6 -> 2.5 ms (5.8 TB/s); twelve at n = 20,160 2.97 -> 0.80 ms.
+constexpr int RM_ROWS = 128, RM_COLS = 128, RM_LD = RM_COLS + 2, RM_NT = 3, RM_SLABS = 16;
+__device__ __forceinline__ void mma884(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+template <int NT, int VEC>
 __global__ void __launch_bounds__(256, 2) k_residual(const double* __restrict__ A, int n,
-                                                     const double2* __restrict__ y, const double2* __restrict__ b,
-                                                     const double2* __restrict__ x, double2* __restrict__ r) {
-  __shared__ double2 sy[NV][R2_COLS];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row0 = (int64_t)blockIdx.x * R2_ROWS + warp * 4;
-  const double* Ar = A + (size_t)min(row0, (int64_t)n - 1) * n + lane * VEC;
-  int64_t off[4];  // rows past the last read it again
+                                                     const double2* __restrict__ y, int nv, int slabs,
+                                                     double2* __restrict__ part) {
+  __shared__ __align__(16) double sy[8 * NT][RM_LD];
+  constexpr int AHEAD = 2, STEP = 16, PER = RM_COLS / STEP;
+  const int tid = threadIdx.x, warp = tid >> 5, r = (tid & 31) >> 2, q = tid & 3;
+  const int chunks = (n + RM_COLS - 1) / RM_COLS;
+  const int c_lo = (int)((long long)chunks * blockIdx.y / slabs) * RM_COLS;
+  const int c_hi = min(n, (int)((long long)chunks * (blockIdx.y + 1) / slabs) * RM_COLS);
+  const int64_t row0 = (int64_t)blockIdx.x * RM_ROWS + warp * 16 + r;
+  const double* Ar[2];  // rows past the last read it again
 #pragma unroll
-  for (int h = 0; h < 4; h++) off[h] = row0 + h < n ? (int64_t)h * n : 0;
-  double sr[4][NV], si[4][NV];
+  for (int m = 0; m < 2; m++) Ar[m] = A + min(row0 + 8 * m, (int64_t)n - 1) * n + 4 * q;
+  auto load = [&](int c, double(&a)[2][4]) {
 #pragma unroll
-  for (int h = 0; h < 4; h++)
+    for (int m = 0; m < 2; m++)
 #pragma unroll
-    for (int v = 0; v < NV; v++) sr[h][v] = si[h][v] = 0.0;
-  constexpr int STEP = 32 * VEC, PER = R2_COLS / STEP;
-  const int steps = (n + STEP - 1) / STEP;
-  auto load = [&](int s, double(&a)[4][VEC]) {
-    const int c = s * STEP;
-    const bool in = c + lane * VEC < n;
-#pragma unroll
-    for (int h = 0; h < 4; h++) {
-      if constexpr (VEC == 2) {
-        const double2 t = in ? __ldcs(reinterpret_cast<const double2*>(Ar + off[h] + c)) : make_double2(0.0, 0.0);
-        a[h][0] = t.x;
-        a[h][1] = t.y;
-      } else {
-        a[h][0] = in ? __ldcs(Ar + off[h] + c) : 0.0;
+      for (int h = 0; h < 4; h += VEC) {
+        const bool in = c + 4 * q + h < c_hi;
+        if constexpr (VEC == 2) {
+          const double2 t = in ? __ldcs(reinterpret_cast<const double2*>(Ar[m] + c + h)) : make_double2(0.0, 0.0);
+          a[m][h] = t.x;
+          a[m][h + 1] = t.y;
+        } else {
+          a[m][h] = in ? __ldcs(Ar[m] + c + h) : 0.0;
+        }
       }
-    }
   };
-  // steps in flight beyond the present one, as the accumulators leave registers
-  constexpr int AHEAD = NV > 2 ? 1 : 2;
-  double a[AHEAD + 1][4][VEC];
+  double acc[2][NT][2] = {};
+  double a[AHEAD + 1][2][4];
 #pragma unroll
-  for (int d = 0; d < AHEAD; d++) load(d, a[d + 1]);
-  for (int s0 = 0; s0 < steps; s0 += PER) {
+  for (int d = 0; d < AHEAD; d++) load(c_lo + d * STEP, a[d + 1]);
+  for (int c0 = c_lo; c0 < c_hi; c0 += RM_COLS) {
     __syncthreads();
 #pragma unroll
-    for (int v = 0; v < NV; v++)
-      for (int i = threadIdx.x; i < R2_COLS; i += 256) {
-        const int c = s0 * STEP + i;
-        sy[v][i] = c < n ? y[(size_t)v * n + c] : make_double2(0.0, 0.0);
-      }
+    for (int e = tid; e < 4 * NT * RM_COLS; e += 256) {
+      const int v = e / RM_COLS, i = e % RM_COLS;
+      const double2 z = v < nv && c0 + i < n ? y[(size_t)v * n + c0 + i] : make_double2(0.0, 0.0);
+      sy[2 * v][i] = z.x;
+      sy[2 * v + 1][i] = z.y;
+    }
     __syncthreads();
-    const int s1 = min(PER, steps - s0);
+    const int s1 = min(PER, (c_hi - c0 + STEP - 1) / STEP);
 #pragma unroll 2
     for (int s = 0; s < s1; s++) {
 #pragma unroll
       for (int d = 0; d < AHEAD; d++)
 #pragma unroll
-        for (int h = 0; h < 4; h++)
+        for (int m = 0; m < 2; m++)
 #pragma unroll
-          for (int q = 0; q < VEC; q++) a[d][h][q] = a[d + 1][h][q];
-      load(s0 + s + AHEAD, a[AHEAD]);
+          for (int h = 0; h < 4; h++) a[d][m][h] = a[d + 1][m][h];
+      load(c0 + (s + AHEAD) * STEP, a[AHEAD]);
 #pragma unroll
-      for (int v = 0; v < NV; v++)
+      for (int j = 0; j < NT; j++) {
+        const double2* p = reinterpret_cast<const double2*>(&sy[8 * j + r][s * STEP + 4 * q]);
+        const double2 b0 = p[0], b1 = p[1];
 #pragma unroll
-        for (int q = 0; q < VEC; q++) {
-          const double2 t = sy[v][s * STEP + lane * VEC + q];
-#pragma unroll
-          for (int h = 0; h < 4; h++) {
-            sr[h][v] += a[0][h][q] * t.x;
-            si[h][v] += a[0][h][q] * t.y;
-          }
+        for (int m = 0; m < 2; m++) {
+          mma884(acc[m][j], a[0][m][0], b0.x);
+          mma884(acc[m][j], a[0][m][1], b0.y);
+          mma884(acc[m][j], a[0][m][2], b1.x);
+          mma884(acc[m][j], a[0][m][3], b1.y);
         }
-    }
-  }
-#pragma unroll
-  for (int h = 0; h < 4; h++)
-#pragma unroll
-    for (int v = 0; v < NV; v++)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sr[h][v] += __shfl_xor_sync(0xffffffffu, sr[h][v], o);
-        si[h][v] += __shfl_xor_sync(0xffffffffu, si[h][v], o);
-      }
-  if (lane == 0) {
-#pragma unroll
-    for (int h = 0; h < 4; h++) {
-      if (row0 + h >= n) break;
-#pragma unroll
-      for (int v = 0; v < NV; v++) {
-        const size_t o = (size_t)v * n + row0 + h;
-        r[o] = make_double2(b[o].x - x[o].x + sr[h][v], b[o].y - x[o].y + si[h][v]);
       }
     }
   }
+#pragma unroll
+  for (int m = 0; m < 2; m++)
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+      if (row0 + 8 * m < n && 4 * j + q < nv)
+        part[((size_t)blockIdx.y * nv + 4 * j + q) * n + row0 + 8 * m] = make_double2(acc[m][j][0], acc[m][j][1]);
+}
+
+// r = b - x + the sum of the slabs, in order
+__global__ void k_residual_sum(const double2* __restrict__ part, int slabs, size_t total,
+                               const double2* __restrict__ b, const double2* __restrict__ x, double2* __restrict__ r) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  double2 s = part[t];
+  for (int i = 1; i < slabs; i++) {
+    const double2 p = part[(size_t)i * total + t];
+    s.x += p.x;
+    s.y += p.y;
+  }
+  r[t] = make_double2(b[t].x - x[t].x + s.x, b[t].y - x[t].y + s.y);
+}
+
+// Slabs of columns: the number whose CTAs fill their last wave best, each costing a
+// pass over the vectors, about a hundredth of a CTA's work
+int residual_slabs(int n) {
+  const int rows = ceil_div(n, RM_ROWS), slots = 2 * device_sm_count();
+  int best = 1;
+  double least = 1e30;
+  for (int s = 1; s <= std::min((int)ceil_div(n, RM_COLS), RM_SLABS); s++) {
+    const double t = (double)ceil_div((size_t)rows * s, slots) / s + 0.01 * s * rows / slots;
+    if (t < least) {
+      least = t;
+      best = s;
+    }
+  }
+  return best;
 }
 
 template <int VEC>
-void launch_residual(int nv, const double* A, int n, const double2* y, const double2* b, const double2* x, double2* r,
-                     cudaStream_t st) {
-  const unsigned grid = ceil_div((size_t)n, R2_ROWS);
-  switch (nv) {
-    case 1: k_residual<1, VEC><<<grid, 256, 0, st>>>(A, n, y, b, x, r); break;
-    case 2: k_residual<2, VEC><<<grid, 256, 0, st>>>(A, n, y, b, x, r); break;
-    case 3: k_residual<3, VEC><<<grid, 256, 0, st>>>(A, n, y, b, x, r); break;
-    default: k_residual<4, VEC><<<grid, 256, 0, st>>>(A, n, y, b, x, r); break;
+void launch_residual(const double* A, int n, const double2* y, int nv, int slabs, double2* part, cudaStream_t st) {
+  const dim3 grid(ceil_div(n, RM_ROWS), slabs);
+  switch ((nv + 3) / 4) {
+    case 1: k_residual<1, VEC><<<grid, 256, 0, st>>>(A, n, y, nv, slabs, part); break;
+    case 2: k_residual<2, VEC><<<grid, 256, 0, st>>>(A, n, y, nv, slabs, part); break;
+    default: k_residual<3, VEC><<<grid, 256, 0, st>>>(A, n, y, nv, slabs, part); break;
   }
 }
 
@@ -446,17 +466,24 @@ int hadamard_device(const double* d_G, const int32_t* d_rhs_e, int n, const doub
 
 int residual_multi_device(const double* d_A, int n, const double* d_y, const double* d_b, const double* d_x, int nrhs,
                           double* d_r, cudaStream_t st) {
-  // one pass over A per group of up to 4 vectors
-  ProfScope prof(TT_PROF_RESIDUAL, st, 4.0 * n * (double)n * nrhs, 8.0 * n * (double)n * ((nrhs + 3) / 4));
-  for (int v0 = 0; v0 < nrhs; v0 += 4) {
-    const int nv = std::min(4, nrhs - v0);
-    const size_t o = (size_t)v0 * n;
+  // one pass over A per group of up to 4 RM_NT vectors
+  constexpr int GROUP = 4 * RM_NT;
+  ProfScope prof(TT_PROF_RESIDUAL, st, 4.0 * n * (double)n * nrhs, 8.0 * n * (double)n * ceil_div(nrhs, GROUP));
+  const int slabs = residual_slabs(n);
+  DevBuf<double2> part;
+  TT_TRY(part.alloc((size_t)slabs * std::min(nrhs, GROUP) * n));
+  for (int v0 = 0; v0 < nrhs; v0 += GROUP) {
+    const int nv = std::min(GROUP, nrhs - v0);
+    const size_t o = (size_t)v0 * n, total = (size_t)nv * n;
     const double2* y = reinterpret_cast<const double2*>(d_y) + o;
-    const double2* b = reinterpret_cast<const double2*>(d_b) + o;
-    const double2* x = reinterpret_cast<const double2*>(d_x) + o;
-    double2* r = reinterpret_cast<double2*>(d_r) + o;
-    if (n % 2 == 0) launch_residual<2>(nv, d_A, n, y, b, x, r, st);
-    else launch_residual<1>(nv, d_A, n, y, b, x, r, st);
+    if (n % 2 == 0) launch_residual<2>(d_A, n, y, nv, slabs, part.ptr, st);
+    else launch_residual<1>(d_A, n, y, nv, slabs, part.ptr, st);
+    count_launch();
+    TT_CUDA_TRY(cudaGetLastError());
+    k_residual_sum<<<ceil_div(total, 256), 256, 0, st>>>(part.ptr, slabs, total,
+                                                        reinterpret_cast<const double2*>(d_b) + o,
+                                                        reinterpret_cast<const double2*>(d_x) + o,
+                                                        reinterpret_cast<double2*>(d_r) + o);
     count_launch();
     TT_CUDA_TRY(cudaGetLastError());
   }
