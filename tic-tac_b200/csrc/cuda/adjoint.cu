@@ -47,6 +47,9 @@ __global__ void k_transpose_inplace(T* __restrict__ a, int n) {
 // in shared memory.  Bound: A read once.  Slabs, not atomics, collect the rows:
 // the sums come out the same every time.  n = 24,300, 4 vectors: 1.17 -> 0.70 ms
 // (6.7 TB/s; a column a thread with atomics before).
+// Rows are added up GT_CHUNK at a time and those sums in turn: a quarter of the
+// rounding of one sum down the slab, at the same time; the Pade determinants amplify it
+// by nine orders (elastic amplitudes of two runs 7e-7 apart, 1e-7 now).
 constexpr int GT_MAXV = 8, GT_CHUNK = 128, GT_THREADS = 256;
 template <int NV, int VEC>
 __global__ void __launch_bounds__(GT_THREADS, 2) k_gemv_t(const double* __restrict__ A, int n, int slab,
@@ -58,11 +61,11 @@ __global__ void __launch_bounds__(GT_THREADS, 2) k_gemv_t(const double* __restri
   const int r0 = blockIdx.y * slab, r1 = min(n, r0 + slab);
   const bool in = c < n;
   const double* Ac = A + (in ? c : 0);
-  double ar[VEC][NV], ai[VEC][NV];
+  double ar[VEC][NV], ai[VEC][NV], sr[VEC][NV], si[VEC][NV];  // sums over a chunk, over the chunks before
 #pragma unroll
   for (int x = 0; x < VEC; x++)
 #pragma unroll
-    for (int k = 0; k < NV; k++) ar[x][k] = ai[x][k] = 0.0;
+    for (int k = 0; k < NV; k++) sr[x][k] = si[x][k] = 0.0;
   double cur[U][VEC], nxt[U][VEC];
   auto load = [&](int r, double(&d)[U][VEC]) {
 #pragma unroll
@@ -86,6 +89,10 @@ __global__ void __launch_bounds__(GT_THREADS, 2) k_gemv_t(const double* __restri
     }
     __syncthreads();
     const int rn = min(GT_CHUNK, r1 - rb);
+#pragma unroll
+    for (int x = 0; x < VEC; x++)
+#pragma unroll
+      for (int k = 0; k < NV; k++) ar[x][k] = ai[x][k] = 0.0;
     for (int i = 0; i < rn; i += U) {
 #pragma unroll
       for (int u = 0; u < U; u++)
@@ -105,6 +112,13 @@ __global__ void __launch_bounds__(GT_THREADS, 2) k_gemv_t(const double* __restri
         }
       }
     }
+#pragma unroll
+    for (int x = 0; x < VEC; x++)
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        sr[x][k] += ar[x][k];
+        si[x][k] += ai[x][k];
+      }
   }
   if (!in) return;
 #pragma unroll
@@ -112,7 +126,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) k_gemv_t(const double* __restri
     if (k < nrhs) {
       double2* o = part + ((size_t)blockIdx.y * nrhs + k) * n + c;
 #pragma unroll
-      for (int x = 0; x < VEC; x++) o[x] = make_double2(ar[x][k], ai[x][k]);
+      for (int x = 0; x < VEC; x++) o[x] = make_double2(sr[x][k], si[x][k]);
     }
 }
 
