@@ -1454,75 +1454,85 @@ __global__ void __launch_bounds__(256) k_trsm_blk(TrsmBatch<T> tb, int n, int r0
 // 64-byte row segment allows).  It stands for the explicit inverse of a mid-panel's
 // block, a pack, a tensor-core product and another pack (66 -> 13 us on average at 128 x up to
 // 384, n = 16,128) and for k_trsm_blk's substitution row by row (10 -> 4 us at 32 x up to 96).
+// complex128 (h = 32, not packed): 11.5 -> 7.2 us on average over the factorisation of
+// n = 8,496.
 constexpr int TR_MAX = 128, TR_COLS = 8, TR_XLD = TR_COLS + 1;
-template <int NB>
+template <typename T, int NB>
 constexpr size_t trsm_rows_smem() {
-  return sizeof(float2) * (32 * NB * (32 * NB + 2) + 32 * NB * TR_XLD + 32 * NB * INV32_LD + INV32_SCRATCH * NB);
+  return sizeof(T) * (32 * NB * (32 * NB + 2) + 32 * NB * TR_XLD + 32 * NB * INV32_LD + INV32_SCRATCH * NB);
 }
-__device__ __forceinline__ void tr_cp_async8(float2* dst, const float2* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
+// two neighbouring elements of shared memory, the first on a 2-element boundary
+__device__ __forceinline__ void load_pair(const float2* p, float2& a, float2& b) {
+  const float4 f = *reinterpret_cast<const float4*>(p);
+  a = make_float2(f.x, f.y);
+  b = make_float2(f.z, f.w);
 }
-template <int NB>
-__global__ void __launch_bounds__(256) k_trsm_rows(TrsmBatch<float2> tb, int n, int r0, int cb, int ce, int pack_mode) {
+__device__ __forceinline__ void load_pair(const double2* p, double2& a, double2& b) {
+  a = p[0];
+  b = p[1];
+}
+template <typename T, int NB>
+__global__ void __launch_bounds__(256) k_trsm_rows(TrsmBatch<T> tb, int n, int r0, int cb, int ce, int pack_mode) {
   constexpr int H = 32 * NB, LD = H + 2;
   extern __shared__ __align__(16) unsigned char tr_raw[];
-  float2* sL = reinterpret_cast<float2*>(tr_raw);  // [H][LD]
-  float2* sX = sL + H * LD;                        // [H][TR_XLD]
-  float2* sD = sX + H * TR_XLD;                    // [H][INV32_LD]
-  float2* sS = sD + H * INV32_LD;
-  float2* A = tb.A[blockIdx.y];
-  void* WB = tb.WB + tb.plane * blockIdx.y;
+  T* sL = reinterpret_cast<T*>(tr_raw);  // [H][LD]
+  T* sX = sL + H * LD;                   // [H][TR_XLD]
+  T* sD = sX + H * TR_XLD;               // [H][INV32_LD]
+  T* sS = sD + H * INV32_LD;
+  T* A = tb.A[blockIdx.y];
+  void* WB = tb.WB ? tb.WB + tb.plane * blockIdx.y : nullptr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = threadIdx.x / TR_COLS, col = threadIdx.x % TR_COLS;
   for (int i = warp; i < H; i += 8)
     for (int q = 0; q <= i / 32; q++)
-      tr_cp_async8(sL + i * LD + 32 * q + lane, A + (size_t)(r0 + i) * n + r0 + 32 * q + lane);
+      sp_cp_async(sL + i * LD + 32 * q + lane, A + (size_t)(r0 + i) * n + r0 + 32 * q + lane);
   for (int c0 = cb + blockIdx.x * TR_COLS; c0 < ce; c0 += gridDim.x * TR_COLS) {
     const int c = c0 + col;
 #pragma unroll
     for (int q = 0; q < NB; q++) {
       const int i = 32 * q + row;
       if (c < ce)
-        tr_cp_async8(sX + i * TR_XLD + col, A + (size_t)(r0 + i) * n + c);
+        sp_cp_async(sX + i * TR_XLD + col, A + (size_t)(r0 + i) * n + c);
       else
-        sX[i * TR_XLD + col] = make_float2(0, 0);
+        sX[i * TR_XLD + col] = T{0, 0};
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     if (c0 == cb + (int)blockIdx.x * TR_COLS) inv_unit32<NB, LD>(sL, sD, sS);
 #pragma unroll
     for (int j = 0; j < NB; j++) {
-      const float2* Y = sD + (32 * j + row) * INV32_LD;
-      const float2* xj = sX + 32 * j * TR_XLD + col;
-      float2 v[2] = {make_float2(0, 0), make_float2(0, 0)};
+      const T* Y = sD + (32 * j + row) * INV32_LD;
+      const T* xj = sX + 32 * j * TR_XLD + col;
+      T v[2] = {T{0, 0}, T{0, 0}};
 #pragma unroll 4
       for (int k = 0; k < warp * 4; k += 2) {
-        const float4 y = *reinterpret_cast<const float4*>(Y + k);
-        cfma_add(v[0], make_float2(y.x, y.y), xj[k * TR_XLD]);
-        cfma_add(v[1], make_float2(y.z, y.w), xj[(k + 1) * TR_XLD]);
+        T y0, y1;
+        load_pair(Y + k, y0, y1);
+        cfma_add(v[0], y0, xj[k * TR_XLD]);
+        cfma_add(v[1], y1, xj[(k + 1) * TR_XLD]);
       }
 #pragma unroll
       for (int u = 0; u < 4; u++)
         if (warp * 4 + u <= row) cfma_add(v[u & 1], Y[warp * 4 + u], xj[(warp * 4 + u) * TR_XLD]);
       __syncthreads();
-      sX[(32 * j + row) * TR_XLD + col] = make_float2(v[0].x + v[1].x, v[0].y + v[1].y);
+      sX[(32 * j + row) * TR_XLD + col] = T{v[0].x + v[1].x, v[0].y + v[1].y};
       __syncthreads();
       if (j + 1 < NB) {
         constexpr int REST = NB > 1 ? NB - 1 : 1;
-        float2 a[REST];
+        T a[REST];
 #pragma unroll
         for (int u = 0; u < REST; u++)
           if (j + 1 + u < NB) a[u] = sX[(32 * (j + 1 + u) + row) * TR_XLD + col];
 #pragma unroll 4
         for (int k = 0; k < 32; k += 2) {
-          const float2 b0 = xj[k * TR_XLD], b1 = xj[(k + 1) * TR_XLD];
+          const T b0 = xj[k * TR_XLD], b1 = xj[(k + 1) * TR_XLD];
 #pragma unroll
           for (int u = 0; u < REST; u++)
             if (j + 1 + u < NB) {
-              const float4 l = *reinterpret_cast<const float4*>(sL + (32 * (j + 1 + u) + row) * LD + 32 * j + k);
-              cfma_sub(a[u], make_float2(l.x, l.y), b0);
-              cfma_sub(a[u], make_float2(l.z, l.w), b1);
+              T l0, l1;
+              load_pair(sL + (32 * (j + 1 + u) + row) * LD + 32 * j + k, l0, l1);
+              cfma_sub(a[u], l0, b0);
+              cfma_sub(a[u], l1, b1);
             }
         }
 #pragma unroll
@@ -1534,10 +1544,12 @@ __global__ void __launch_bounds__(256) k_trsm_rows(TrsmBatch<float2> tb, int n, 
 #pragma unroll
     for (int q = 0; q < NB; q++)
       if (c < ce) A[(size_t)(r0 + 32 * q + row) * n + c] = sX[(32 * q + row) * TR_XLD + col];
-    if (c0 + warp < ce) {
+    if constexpr (sizeof(T) == sizeof(float2)) {
+      if (pack_mode && c0 + warp < ce) {
 #pragma unroll
-      for (int q = 0; q < NB; q++)
-        tc2_pack_b(pack_mode, WB, ce - cb, H, c0 + warp - cb, 32 * q + lane, sX[(32 * q + lane) * TR_XLD + warp]);
+        for (int q = 0; q < NB; q++)
+          tc2_pack_b(pack_mode, WB, ce - cb, H, c0 + warp - cb, 32 * q + lane, sX[(32 * q + lane) * TR_XLD + warp]);
+      }
     }
     __syncthreads();
   }
@@ -1676,12 +1688,46 @@ int inv_unit_lower(const T* const* As, int B, int n, int r0, int w, T* X, T* Tsc
   return TT_OK;
 }
 
+// k_trsm_rows of B <= 4 matrices, h a multiple of 32 up to TR_MAX; no more CTAs than fit
+// at once, as a CTA's block inverses serve all its chunks
+template <typename T, int NB>
+int launch_trsm_rows(const TrsmBatch<T>& tb, int B, int n, int r0, int cb, int ce, int pack_mode, cudaStream_t st) {
+  constexpr size_t smem = trsm_rows_smem<T, NB>();
+  constexpr int resident = std::max(1, std::min(4, (int)(200 * 1024 / smem)));
+  const int chunks = ceil_div(ce - cb, TR_COLS), per = std::max(1, resident * device_sm_count() / B);
+  TT_TRY(smem_limit_once((const void*)k_trsm_rows<T, NB>, (int)smem));
+  k_trsm_rows<T, NB>
+      <<<dim3(ceil_div(chunks, ceil_div(chunks, per)), B), 256, smem, st>>>(tb, n, r0, cb, ce, pack_mode);
+  count_launch();
+  TT_CUDA_TRY(cudaGetLastError());
+  return TT_OK;
+}
+template <typename T>
+int trsm_rows_batched(T* const* As, int B, int n, int r0, int h, int cb, int ce, int pack_mode, unsigned char* WB,
+                      size_t plane, cudaStream_t st) {
+  ProfScope prof(TT_PROF_PANEL_TRSM, st, 4.0 * h * h * (double)(ce - cb) * B,
+                 2.0 * h * (double)(ce - cb) * sizeof(T) * B);
+  TrsmBatch<T> tb{};
+  for (int b = 0; b < B; b++) tb.A[b] = As[b];
+  tb.WB = WB;
+  tb.plane = plane;
+  if constexpr (sizeof(T) == sizeof(float2)) {
+    switch (h / 32) {
+      case 2: return launch_trsm_rows<T, 2>(tb, B, n, r0, cb, ce, pack_mode, st);
+      case 3: return launch_trsm_rows<T, 3>(tb, B, n, r0, cb, ce, pack_mode, st);
+      case 4: return launch_trsm_rows<T, 4>(tb, B, n, r0, cb, ce, pack_mode, st);
+    }
+  }
+  return launch_trsm_rows<T, 1>(tb, B, n, r0, cb, ce, pack_mode, st);
+}
+
 // the same block of B <= 4 matrices (pack_mode: matrix b's solved rows also
 // go to its operand planes at WB + b plane)
 template <typename T>
 int trsm_blk_batched(T* const* As, int B, int n, int r0, int w, int cb, int ce, cudaStream_t st, int pack_mode = 0,
                      unsigned char* WB = nullptr, size_t plane = 0) {
   if (ce <= cb) return TT_OK;
+  if (w == IB) return trsm_rows_batched<T>(As, B, n, r0, w, cb, ce, pack_mode, WB, plane, st);
   ProfScope prof(TT_PROF_PANEL_TRSM, st, 4.0 * w * w * (double)(ce - cb) * B,
                  2.0 * w * (double)(ce - cb) * sizeof(T) * B);
   TrsmBatch<T> tb{};
@@ -1692,35 +1738,6 @@ int trsm_blk_batched(T* const* As, int B, int n, int r0, int w, int cb, int ce, 
   count_launch();
   TT_CUDA_TRY(cudaGetLastError());
   return TT_OK;
-}
-
-// k_trsm_rows of B <= 4 matrices, h a multiple of 32 up to TR_MAX; one CTA an SM at
-// most, as its block inverses serve all its chunks
-template <int NB>
-int launch_trsm_rows(const TrsmBatch<float2>& tb, int B, int n, int r0, int cb, int ce, int pack_mode,
-                     cudaStream_t st) {
-  const int chunks = ceil_div(ce - cb, TR_COLS), per = std::max(1, device_sm_count() / B);
-  constexpr size_t smem = trsm_rows_smem<NB>();
-  TT_TRY(smem_limit_once((const void*)k_trsm_rows<NB>, (int)smem));
-  k_trsm_rows<NB><<<dim3(ceil_div(chunks, ceil_div(chunks, per)), B), 256, smem, st>>>(tb, n, r0, cb, ce, pack_mode);
-  count_launch();
-  TT_CUDA_TRY(cudaGetLastError());
-  return TT_OK;
-}
-int trsm_rows_batched(float2* const* As, int B, int n, int r0, int h, int cb, int ce, int pack_mode, unsigned char* WB,
-                      size_t plane, cudaStream_t st) {
-  ProfScope prof(TT_PROF_PANEL_TRSM, st, 4.0 * h * h * (double)(ce - cb) * B,
-                 2.0 * h * (double)(ce - cb) * sizeof(float2) * B);
-  TrsmBatch<float2> tb{};
-  for (int b = 0; b < B; b++) tb.A[b] = As[b];
-  tb.WB = WB;
-  tb.plane = plane;
-  switch (h / 32) {
-    case 1: return launch_trsm_rows<1>(tb, B, n, r0, cb, ce, pack_mode, st);
-    case 2: return launch_trsm_rows<2>(tb, B, n, r0, cb, ce, pack_mode, st);
-    case 3: return launch_trsm_rows<3>(tb, B, n, r0, cb, ce, pack_mode, st);
-    default: return launch_trsm_rows<4>(tb, B, n, r0, cb, ce, pack_mode, st);
-  }
 }
 
 template <typename T>
@@ -2058,10 +2075,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
           const float2* Us[kMaxBatch];
           float2* Af[kMaxBatch];
           for (int b = 0; b < B; b++) Af[b] = reinterpret_cast<float2*>(As[b]);
-          if (w == 32)
-            TT_TRY(trsm_rows_batched(Af, B, n, j0, w, j0 + w, m0 + mw, mode, WB, plane, st));
-          else
-            TT_TRY(trsm_blk_batched<T>(As, B, n, j0, w, j0 + w, m0 + mw, st, mode, WB, plane));
+          TT_TRY(trsm_blk_batched<T>(As, B, n, j0, w, j0 + w, m0 + mw, st, mode, WB, plane));
           for (int b = 0; b < B; b++) {
             float2* A = Af[b];
             Cs[b] = A + (size_t)(j0 + w) * n + (j0 + w);
