@@ -37,6 +37,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "ll_record.cuh"
 #include "tc2_pack.cuh"
 #include "tt_kernels.h"
 #include "tt_lu_internal.h"
@@ -541,6 +542,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  pdl_wait();
+  pdl_launch_next();
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs)
@@ -881,11 +884,12 @@ int launch_tc2(int nb, float2* const* C, int ldc, const float2* const* L, int ld
     const void* kfn = (const void*)tc2::k_lu_update_tc2_pair<MODE>;
     TT_TRY(smem_limit_once(kfn, (int)smem));
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2] = {};
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1] = pdl_attribute();
     cfg.blockDim = dim3(tc2::NUM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -901,6 +905,7 @@ int launch_tc2(int nb, float2* const* C, int ldc, const float2* const* L, int ld
     }
     const int tiles = nb * ((M + 2 * tc2::BM - 1) / (2 * tc2::BM)) * ((N + tc2::BN - 1) / tc2::BN);
     cfg.gridDim = dim3(2 * std::min(tiles, mp));
+    cfg.numAttrs = 2;
     TT_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc2::k_lu_update_tc2_pair<MODE>, ops, mB, ldc, M, N, K, M, store,
                                    ws.err.ptr));
   } else {

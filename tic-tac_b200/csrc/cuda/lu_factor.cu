@@ -697,6 +697,8 @@ __global__ void __launch_bounds__(32 * SP_WARPS, 1) k_subpanel_ll(SubpanelBatch<
   extern __shared__ __align__(16) unsigned char sp_raw[];
   const int Gb = gridDim.x / bt.B, grp = blockIdx.x / Gb, cta = blockIdx.x - grp * Gb;
   T* __restrict__ A = batch_pick(bt.A, grp);
+  pdl_wait();
+  pdl_launch_next();
   const int m = n - c0;
   const int chunk = (m + Gb - 1) / Gb;
   const int lo = cta * chunk;  // first row of this CTA, from c0
@@ -1483,6 +1485,8 @@ __global__ void __launch_bounds__(256) k_trsm_rows(TrsmBatch<T> tb, int n, int r
   void* WB = tb.WB ? tb.WB + tb.plane * blockIdx.y : nullptr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = threadIdx.x / TR_COLS, col = threadIdx.x % TR_COLS;
+  pdl_wait();
+  pdl_launch_next();
   for (int i = warp; i < H; i += 8)
     for (int q = 0; q <= i / 32; q++)
       sp_cp_async(sL + i * LD + 32 * q + lane, A + (size_t)(r0 + i) * n + r0 + 32 * q + lane);
@@ -1696,10 +1700,16 @@ int launch_trsm_rows(const TrsmBatch<T>& tb, int B, int n, int r0, int cb, int c
   constexpr int resident = std::max(1, std::min(4, (int)(200 * 1024 / smem)));
   const int chunks = ceil_div(ce - cb, TR_COLS), per = std::max(1, resident * device_sm_count() / B);
   TT_TRY(smem_limit_once((const void*)k_trsm_rows<T, NB>, (int)smem));
-  k_trsm_rows<T, NB>
-      <<<dim3(ceil_div(chunks, ceil_div(chunks, per)), B), 256, smem, st>>>(tb, n, r0, cb, ce, pack_mode);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1] = {pdl_attribute()};
+  cfg.gridDim = dim3(ceil_div(chunks, ceil_div(chunks, per)), B);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  TT_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_trsm_rows<T, NB>, tb, n, r0, cb, ce, pack_mode));
   count_launch();
-  TT_CUDA_TRY(cudaGetLastError());
   return TT_OK;
 }
 template <typename T>
@@ -1901,17 +1911,18 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
     const size_t smem = (size_t)chunk * SP * sizeof(T) + SC::EXTRA;
     if (cluster) {
       cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
+      cudaLaunchAttribute attr[2] = {};
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = gb;
       attr[0].val.clusterDim.y = 1;
       attr[0].val.clusterDim.z = 1;
+      attr[1] = pdl_attribute();
       cfg.gridDim = dim3(gb * nb);
       cfg.blockDim = dim3(sp_threads(chunk));
       cfg.dynamicSmemBytes = smem;
       cfg.stream = st;
       cfg.attrs = attr;
-      cfg.numAttrs = 1;
+      cfg.numAttrs = 2;
       TT_CUDA_TRY(cudaLaunchKernelExC(&cfg, kernel, args));
     } else {
       TT_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(gb * nb), dim3(sp_threads(chunk)), args, smem, st));

@@ -188,6 +188,14 @@ struct DeviceCSR {
   DevBuf<double> val;
 };
 
+// Launch attribute of a kernel that begins with pdl_wait()
+inline cudaLaunchAttribute pdl_attribute() {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+
 inline unsigned ceil_div(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
 // Raises a kernel's dynamic shared-memory limit on the current device to at
