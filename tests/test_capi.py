@@ -31,3 +31,14 @@ def test_error_paths_without_device():
     assert lib.tt_run_num_channels(None, None) == tt.TT_ERR_BADARG
     rp = tt.run_params()
     assert rp.Nphi == 48 and rp.Nx == 48 and rp.precision == tt.PRECISION_MIXED
+
+
+def test_device_memory_is_written_in_stream_order():
+    # the library's streams are non-blocking: a plain cudaMemcpy into device memory is
+    # ordered with none of them, and from pageable memory may return before the data is there
+    src = os.path.join(ROOT, "tic-tac_b200", "csrc")
+    files = [os.path.join(d, f) for d, _, fs in os.walk(src) for f in fs if f.endswith((".cpp", ".cu", ".h", ".cuh"))]
+    assert len(files) > 20
+    for f in files:
+        for call in re.findall(r"\bcudaMem(?:cpy|set)(?:2D)?\s*\([^;]*", open(f).read()):
+            assert "cudaMemcpyDeviceToHost" in call, (f, call)

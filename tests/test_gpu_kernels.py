@@ -225,3 +225,23 @@ def test_pivots_in_and_below_the_diagonal_block(precision, Np, kinds):
         row = Np * Np + int(q_idx[j]) * Np
         want = torch.linalg.solve(L, A[:, row].to(L.dtype))[row].item()
         assert abs(U[j] - want) <= 1e-10 * abs(want), (kinds[j], U[j], want, rep)
+
+
+@pytest.mark.parametrize("precision", [tt.PRECISION_FP64, tt.PRECISION_MIXED])
+def test_drop_in_solve_uses_the_callers_resolvents(precision):
+    # A = diag(a): U = a / (1 - a G) at the on-shell element.  Every call brings other
+    # resolvents in pageable memory (147 KB), none of them the resolvent of the grid, whose
+    # first element at E = 0 is 0 log 0
+    Np = Nq = 48
+    n, rng = 2 * Np * Nq, np.random.default_rng(11)
+    pw = np.array([[0, 0, 0, 1, 0, 1, 1, 1, 1], [0, 1, 1, 0, 0, 1, 1, 1, 1]], dtype=np.int32)
+    eye, e = np.tile(np.eye(Np).ravel(), 6), np.tile(np.linspace(0, 100, Np + 1), 6)
+    swp = tt.SWP(Np, Nq, 6, 0, -2.0, e, None, eye, None, np.linspace(0, 1000, Nq + 1))
+    v, q_idx = rng.uniform(0.5, 1.5, n), np.array([3, 40])
+    at = Np * Nq + q_idx * Np
+    for _ in range(8):
+        G = rng.uniform(0.1, 0.3, (2, n)) * np.exp(1j * rng.uniform(0, 2 * np.pi, (2, n)))
+        U, _ = tt.solve_faddeev(G, v, np.arange(n, dtype=np.int32), np.arange(n + 1, dtype=np.uint64), eye, None, swp,
+                                q_idx, [1], tt.PW(pw), precision=precision, tensor_force=0, isospin_breaking_1S0=0)
+        want = 2 * v[at] / (1 - 2 * v[at] * G[[0, 1], at])
+        assert np.all(abs(U - want) <= 1e-10 * abs(want))

@@ -221,13 +221,8 @@ int dropin_solve(tt_complex* U, tt_complex* dU, int n_theta, const double* dVu, 
   double msA = 0;
   s = cs.build_A(st, &msA);
   if (s != TT_OK) return s;
-  // G supplied by the caller: upload into the solver through resolvent-shaped storage
-  std::vector<double> dummyE(os->num_T_lab, 0.0);
-  s = cs.resolvent(dummyE, st);
+  s = cs.set_G_host(reinterpret_cast<const double*>(G), os->num_T_lab, st);
   if (s != TT_OK) return s;
-  if (cudaMemcpy((void*)cs.G(), G, sizeof(tt_complex) * (size_t)n * os->num_T_lab, cudaMemcpyHostToDevice) !=
-      cudaSuccess)
-    return fail(TT_ERR_CUDA, "upload of G failed");
   std::vector<int> q_idx(os->q_com_idx_array, os->q_com_idx_array + os->num_T_lab);
   std::vector<int> deut(os->deuteron_idx_array, os->deuteron_idx_array + os->num_deuteron_states);
   std::vector<double> Uh, dUh, dvc;

@@ -207,6 +207,19 @@ int ChannelSolver::resolvent(const std::vector<double>& E, cudaStream_t st) {
   return TT_OK;
 }
 
+// Copied in the order of st, not by cudaMemcpy: the legacy stream does not order the
+// solver's non-blocking one, and a copy from pageable memory may return before the
+// data has reached the device, so L = 1 - A G could be formed from what the buffer
+// held before (from a pinned G the copy is in flight until the solve has waited for st).
+int ChannelSolver::set_G_host(const double* G, int nE, cudaStream_t st) {
+  nE_ = nE;
+  Eh_.assign(nE, 0.0);  // the energies of a caller's resolvents are not known
+  TT_TRY(G_.alloc((size_t)2 * n * std::max(1, nE)));
+  if (n > 0 && nE > 0)
+    TT_CUDA_TRY(cudaMemcpyAsync(G_.ptr, G, sizeof(double) * 2 * n * nE, cudaMemcpyHostToDevice, st));
+  return TT_OK;
+}
+
 namespace {
 
 // Panel width of the complex64 LU for order n and tensor-core product.

@@ -99,6 +99,9 @@ class ChannelSolver {
   int build_A(cudaStream_t st, double* ms = nullptr);
   // resolvent for energies E (= E_com + E_bound) into device G [nE][n]
   int resolvent(const std::vector<double>& E, cudaStream_t st);
+  // the caller's resolvents G [nE][n] (complex128, host) in their place; the copy may
+  // still read G until st has been waited for
+  int set_G_host(const double* G, int nE, cudaStream_t st);
   // U[d'*nd*nE + d*nE + j] for each on-shell q bin j and deuteron states
   int solve(const std::vector<int>& q_idx, const std::vector<int>& deut, const SolveOptions& opt,
             std::vector<double>& U_interleaved, SolveReport* rep, cudaStream_t st,
