@@ -136,6 +136,40 @@ def test_empty_matrix(tmp_path):
     assert len(r) == len(c) == len(v) == 0
 
 
+def test_arrays_outlive_exit_handlers(tmp_path):
+    # a handler registered before the library is loaded runs after all that the library
+    # itself may do at exit; blocks of 8 MB go back to the system when they are freed
+    import os
+    import subprocess
+    import sys
+
+    ch = channel("mt_swave_n16", 0)
+    m = 1 << 21
+    p, q = np.linspace(0, 1, 1449), np.linspace(0, 1, 1449)
+    path = tmp_path / "P123.h5"
+    at = np.arange(m, dtype=np.int32)
+    tt.store_P123_h5(path, at, at, at + 0.5, ch["pw"], p, q)
+    code = """
+import atexit, os, sys
+kept = []
+def at_exit():
+    at, val = np.arange(%d, dtype=np.int32), np.arange(%d) + 0.5
+    r, c, v = kept
+    ok = np.array_equal(r, at) and np.array_equal(c, at) and np.array_equal(v, val)
+    print("equal" if ok else "garbage", flush=True)
+atexit.register(at_exit)
+import numpy as np
+import tictac_b200 as tt
+z = np.load(sys.argv[2])
+kept += tt.read_P123_h5(sys.argv[1], tt.PW(z["pw"]), z["p"], z["q"])
+""" % (m, m)
+    np.savez(tmp_path / "in.npz", pw=np.asarray(ch["pwt"]).reshape(-1, 9), p=p, q=q)
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join(sys.path))
+    out = subprocess.run([sys.executable, "-c", code, str(path), str(tmp_path / "in.npz")], env=env, text=True,
+                         capture_output=True, timeout=300)
+    assert out.returncode == 0 and out.stdout.split() == ["equal"], (out.returncode, out.stdout, out.stderr)
+
+
 def _library_style_file(path, ch, leaf_k, split=False):
     """The same objects with the tables chunked (10 records per chunk) and of
     unlimited maximum size, as H5TBmake_table stores them, the links spread

@@ -205,9 +205,10 @@ class PW:
 
 
 def _owned_array(ptr, m):
-    """The library's m elements at ptr as an array that frees them with itself (no copy)."""
+    """The library's m elements at ptr as an array that frees them with itself (no copy),
+    at the interpreter's exit not before it is gone: exit handlers and daemon threads may use it."""
     buf = (ptr._type_ * max(m, 1)).from_address(ctypes.addressof(ptr.contents))
-    weakref.finalize(buf, _lib.tt_free, ctypes.cast(ptr, c_void_p))
+    weakref.finalize(buf, _lib.tt_free, ctypes.cast(ptr, c_void_p)).atexit = False
     return np.frombuffer(buf, dtype=np.dtype(ptr._type_), count=m)
 
 
