@@ -245,3 +245,29 @@ def test_drop_in_solve_uses_the_callers_resolvents(precision):
                                 q_idx, [1], tt.PW(pw), precision=precision, tensor_force=0, isospin_breaking_1S0=0)
         want = 2 * v[at] / (1 - 2 * v[at] * G[[0, 1], at])
         assert np.all(abs(U - want) <= 1e-10 * abs(want))
+
+
+def test_pade_determinants_with_rows_exchanged():
+    # coefficients that grow threefold an order: every column of the determinants has its
+    # pivot in the last row.  Approximants stop 1e-7 apart on elements of 0.02 to 0.05, so
+    # 5e-6 relative, and a few times that from the solution; a wrong pivot gives another value
+    import torch
+
+    Np = Nq = 8
+    n, rng = 2 * Np * Nq, np.random.default_rng(3)
+    pw = np.array([[0, 0, 0, 1, 0, 1, 1, 1, 1], [0, 1, 1, 0, 0, 1, 1, 1, 1]], dtype=np.int32)
+    eye, e = np.tile(np.eye(Np).ravel(), 6), np.tile(np.linspace(-2, 100, Np + 1), 6)
+    swp = tt.SWP(Np, Nq, 6, 0, -2.0, e, None, eye, None, np.linspace(0, 1000, Nq + 1))
+    Q, _ = np.linalg.qr(rng.standard_normal((n, 8)))
+    A = (Q * 3.0 * 0.4 ** np.arange(8)) @ Q.T
+    q_idx, G = np.arange(8), np.exp(1j * np.linspace(0.5, 2.5, 8))[:, None] * np.ones(n)
+    args = (G, (A / 2).T.ravel(), np.tile(np.arange(n, dtype=np.int32), n), np.arange(0, n * n + 1, n, dtype=np.uint64),
+            eye, None, swp, q_idx, [1], tt.PW(pw))
+    U = [tt.solve_faddeev(*args, precision=tt.PRECISION_PADE, tensor_force=0, isospin_breaking_1S0=0)[0]
+         for _ in range(3)]
+    at = Np * Nq + q_idx * Np
+    want = np.array([torch.linalg.solve(torch.eye(n, dtype=torch.complex128) - torch.from_numpy(A * G[j]),
+                                        torch.from_numpy(A[:, at[j]]).to(torch.complex128))[at[j]].item()
+                     for j in range(8)])
+    assert np.all(abs(U[0] - want) <= 1e-4 * abs(want).max())
+    assert np.array_equal(U[0], U[1]) and np.array_equal(U[0], U[2])

@@ -58,6 +58,7 @@ __device__ double2 warp_det(double2* m, int S, int lane) {
     }
     if (v < 0) p = k;
     const double2 piv = m[p * PD_S + k];
+    __syncwarp();  // every lane has it before the rows change places
     if (piv.x == 0.0 && piv.y == 0.0) return make_double2(0.0, 0.0);
     if (p != k) {
       if (lane >= k && lane < S) {
