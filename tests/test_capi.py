@@ -2,6 +2,7 @@
 import ctypes
 import os
 import re
+import subprocess
 
 import tictac_b200 as tt
 from conftest import ROOT
@@ -42,3 +43,53 @@ def test_device_memory_is_written_in_stream_order():
     for f in files:
         for call in re.findall(r"\bcudaMem(?:cpy|set)(?:2D)?\s*\([^;]*", open(f).read()):
             assert "cudaMemcpyDeviceToHost" in call, (f, call)
+
+
+def test_a_failed_call_waits_for_its_stream(tmp_path):
+    # the buffers' scope against a CUDA runtime of counters: what a failed call left queued
+    # may use buffers that the next call frees on another stream
+    (tmp_path / "main.cpp").write_text(r"""
+#include <cstdio>
+#include "cuda/tt_device.h"
+static int waits = 0;
+static unsigned long errors = 0;
+namespace tt {
+void set_error(const std::string&) { errors++; }
+unsigned long error_count() { return errors; }
+}
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaMalloc(void**, size_t) { return cudaErrorMemoryAllocation; }
+cudaError_t cudaFree(void*) { return cudaSuccess; }
+cudaError_t cudaFreeAsync(void*, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { waits += s == (cudaStream_t)8; return cudaSuccess; }
+cudaError_t cudaMallocFromPoolAsync(void**, size_t, cudaMemPool_t, cudaStream_t) { return cudaErrorMemoryAllocation; }
+cudaError_t cudaMemPoolCreate(cudaMemPool_t*, const cudaMemPoolProps*) { return cudaErrorNotSupported; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
+cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaErrorNotSupported; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+}
+static void call(cudaStream_t st, bool fails) {
+  tt::StreamScope scope(st);
+  if (fails) tt::set_error("x");
+}
+int main() {
+  call((cudaStream_t)8, false);
+  const int good = waits;
+  call((cudaStream_t)8, true);
+  const int failed = waits;
+  call(nullptr, true);
+  { tt::StreamScope outer((cudaStream_t)8); call((cudaStream_t)16, true); }
+  std::printf("%d %d %d", good, failed, waits);
+}
+""")
+    src = os.path.join(ROOT, "tic-tac_b200", "csrc")
+    cuda = os.environ.get("CUDA", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-I" + src, "-I" + os.path.join(ROOT, "include"), "-I" + cuda + "/include",
+                    str(tmp_path / "main.cpp"), os.path.join(src, "host", "tt_device_cache.cpp"), "-o",
+                    str(tmp_path / "main")], check=True, capture_output=True, text=True)
+    good, failed, both = map(int, subprocess.run([str(tmp_path / "main")], capture_output=True, text=True,
+                                                 check=True).stdout.split())
+    assert (good, failed, both) == (0, 1, 2)

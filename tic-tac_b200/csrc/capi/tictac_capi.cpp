@@ -29,7 +29,12 @@
 namespace tt {
 
 static thread_local std::string g_last_error;
-void set_error(const std::string& msg) { g_last_error = msg; }
+static thread_local unsigned long g_errors = 0;
+void set_error(const std::string& msg) {
+  g_errors++;
+  g_last_error = msg;
+}
+unsigned long error_count() { return g_errors; }
 const char* last_error() { return g_last_error.c_str(); }
 
 static std::atomic<unsigned long long> g_launches{0};

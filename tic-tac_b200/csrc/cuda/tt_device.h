@@ -11,6 +11,7 @@
 namespace tt {
 
 void set_error(const std::string& msg);
+unsigned long error_count();  // set_error() calls of this thread so far
 const char* last_error();
 
 // Count of kernels this library has launched (reported by tt_kernel_launches).
@@ -70,7 +71,9 @@ void device_cache_trim();     // frees the current device's cached blocks
 // on; a buffer released under a scope is freed in that stream's order, so it may
 // still be in use there, and the driver orders its reuse on other streams and
 // threads.  Every entry point waits for its stream before it returns, so a
-// buffer that outlives the call may next be used under another stream's scope.
+// buffer that outlives the call (a thread's operand planes) may next be used or freed
+// under another stream's scope, and the caller's arrays may go; a scope in which an
+// error was set waits for its stream itself, since error returns leave work queued.
 // Without a scope buffers are allocated with cudaMalloc and released with
 // cudaFree, which waits.  The pool keeps at most kPoolKeepBytes of idle memory;
 // device_pool_trim() (an allocation that would fail,
@@ -84,6 +87,7 @@ struct StreamScope {
 
  private:
   cudaStream_t prev_;
+  unsigned long errors_;
 };
 cudaError_t device_pool_alloc(void** p, size_t bytes, bool* pooled);
 void device_pool_free(void* p);

@@ -54,8 +54,11 @@ thread_local cudaStream_t g_scope = nullptr;
 
 }  // namespace
 
-StreamScope::StreamScope(cudaStream_t st) : prev_(g_scope) { g_scope = st; }
-StreamScope::~StreamScope() { g_scope = prev_; }
+StreamScope::StreamScope(cudaStream_t st) : prev_(g_scope), errors_(error_count()) { g_scope = st; }
+StreamScope::~StreamScope() {
+  if (g_scope && error_count() != errors_ && cudaStreamSynchronize(g_scope) != cudaSuccess) cudaGetLastError();
+  g_scope = prev_;
+}
 
 cudaError_t device_pool_alloc(void** p, size_t bytes, bool* pooled) {
   *pooled = false;
