@@ -93,3 +93,17 @@ int main() {
     good, failed, both = map(int, subprocess.run([str(tmp_path / "main")], capture_output=True, text=True,
                                                  check=True).stdout.split())
     assert (good, failed, both) == (0, 1, 2)
+
+
+def test_aligned_barriers_follow_a_converged_warp():
+    # inline bar.sync and barrier.cluster.*.aligned are undefined for a warp whose lanes
+    # arrive apart, and the compiler does not converge it for them
+    src = os.path.join(ROOT, "tic-tac_b200", "csrc", "cuda")
+    found = 0
+    for f in ("lu_factor.cu",):
+        lines = open(os.path.join(src, f)).read().split("\n")
+        for i, line in enumerate(lines):
+            if "asm" in line and re.search(r"\bbar\.sync|barrier\.cluster\.arrive", line):
+                assert lines[i - 1].strip().startswith("__syncwarp();"), (f, i + 1)
+                found += 1
+    assert found == 2

@@ -395,6 +395,14 @@ inline int sp_threads(int rows) {
   return std::max(TRY_THREADS, 32 * ((rows + 32 * sp_rpt(rows) - 1) / (32 * sp_rpt(rows)) + 1));
 }
 
+// Barrier of the warps that factor the diagonal block.  Its aligned form is for converged
+// warps, and inline code is not converged by the compiler: lanes that took different
+// branches meet first.
+__device__ __forceinline__ void sp_block_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(TRY_THREADS) : "memory");
+}
+
 // LU of the sub-panel's w x w diagonal block in sD (row stride TRY_LD), every pivot on the
 // diagonal; false (to some thread) if an element of the block would have been the pivot.
 // Thread t of 256 keeps row t / 8, columns 4 (t % 8) to + 3.  A step takes four columns:
@@ -471,7 +479,7 @@ __device__ __forceinline__ bool sp_factor_diag(T* sD, T* sRd, Key* sBest, int w,
           }
       }
     }
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+    sp_block_sync();
   }
 #pragma unroll
   for (int c = 0; c < W; c++) sD[i * TRY_LD + W * g + c] = a[c];
@@ -495,7 +503,7 @@ __device__ __forceinline__ void sp_factor_block(T* sD, T* sRd, Key* sBest, int* 
   T a[CW];
 #pragma unroll
   for (int k = 0; k < CW; k++) a[k] = sD[lane * TRY_LD + CW * warp + k];
-  asm volatile("bar.sync 1, 256;" ::: "memory");  // the block is in registers, sD holds multipliers from here on
+  sp_block_sync();  // the block is in registers, sD holds multipliers from here on
 #pragma unroll 1
   for (int q = 0; CW * q < w; q++) {
     T* mult = sD + (q & 1) * CW * IB;  // [CW][IB]
@@ -535,7 +543,7 @@ __device__ __forceinline__ void sp_factor_block(T* sD, T* sRd, Key* sBest, int* 
         }
       }
     }
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+    sp_block_sync();
     if (warp != q) {
 #pragma unroll
       for (int k = 0; k < CW; k++) {
@@ -561,7 +569,7 @@ __device__ __forceinline__ void sp_factor_block(T* sD, T* sRd, Key* sBest, int* 
       }
     }
   }
-  asm volatile("bar.sync 1, 256;" ::: "memory");
+  sp_block_sync();
 #pragma unroll
   for (int k = 0; k < CW; k++) sD[lane * TRY_LD + CW * warp + k] = a[k];
 }
@@ -664,6 +672,7 @@ __device__ __forceinline__ bool sp_try_row(T* row, const T* sD, const T* sRd, co
 // 84 us, and a verdict costs 900 cycles against 2,500 to 5,000.  Taller sub-panels would
 // need more rows a CTA than SP_ROWS, and meet in L2.
 __device__ __forceinline__ void sp_cluster_sync() {
+  __syncwarp();  // an aligned barrier, as sp_block_sync's
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t sp_remote(const void* p, int rank) {
