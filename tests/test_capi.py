@@ -96,14 +96,14 @@ int main() {
 
 
 def test_aligned_barriers_follow_a_converged_warp():
-    # inline bar.sync and barrier.cluster.*.aligned are undefined for a warp whose lanes
-    # arrive apart, and the compiler does not converge it for them
+    # inline bar.sync, barrier.cluster.*.aligned and tcgen05.*.sync.aligned are undefined for
+    # a warp whose lanes arrive apart, and the compiler does not converge it for them
     src = os.path.join(ROOT, "tic-tac_b200", "csrc", "cuda")
     found = 0
-    for f in ("lu_factor.cu",):
-        lines = open(os.path.join(src, f)).read().split("\n")
-        for i, line in enumerate(lines):
-            if "asm" in line and re.search(r"\bbar\.sync|barrier\.cluster\.arrive", line):
-                assert lines[i - 1].strip().startswith("__syncwarp();"), (f, i + 1)
-                found += 1
-    assert found == 2
+    for f in ("lu_factor.cu", "gemm_tc2.cu", "gemm_tc.cu"):
+        text = open(os.path.join(src, f)).read()
+        for m in re.finditer(r'asm volatile\(\s*"(bar\.sync|barrier\.cluster\.arrive|tcgen05\.(?:alloc|ld))', text):
+            before = re.sub(r"//.*|if \(warp == 0\) \{", "", text[:m.start()]).rstrip()
+            assert before.endswith("__syncwarp();"), (f, text.count("\n", 0, m.start()) + 1)
+            found += 1
+    assert found == 8

@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(AB_THREADS, 2) k_abuild(AbLayout ly1, AbLayout
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[j][0] = acc[j][1] = 0.0;
         const double* Tk = sT + (size_t)tig * LD + gid;
+        __syncwarp();  // after the stores' branches: mma.sync.aligned
 #pragma unroll
         for (int ks = 0; ks < KMAX; ks++) {
           if (ks >= KS) break;

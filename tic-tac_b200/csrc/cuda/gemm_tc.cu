@@ -130,6 +130,7 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
       "%15}, [%16];"
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();  // .sync.aligned is for converged warps
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)),
                  "r"(TMEM_COLS));
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       sched.coords(t, tm, tn);
       const int ab = local & 1;
       const uint32_t aph = (uint32_t)(local >> 1) & 1u;
-      if (!mbar_wait(&acc_full[ab], aph, err, 4)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[ab], aph, err, 4))) break;
       tc_fence_after();
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * (2 * BN);
       const int row0 = tm * BM + quarter * 32;

@@ -186,6 +186,7 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
       "%15}, [%16];"
@@ -268,6 +269,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();  // .sync.aligned is for converged warps
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)),
                  "r"(TMEM_COLS));
@@ -372,7 +374,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       float2 cv[16];
       // the first chunk's C is fetched while the accumulator fills (store: C = acc, nothing to fetch)
       if (!store) load_c_chunk(C, ldc, M, N, row0, tn * BN + half * (BN / 2), lane, cv);
-      if (!mbar_wait(&acc_full[ab], aph, err, 4)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[ab], aph, err, 4))) break;
       tc_fence_after();
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * (2 * BN);
 #pragma unroll 1
@@ -481,6 +483,7 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // 2D tile copy into this CTA's shared memory completing on an mbarrier of the
@@ -532,6 +535,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     mbar_init(fin, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();  // .sync.aligned is for converged warps
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)),
                  "r"(TMEM_COLS));
@@ -642,7 +646,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       const int row0 = tm * 2 * BM + (int)rank * BM + quarter * 32;
       float2 cv[16];
       if (!store) load_c_chunk(C, ldc, M, N, row0, tn * BN + half * (BN / 2), lane, cv);
-      if (!mbar_wait(&acc_full[ab], aph, err, 4)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[ab], aph, err, 4))) break;
       tc_fence_after();
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + ab * (2 * BN);
 #pragma unroll 1
