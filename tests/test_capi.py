@@ -45,6 +45,15 @@ def test_device_memory_is_written_in_stream_order():
             assert "cudaMemcpyDeviceToHost" in call, (f, call)
 
 
+def compile_and_run(tmp_path, *sources):
+    """main.cpp of tmp_path with sources of csrc, by the host compiler; the numbers it prints."""
+    src, exe = os.path.join(ROOT, "tic-tac_b200", "csrc"), str(tmp_path / "main")
+    cuda = os.environ.get("CUDA", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-I" + src, "-I" + os.path.join(ROOT, "include"), "-I" + cuda + "/include",
+                    str(tmp_path / "main.cpp"), *(os.path.join(src, f) for f in sources), "-o", exe], check=True)
+    return [int(x) for x in subprocess.run([exe], capture_output=True, text=True, check=True).stdout.split()]
+
+
 def test_a_failed_call_waits_for_its_stream(tmp_path):
     # the buffers' scope against a CUDA runtime of counters: what a failed call left queued
     # may use buffers that the next call frees on another stream
@@ -85,14 +94,22 @@ int main() {
   std::printf("%d %d %d", good, failed, waits);
 }
 """)
-    src = os.path.join(ROOT, "tic-tac_b200", "csrc")
-    cuda = os.environ.get("CUDA", "/usr/local/cuda")
-    subprocess.run(["g++", "-std=c++17", "-I" + src, "-I" + os.path.join(ROOT, "include"), "-I" + cuda + "/include",
-                    str(tmp_path / "main.cpp"), os.path.join(src, "host", "tt_device_cache.cpp"), "-o",
-                    str(tmp_path / "main")], check=True, capture_output=True, text=True)
-    good, failed, both = map(int, subprocess.run([str(tmp_path / "main")], capture_output=True, text=True,
-                                                 check=True).stdout.split())
-    assert (good, failed, both) == (0, 1, 2)
+    assert compile_and_run(tmp_path, "host/tt_device_cache.cpp") == [0, 1, 2]
+
+
+def test_subpanel_clusters(tmp_path):
+    # rows of a sub-panel -> CTAs of its cluster, on devices whose largest cluster is 1, 8 or 16
+    (tmp_path / "main.cpp").write_text(r"""
+#include <cstdio>
+#include "cuda/tt_lu_internal.h"
+namespace tt { void set_error(const std::string&) {} }
+int main() {
+  for (int most : {1, 8, 16})
+    for (size_t m : {224, 225, 256, 512, 513, 2048, 2049, 4096, 4097})
+      std::printf("%d ", tt::subpanel_cluster_ctas(m, 224, 256, most));
+}
+""")
+    assert compile_and_run(tmp_path) == [0] * 9 + [0, 2, 2, 2, 4, 8, 0, 0, 0] + [0, 2, 2, 2, 4, 8, 16, 16, 0]
 
 
 def test_aligned_barriers_follow_a_converged_warp():

@@ -1880,15 +1880,8 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   for (const auto& row : sp_kernel)
     for (const void* k : row) TT_TRY(smem_limit_once(k, (int)kSubpanelSmem));
   const int max_cluster = subpanel_cluster<T>();
-  // CTAs of the cluster that holds m rows, a row per thread: the smallest power of
-  // two of about SP_CLUSTER_ROWS rows a CTA; 0: too tall, or one CTA holds them
   const size_t one_row = std::min(SP_ROWS, SC::MAX_ROWS);  // rows of a CTA with a row per thread
-  auto cluster_ctas = [&](size_t m) -> int {
-    if (m <= one_row || m > SP_CLUSTER_ROWS * max_cluster) return 0;
-    int g = 2;
-    while (g < max_cluster && (m + g - 1) / g > SP_CLUSTER_ROWS) g *= 2;
-    return g;
-  };
+  auto cluster_ctas = [&](size_t m) { return subpanel_cluster_ctas(m, one_row, SP_CLUSTER_ROWS, max_cluster); };
   // CTAs of a matrix of m rows, of at most `most`: one while its shared memory
   // holds them (no exchange through L2), else about SP_ROWS rows each; 0: too tall
   auto ctas = [&](size_t m, int most) -> int {

@@ -46,6 +46,16 @@ int zgemm_sub_dmma(double2* C, int ldc, const double2* L, int ldl, const double2
 int tc_gemm_sub(float2* C, int ldc, const float2* L, int ldl, const float2* U, int ldu, int M, int N, int K,
                 cudaStream_t st);
 
+// CTAs of the cluster that holds a sub-panel of m rows, a row per thread: the smallest
+// power of two, up to the device's largest cluster (1: none), of at most cluster_rows
+// rows a CTA.  0: no cluster does, or one CTA holds the rows (one_cta).
+inline int subpanel_cluster_ctas(size_t m, size_t one_cta, size_t cluster_rows, int max_cluster) {
+  if (max_cluster < 2 || m <= one_cta || m > cluster_rows * max_cluster) return 0;
+  int g = 2;
+  while (g < max_cluster && (m + g - 1) / g > cluster_rows) g *= 2;
+  return g;
+}
+
 inline int lu_update_tc(double2*, int, int, int, cudaStream_t) {
   set_error("tensor-core trailing update is only defined for the complex64 factorisation");
   return TT_ERR_UNSUPPORTED;
