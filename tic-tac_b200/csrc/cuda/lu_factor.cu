@@ -20,6 +20,8 @@
 
 #include <algorithm>
 #include <functional>
+#include <map>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -1779,21 +1781,16 @@ int panel_gemm_sub(int mode, T* C, int ldc, const T* L, int ldl, const T* U, int
   return gemm_sub(C, ldc, L, ldl, U, ldu, M, N, K, st);
 }
 
-// Largest cluster of full-size sub-panel CTAs the device runs: 16, 8 or 1
+// Largest cluster of full-size sub-panel CTAs the current device runs: 16, 8 or 1
 template <typename T>
-int subpanel_cluster() {
-  static int largest[16] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int& c = largest[dev & 15];
-  if (c) return c;
+int query_subpanel_cluster() {
   const void* k = (const void*)k_subpanel_ll<T, 1, true>;
   const void* k2 = (const void*)k_subpanel_ll<T, sizeof(T) == 8 ? 2 : 1, true>;
   for (const void* f : {k, k2})
     if (smem_limit_once(f, (int)kSubpanelSmem) != TT_OK ||
         cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
       cudaGetLastError();
-      return c = 1;
+      return 1;
     }
   for (int g : {16, 8}) {
     cudaLaunchConfig_t cfg = {};
@@ -1810,10 +1807,21 @@ int subpanel_cluster() {
     int n = 0, n2 = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&n2, k2, &cfg) == cudaSuccess && n > 0 && n2 > 0)
-      return c = g;
+      return g;
     cudaGetLastError();
   }
-  return c = 1;
+  return 1;
+}
+// ... asked once per device
+template <typename T>
+int subpanel_cluster() {
+  static std::mutex mu;
+  static std::map<int, int> largest;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = largest.find(dev);
+  return it != largest.end() ? it->second : largest[dev] = query_subpanel_cluster<T>();
 }
 
 }  // namespace
