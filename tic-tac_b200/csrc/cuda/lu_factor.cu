@@ -11,7 +11,7 @@
 //                on the rest of the panel (k_subpanel: from global memory with a
 //                grid barrier per column, for sub-panels too tall for shared
 //                memory)
-//   k_trsm_rows / k_trsm_blk  U = L^{-1} U for the unit-lower diagonal block
+//   k_trsm_rows  U = L^{-1} U for the unit-lower diagonal block
 //   the update of the remaining panel columns
 // then the panel's interchanges outside the panel (k_laswp2), the triangular
 // solve for U12 and the trailing update A22 -= L21 U12 (tcgen05 for complex64,
@@ -1402,9 +1402,6 @@ __global__ void __launch_bounds__(LS_THREADS) k_laswp2(SubpanelBatch<T> bt, int 
   }
 }
 
-// X <- L^{-1} X, L the w x w unit-lower block at (r0, r0), X = rows [r0, r0+w) of columns [cb, ce).
-// With pack_mode (complex64 only), X is also written as the packed B operand
-// of the real-row tensor-core update that follows (w deep, ce - cb columns).
 // The matrices of a batch whose same 32-row block is solved in one launch
 // (blockIdx.y = matrix); matrix b's operand planes start at WB + b plane.
 template <typename T>
@@ -1414,50 +1411,6 @@ struct TrsmBatch {
   size_t plane;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_trsm_blk(TrsmBatch<T> tb, int n, int r0, int w, int cb, int ce,
-                                                  int pack_mode) {
-  __shared__ T sL[IB][IB + 1];
-  __shared__ T sX[IB][33];
-  T* __restrict__ A = tb.A[blockIdx.y];
-  void* __restrict__ WB = tb.WB ? tb.WB + tb.plane * blockIdx.y : nullptr;
-  const int c0 = cb + blockIdx.x * 32;
-  for (int t = threadIdx.x; t < w * w; t += blockDim.x) sL[t / w][t % w] = A[(size_t)(r0 + t / w) * n + r0 + t % w];
-  for (int t = threadIdx.x; t < w * 32; t += blockDim.x) {
-    const int i = t / 32, c = c0 + t % 32;
-    T v;
-    v.x = 0;
-    v.y = 0;
-    if (c < ce) v = A[(size_t)(r0 + i) * n + c];
-    sX[i][t % 32] = v;
-  }
-  __syncthreads();
-  const int cc = threadIdx.x % 32, grp = threadIdx.x / 32;
-  for (int i = 0; i < w; i++) {
-    const T xi = sX[i][cc];
-    for (int r = i + 1 + grp; r < w; r += 8) {
-      const T l = sL[r][i];
-      T v = sX[r][cc];
-      v.x -= l.x * xi.x - l.y * xi.y;
-      v.y -= l.x * xi.y + l.y * xi.x;
-      sX[r][cc] = v;
-    }
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < w * 32; t += blockDim.x) {
-    const int i = t / 32, c = c0 + t % 32;
-    if (c < ce) {
-      A[(size_t)(r0 + i) * n + c] = sX[i][t % 32];
-      if constexpr (sizeof(T) == sizeof(float2)) {
-        if (pack_mode) {
-          const T v = sX[i][t % 32];
-          tc2_pack_b(pack_mode, WB, ce - cb, w, c - cb, i, make_float2(v.x, v.y));
-        }
-      }
-    }
-  }
-}
-
 // X <- L^{-1} X for the h x h unit-lower block (h = 32 NB <= 128) at (r0, r0) of each
 // matrix of the batch (blockIdx.y), X = rows [r0, r0 + h) of columns [cb, ce),
 // complex64, also packed as the B operand of the update that follows.  A CTA inverts
@@ -1466,7 +1419,7 @@ __global__ void __launch_bounds__(256) k_trsm_blk(TrsmBatch<T> tb, int n, int r0
 // 16-byte broadcasts.  Bound: latency of these steps (8 columns a CTA, as narrow as a
 // 64-byte row segment allows).  It stands for the explicit inverse of a mid-panel's
 // block, a pack, a tensor-core product and another pack (66 -> 13 us on average at 128 x up to
-// 384, n = 16,128) and for k_trsm_blk's substitution row by row (10 -> 4 us at 32 x up to 96).
+// 384, n = 16,128) and for a substitution row by row (10 -> 4 us at 32 x up to 96).
 // complex128 (h = 32, not packed): 11.5 -> 7.2 us on average over the factorisation of
 // n = 8,496.
 constexpr int TR_MAX = 128, TR_COLS = 8, TR_XLD = TR_COLS + 1;
@@ -1723,9 +1676,16 @@ int launch_trsm_rows(const TrsmBatch<T>& tb, int B, int n, int r0, int cb, int c
   count_launch();
   return TT_OK;
 }
+// Pack_mode: matrix b's solved rows also go to its operand planes at WB + b plane.  Panels, mid-panels and their halves are multiples of 32 wide and only the matrix's last
+// sub-panel is narrower, with nothing behind it.
 template <typename T>
-int trsm_rows_batched(T* const* As, int B, int n, int r0, int h, int cb, int ce, int pack_mode, unsigned char* WB,
-                      size_t plane, cudaStream_t st) {
+int trsm_rows_batched(T* const* As, int B, int n, int r0, int h, int cb, int ce, cudaStream_t st, int pack_mode = 0,
+                      unsigned char* WB = nullptr, size_t plane = 0) {
+  if (ce <= cb) return TT_OK;
+  if (h % IB != 0 || h > (sizeof(T) == sizeof(float2) ? TR_MAX : IB)) {
+    set_error("block row solve of " + std::to_string(h) + " rows");
+    return TT_ERR_BADARG;
+  }
   ProfScope prof(TT_PROF_PANEL_TRSM, st, 4.0 * h * h * (double)(ce - cb) * B,
                  2.0 * h * (double)(ce - cb) * sizeof(T) * B);
   TrsmBatch<T> tb{};
@@ -1740,30 +1700,6 @@ int trsm_rows_batched(T* const* As, int B, int n, int r0, int h, int cb, int ce,
     }
   }
   return launch_trsm_rows<T, 1>(tb, B, n, r0, cb, ce, pack_mode, st);
-}
-
-// the same block of B <= 4 matrices (pack_mode: matrix b's solved rows also
-// go to its operand planes at WB + b plane)
-template <typename T>
-int trsm_blk_batched(T* const* As, int B, int n, int r0, int w, int cb, int ce, cudaStream_t st, int pack_mode = 0,
-                     unsigned char* WB = nullptr, size_t plane = 0) {
-  if (ce <= cb) return TT_OK;
-  if (w == IB) return trsm_rows_batched<T>(As, B, n, r0, w, cb, ce, pack_mode, WB, plane, st);
-  ProfScope prof(TT_PROF_PANEL_TRSM, st, 4.0 * w * w * (double)(ce - cb) * B,
-                 2.0 * w * (double)(ce - cb) * sizeof(T) * B);
-  TrsmBatch<T> tb{};
-  for (int b = 0; b < B; b++) tb.A[b] = As[b];
-  tb.WB = WB;
-  tb.plane = plane;
-  k_trsm_blk<T><<<dim3(ceil_div(ce - cb, 32), B), 256, 0, st>>>(tb, n, r0, w, cb, ce, pack_mode);
-  count_launch();
-  TT_CUDA_TRY(cudaGetLastError());
-  return TT_OK;
-}
-
-template <typename T>
-int trsm_blk(T* A, int n, int r0, int w, int cb, int ce, cudaStream_t st) {
-  return trsm_blk_batched<T>(&A, 1, n, r0, w, cb, ce, st);
 }
 
 // C -= L U on the tensor cores in the factorisation's product mode when K is
@@ -1785,13 +1721,11 @@ int panel_gemm_sub(int mode, T* C, int ldc, const T* L, int ldl, const T* U, int
 template <typename T>
 int query_subpanel_cluster() {
   const void* k = (const void*)k_subpanel_ll<T, 1, true>;
-  const void* k2 = (const void*)k_subpanel_ll<T, sizeof(T) == 8 ? 2 : 1, true>;
-  for (const void* f : {k, k2})
-    if (smem_limit_once(f, (int)kSubpanelSmem) != TT_OK ||
-        cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-      cudaGetLastError();
-      return 1;
-    }
+  if (smem_limit_once(k, (int)kSubpanelSmem) != TT_OK ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
   for (int g : {16, 8}) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -1804,10 +1738,8 @@ int query_subpanel_cluster() {
     cfg.dynamicSmemBytes = kSubpanelSmem;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    int n = 0, n2 = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n2, k2, &cfg) == cudaSuccess && n > 0 && n2 > 0)
-      return g;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0) return g;
     cudaGetLastError();
   }
   return 1;
@@ -1881,12 +1813,14 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   TT_CUDA_TRY(cudaMemsetAsync(srec.ptr, 0, rec_bytes + verdicts * B, st));
   PivotScratch<T> scr{sval.ptr, sidx.ptr, srow.ptr, stop.ptr};
   using SC = SubpanelCfg<T>;
-  // rows per thread: complex128 rows fill shared memory before they outnumber the threads
+  // rows per thread: complex128 rows fill shared memory before they outnumber the threads,
+  // and a cluster's CTA holds at most SP_CLUSTER_ROWS
   constexpr int RPT2 = sizeof(T) == 8 ? 2 : 1;
+  static_assert(SP_CLUSTER_ROWS <= 32 * (SP_WARPS - 1), "a row per thread in a cluster");
   const void* sp_kernel[2][2] = {{(const void*)k_subpanel_ll<T, 1, false>, (const void*)k_subpanel_ll<T, RPT2, false>},
-                                 {(const void*)k_subpanel_ll<T, 1, true>, (const void*)k_subpanel_ll<T, RPT2, true>}};
-  for (const auto& row : sp_kernel)
-    for (const void* k : row) TT_TRY(smem_limit_once(k, (int)kSubpanelSmem));
+                                 {(const void*)k_subpanel_ll<T, 1, true>, nullptr}};
+  for (const void* k : {sp_kernel[0][0], sp_kernel[0][1], sp_kernel[1][0]})
+    TT_TRY(smem_limit_once(k, (int)kSubpanelSmem));
   const int max_cluster = subpanel_cluster<T>();
   const size_t one_row = std::min(SP_ROWS, SC::MAX_ROWS);  // rows of a CTA with a row per thread
   auto cluster_ctas = [&](size_t m) { return subpanel_cluster_ctas(m, one_row, SP_CLUSTER_ROWS, max_cluster); };
@@ -1978,7 +1912,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
   // rows [r0, r0 + h) of columns [cb, ce) <- L^{-1} of them, L the unit-lower h x h block at (r0, r0):
   // halves recursively, so that most of the work is one update of depth h / 2
   std::function<int(T*, int, int, int, int)> trsm_rec = [&](T* A, int r0, int h, int cb, int ce) -> int {
-    if (h <= IB) return trsm_blk(A, n, r0, h, cb, ce, st);
+    if (h <= IB) return trsm_rows_batched(&A, 1, n, r0, h, cb, ce, st);
     if (inv_solve && h % 32 == 0 && h <= IVB) {
       const T* A1 = A;
       TT_TRY(inv_unit_lower(&A1, 1, n, r0, h, Xinv.ptr, Tinv.ptr, st));
@@ -2096,7 +2030,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
           const float2* Us[kMaxBatch];
           float2* Af[kMaxBatch];
           for (int b = 0; b < B; b++) Af[b] = reinterpret_cast<float2*>(As[b]);
-          TT_TRY(trsm_blk_batched<T>(As, B, n, j0, w, j0 + w, m0 + mw, st, mode, WB, plane));
+          TT_TRY(trsm_rows_batched(As, B, n, j0, w, j0 + w, m0 + mw, st, mode, WB, plane));
           for (int b = 0; b < B; b++) {
             float2* A = Af[b];
             Cs[b] = A + (size_t)(j0 + w) * n + (j0 + w);
@@ -2107,7 +2041,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
         } else if (right > 0) {
           for (int b = 0; b < B; b++) {
             T* A = As[b];
-            TT_TRY(trsm_blk(A, n, j0, w, j0 + w, m0 + mw, st));
+            TT_TRY(trsm_rows_batched(&A, 1, n, j0, w, j0 + w, m0 + mw, st));
             TT_TRY(panel_gemm_sub(mode, A + (size_t)(j0 + w) * n + (j0 + w), n, A + (size_t)(j0 + w) * n + j0, n,
                                   A + (size_t)j0 * n + (j0 + w), n, n - j0 - w, right, w, st));
           }
@@ -2129,8 +2063,8 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
             Ls[b] = A + (size_t)(m0 + mw) * n + m0;
             Us[b] = A + (size_t)m0 * n + (m0 + mw);
           }
-          TT_TRY(trsm_rows_batched(Af, B, n, m0, mw, m0 + mw, k + kb, mode, WB, tc2_b_plane_bytes(mode, right_out, mw),
-                                  st));
+          TT_TRY(trsm_rows_batched(Af, B, n, m0, mw, m0 + mw, k + kb, st, mode, WB,
+                                  tc2_b_plane_bytes(mode, right_out, mw)));
           TT_TRY(tc2_gemm_sub_batched(mode, B, Cs, n, Ls, n, Us, n, n - m0 - mw, right_out, mw, st, 0, true));
         } else {
           TT_TRY(trsm_all(m0, mw, m0 + mw, k + kb));
@@ -2148,7 +2082,7 @@ int lu_factor_batched_device(T* const* As, int B, int n, int32_t* const* ipivs, 
       // ---- U12 blocked by IB without tensor cores
       if (!inv_solve) for (int i0 = k; i0 < k + kb; i0 += IB) {
         const int wi = std::min(IB, k + kb - i0);
-        TT_TRY(trsm_blk(A, n, i0, wi, k + kb, n, st));
+        TT_TRY(trsm_rows_batched(&A, 1, n, i0, wi, k + kb, n, st));
         const int below = k + kb - (i0 + wi);
         if (below > 0)
           TT_TRY(panel_gemm_sub(mode, A + (size_t)(i0 + wi) * n + (k + kb), n, A + (size_t)(i0 + wi) * n + i0, n,
