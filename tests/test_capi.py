@@ -124,3 +124,13 @@ def test_aligned_barriers_follow_a_converged_warp():
             assert before.endswith("__syncwarp();"), (f, text.count("\n", 0, m.start()) + 1)
             found += 1
     assert found == 8
+
+
+def test_changed_headers_rebuild_the_library():
+    root = os.path.join(ROOT, "tic-tac_b200")
+    headers = [os.path.join(d, f) for d, _, fs in os.walk(os.path.join(root, "csrc")) for f in fs
+               if f.endswith((".h", ".cuh"))]
+    assert len(headers) > 8
+    for h in headers:
+        out = subprocess.run(["make", "-n", "-C", root, "-W", h], capture_output=True, text=True, check=True).stdout
+        assert ".cu " in out and " -shared " in out, h

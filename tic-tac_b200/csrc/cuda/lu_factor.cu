@@ -1676,7 +1676,8 @@ int launch_trsm_rows(const TrsmBatch<T>& tb, int B, int n, int r0, int cb, int c
   count_launch();
   return TT_OK;
 }
-// Pack_mode: matrix b's solved rows also go to its operand planes at WB + b plane.  Panels, mid-panels and their halves are multiples of 32 wide and only the matrix's last
+// Pack_mode: matrix b's solved rows also go to its operand planes at WB + b plane.
+// Panels, mid-panels and their halves are multiples of 32 wide; only the matrix's last
 // sub-panel is narrower, with nothing behind it.
 template <typename T>
 int trsm_rows_batched(T* const* As, int B, int n, int r0, int h, int cb, int ce, cudaStream_t st, int pack_mode = 0,
