@@ -271,3 +271,68 @@ def test_pade_determinants_with_rows_exchanged():
                      for j in range(8)])
     assert np.all(abs(U[0] - want) <= 1e-4 * abs(want).max())
     assert np.array_equal(U[0], U[1]) and np.array_equal(U[0], U[2])
+
+
+@pytest.mark.parametrize("precision", [tt.PRECISION_FP64, tt.PRECISION_MIXED])
+def test_pivots_found_in_two_trips(precision):
+    # n = 8,192: 37 CTAs a matrix and so two trips through L2 for a search (records of one
+    # element, then the winner's row) down to 7,168 rows; a fifth to a third of the sub-panels
+    # have pivots below their block.  P has 80 nonzeros a column (the condition numbers are
+    # 4e5 to 4e7, the elements come out to 1e-15 in 64 bits).
+    import torch
+
+    Np = 64
+    n, rng = 2 * Np * Np, np.random.default_rng(7)
+    pw = np.array([[0, 0, 0, 1, 0, 1, 1, 1, 1], [0, 1, 1, 0, 0, 1, 1, 1, 1]], dtype=np.int32)
+    eye, e = np.tile(np.eye(Np).ravel(), 6), np.tile(np.linspace(-2, 100, Np + 1), 6)
+    swp = tt.SWP(Np, Np, 6, 0, -2.0, e, None, eye, None, np.linspace(0, 1000, Np + 1))
+    far = np.arange(17, n - 300, 97)
+    far = far[(far % 32 != 0) & (far % 7 != 0)]
+    i = np.arange(n)
+    row = np.concatenate([np.repeat(i, 32), np.repeat(i, 48), far + 300])
+    col = np.concatenate([(i[:, None] // 32 * 32 + np.arange(32)).ravel(), rng.integers(0, n, n * 48), far])
+    val = np.concatenate([rng.standard_normal(n * 32) * 2e-2, rng.standard_normal(n * 48) * (1e-2 / np.sqrt(48)),
+                          np.ones(len(far))])
+    at, which = np.unique(col.astype(np.int64) * n + row, return_inverse=True)  # by column, then row
+    val = np.bincount(which, weights=val)
+    colptr = np.concatenate([[0], np.cumsum(np.bincount(at // n, minlength=n))]).astype(np.uint64)
+    scale = {"below": 0.1, "block": 100.0, "anywhere": 3e4}
+    G = np.stack([scale[k] * np.exp(1j * rng.uniform(0, 2 * np.pi, n)) for k in scale])
+    G[:, far] = np.array([40.0, 0.01, 0.01])[:, None]
+    q_idx = np.array([3, 20, 50])
+    U, rep = tt.solve_faddeev(G, val, (at % n).astype(np.int32), colptr, eye, None, swp, q_idx, [1], tt.PW(pw),
+                              precision=precision, tensor_force=0, isospin_breaking_1S0=0)
+    A = torch.zeros(n * n, dtype=torch.float64, device="cuda")
+    A[torch.from_numpy(at % n * n + at // n).cuda()] = torch.from_numpy(2 * val).cuda()
+    A = A.view(n, n)
+    for j in range(3):
+        L = torch.eye(n, dtype=torch.complex128, device="cuda") - A * torch.from_numpy(G[j]).cuda()
+        r = Np * Np + int(q_idx[j]) * Np
+        want = torch.linalg.solve(L, A[:, r].to(L.dtype))[r].item()
+        assert abs(U[j] - want) <= 1e-10 * abs(want), (j, U[j], want, rep)
+
+
+@pytest.mark.parametrize("precision", [tt.PRECISION_FP64, tt.PRECISION_MIXED])
+@pytest.mark.parametrize("Np", [16, 48])  # clusters and one CTA; records in L2
+def test_resolvents_that_are_not_finite(precision, Np):
+    # A = diag(2): a NaN in G makes its column of 1 - A G NaN, which has no pivot.  So does an
+    # infinity (0 inf is NaN, and elimination carries the NaN above down onto the infinity),
+    # except in the first column, where it is the pivot and makes everything behind it NaN.
+    n = 2 * Np * Np
+    pw = np.array([[0, 0, 0, 1, 0, 1, 1, 1, 1], [0, 1, 1, 0, 0, 1, 1, 1, 1]], dtype=np.int32)
+    eye, e = np.tile(np.eye(Np).ravel(), 6), np.tile(np.linspace(-2, 100, Np + 1), 6)
+    swp = tt.SWP(Np, Np, 6, 0, -2.0, e, None, eye, None, np.linspace(0, 1000, Np + 1))
+
+    def solve(g, at):
+        G = np.full(n, 0.125 + 0.25j)
+        G[at] = g
+        return tt.solve_faddeev(G, np.ones(n), np.arange(n, dtype=np.int32), np.arange(n + 1, dtype=np.uint64), eye,
+                                None, swp, [3], [1], tt.PW(pw), precision=precision, tensor_force=0,
+                                isospin_breaking_1S0=0)[0]
+
+    for g, at, col in ((np.nan, 0, 1), (np.nan, 40, 41), (np.nan, n - 1, n), (np.inf, 0, 2), (np.inf, 31, 32),
+                       (np.inf, n - 200, n - 199), (np.inf, n - 1, n)):
+        with pytest.raises(tt.TicTacError) as err:
+            solve(g, at)
+        assert err.value.code == tt.TT_ERR_SINGULAR and f"column {col} " in str(err.value), (g, at, str(err.value))
+    assert np.all(np.isfinite(solve(0.5j, 5)))
