@@ -84,7 +84,7 @@ struct AbLayout {
 // the warps contract the chunk with Ct on the FP64 tensor cores (mma m8n8k4); the
 // Ct fragments stay in registers for all chunks.  MT row tiles of 8 (4 for
 // Np <= 32, 8 for Np <= 64).  Bound: latency of the T rows and the FP64 tensor
-// pipe (28% busy); the two resident CTAs overlap them.  n = 24,300 10.9 -> 6.0 ms,
+// pipe (28% busy at Np = 30); the two resident CTAs overlap them.  n = 24,300 10.9 -> 6.0 ms,
 // n = 42,300 35.5 -> 19.4 ms, n = 16,128 9.1 -> 4.0 ms (64-column chunks, a read-add-write of T per nonzero,
 // Ct read from it per chunk before).
 template <int MT>

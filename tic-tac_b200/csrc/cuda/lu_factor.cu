@@ -281,14 +281,16 @@ __global__ void __launch_bounds__(256) k_subpanel(T* __restrict__ A, int n, int 
 // Of a column's 2.5 to 6 thousand cycles the trips through L2 take about 1,200
 // each; the rest is the latency of its own instructions.
 //
-// The matrices are 1 - A G: all 32 pivots of a sub-panel lie in its 32 x 32 diagonal
-// block in 96 to 100% of the sub-panels, nearly always on the diagonal.  So the kernel
+// The matrices are 1 - A G: all 32 pivots of a sub-panel mostly lie in its 32 x 32 diagonal
+// block, nearly always on the diagonal (in 96 to 100% of the sub-panels of channels of
+// n = 8,496 to 42,300; two in three at n = 512 of Malfliet-Tjon s-waves).  So the kernel
 // first tries that, without any exchange: every CTA factors the diagonal block for
 // itself (sp_factor_diag, and with interchanges in the block, sp_factor_block, where the
 // diagonal will not do), takes its own rows through the block's U (sp_try_row) and looks
 // at each element before its division: none may exceed the pivot of its column by the
 // same keys that the search compares.  One verdict a CTA, one trip, and if all agree these
-// are the search's pivots and its result.  Else the rows, still unchanged in A, are read
+// are pivots that the search may choose (its elements differ in their rounding, so near
+// ties may fall the other way).  Else the rows, still unchanged in A, are read
 // again for the search; a matrix whose tries fail in a row goes 1, 3, 7, then 15
 // sub-panels without one, so that a try (a fifth of a search) is lost on few.
 // Bound: the latency of the block's 32 steps (~5 us) and the rows' FP32 multiply-adds.

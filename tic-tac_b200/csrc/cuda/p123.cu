@@ -192,7 +192,8 @@ __global__ void k_legendre(int row0, int nrows, const double* __restrict__ x, in
 // neighbouring doubles, and each B is made once for all alpha pairs; evaluating
 // every pair's own term list (gathers from the spharm tables) took 624 ms of the
 // 63-wave channel at N = 16 and 70 ms of the 31-wave one at N = 24, this takes
-// 2.0 and 0.9 ms.  Bound: F written once to HBM.
+// 2.0 and 0.9 ms.  Bound: latency of the term lists and table reads (58% of the issue
+// slots busy, F stored at 1.1 TB/s at n = 9,072).
 constexpr int ORB_K = 32, ORB_THREADS = 256;
 constexpr size_t kOrbSmem = 220 * 1024;
 // STAGED: the spharm columns in shared memory (up to l = 25 or so); else read

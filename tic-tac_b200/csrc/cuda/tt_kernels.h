@@ -78,8 +78,8 @@ int residual_multi_device(const double* d_A, int n, const double* d_y, const dou
 // LU with partial pivoting, in place, row-major (lu.cu).  ipiv[k] = row swapped with k.
 template <typename T>
 int lu_factor_device(T* d_L, int n, int32_t* d_ipiv, cudaStream_t st, int use_tensor_cores, int* info);
-// B <= 4 matrices of equal n factored together (each sub-panel of all of them
-// in one cooperative launch, one grid barrier per column for the batch);
+// B <= 4 matrices of equal n factored together (each sub-panel of all of them in
+// one launch, the CTAs of a matrix meeting in their cluster or through records);
 // info[B] receives each matrix's first zero pivot (1-based) or 0.
 // blocked: the panel in 32-column steps, each followed by its rank-32 update
 // (otherwise recursive halving of the panel and of the U12 solve).

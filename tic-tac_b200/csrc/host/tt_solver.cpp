@@ -482,7 +482,7 @@ int ChannelSolver::solve(const std::vector<int>& q_idx, const std::vector<int>& 
   }
   const int Nq = L_.Nq, Np = L_.Np;
   // complex64: up to opt.energy_batch (<= 4) energies' matrices formed and
-  // factored together (their sub-panels share each grid barrier), as many as
+  // factored together (their sub-panels share each launch), as many as
   // free HBM holds
   int B = 1;
   if (opt.mixed && nE > 1 && opt.energy_batch > 1) {
